@@ -61,8 +61,8 @@ int occupancy() {
     default: MACRO(8, 64); break;    \
   }
 
-template <class T, bool FAST>
-void BatchLaunch<T, FAST>::box(int cfg, bool blend, unsigned* cols, unsigned* rows) {
+template <class H, bool FAST>
+void BatchLaunch<H, FAST>::box(int cfg, bool blend, unsigned* cols, unsigned* rows) {
 #define WENO_BOX(TX, TY)                                      \
   *cols = (unsigned)TileGeom<TX, TY, false>::UC;              \
   *rows = blend ? (unsigned)TileGeom<TX, TY, true>::UR : (unsigned)TileGeom<TX, TY, false>::UR;
@@ -70,8 +70,9 @@ void BatchLaunch<T, FAST>::box(int cfg, bool blend, unsigned* cols, unsigned* ro
 #undef WENO_BOX
 }
 
-template <class T, bool FAST>
-size_t BatchLaunch<T, FAST>::smem_bytes(int cfg, bool blend) {
+template <class H, bool FAST>
+size_t BatchLaunch<H, FAST>::smem_bytes(int cfg, bool blend) {
+  using T = dev_t<H>;
   size_t r = 0;
 #define WENO_SM(TX, TY) \
   r = blend ? bdetail::tile_smem<T, TX, TY, true>() : bdetail::tile_smem<T, TX, TY, false>()
@@ -80,8 +81,9 @@ size_t BatchLaunch<T, FAST>::smem_bytes(int cfg, bool blend) {
   return r > 227 * 1024 ? 0 : r;
 }
 
-template <class T, bool FAST>
-int BatchLaunch<T, FAST>::ctas_per_sm(int cfg, bool chr, bool blend) {
+template <class H, bool FAST>
+int BatchLaunch<H, FAST>::ctas_per_sm(int cfg, bool chr, bool blend) {
+  using T = dev_t<H>;
   int r = 0;
 #define WENO_OCC(TX, TY)                                                                   \
   if (chr && blend) r = bdetail::occupancy<T, FAST, true, true, TX, TY>();                 \
@@ -93,11 +95,12 @@ int BatchLaunch<T, FAST>::ctas_per_sm(int cfg, bool chr, bool blend) {
   return r;
 }
 
-template <class T, bool FAST>
-cudaError_t BatchLaunch<T, FAST>::stage(int cfg, bool chr, bool blend, const SolveDesc* solves, SolveCtl* ctl,
+template <class H, bool FAST>
+cudaError_t BatchLaunch<H, FAST>::stage(int cfg, bool chr, bool blend, const SolveDesc* solves, SolveCtl* ctl,
                                         const void* tiles, int ntiles, int grid, const void* tmaps, const void* qn,
                                         void* qo, int stage, double gamma, double jp_lo, double jp_hi,
                                         double weps, int skip_tile, unsigned long long wait_ns, cudaStream_t st) {
+  using T = dev_t<H>;
   if (ntiles <= 0 || grid <= 0) return cudaSuccess;
   const int4* tl = static_cast<const int4*>(tiles);
   const CUtensorMap* a = static_cast<const CUtensorMap*>(tmaps);
@@ -122,11 +125,12 @@ cudaError_t BatchLaunch<T, FAST>::stage(int cfg, bool chr, bool blend, const Sol
   return e;
 }
 
-template <class T, bool FAST>
-cudaError_t BatchLaunch<T, FAST>::staged(bool chr, bool blend, const SolveDesc* solves, SolveCtl* ctl,
+template <class H, bool FAST>
+cudaError_t BatchLaunch<H, FAST>::staged(bool chr, bool blend, const SolveDesc* solves, SolveCtl* ctl,
                                          const void* tiles, int ntiles, int grid, const void* qs, const void* qn,
                                          void* qo, void* ws, int stage, double gamma, double jp_lo, double jp_hi,
                                          double weps, cudaStream_t st) {
+  using T = dev_t<H>;
   if (ntiles <= 0 || grid <= 0) return cudaSuccess;
   constexpr int TX = kTileTX[kStagedConfig], TY = kTileTY[kStagedConfig], NT = bdetail::kNT;
   const int4* tl = static_cast<const int4*>(tiles);
@@ -155,9 +159,10 @@ cudaError_t BatchLaunch<T, FAST>::staged(bool chr, bool blend, const SolveDesc* 
   return cudaGetLastError();
 }
 
-template <class T, bool FAST>
-cudaError_t BatchLaunch<T, FAST>::cfl(int cfg, const SolveDesc* solves, SolveCtl* ctl, const void* tiles, int ntiles,
+template <class H, bool FAST>
+cudaError_t BatchLaunch<H, FAST>::cfl(int cfg, const SolveDesc* solves, SolveCtl* ctl, const void* tiles, int ntiles,
                                       int grid, const void* q, double gamma, cudaStream_t st) {
+  using T = dev_t<H>;
   if (ntiles <= 0 || grid <= 0) return cudaSuccess;
   const int tx = kTileTX[cfg < kNumTileConfigs ? cfg : 0], ty = kTileTY[cfg < kNumTileConfigs ? cfg : 0];
   k_cfl_tiles<T, bdetail::kNT><<<grid, bdetail::kNT, 0, st>>>(solves, ctl, static_cast<const int4*>(tiles), ntiles,
@@ -165,8 +170,8 @@ cudaError_t BatchLaunch<T, FAST>::cfl(int cfg, const SolveDesc* solves, SolveCtl
   return cudaGetLastError();
 }
 
-template <class T, bool FAST>
-cudaError_t BatchLaunch<T, FAST>::clock(SolveCtl* ctl, int nsolves, int phase, cudaStream_t st) {
+template <class H, bool FAST>
+cudaError_t BatchLaunch<H, FAST>::clock(SolveCtl* ctl, int nsolves, int phase, cudaStream_t st) {
   if (nsolves <= 0) return cudaSuccess;
   k_solve_clock<<<(nsolves + 127) / 128, 128, 0, st>>>(ctl, nsolves, phase);
   return cudaGetLastError();

@@ -52,13 +52,14 @@ struct SolveCtl {
 
 inline namespace WENO_TU_NS {
 
+// Running maximum of wave speeds (non-negative, or NaN of either sign) as
+// unsigned integers: NaN's bits order above +inf's, as np.max propagates NaN.
+__device__ __forceinline__ unsigned long long max_bits(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
+__device__ __forceinline__ unsigned long long speed_bits(double x) { return (unsigned long long)__double_as_longlong(x); }
+
 // Where the boundary fill would take ghost cell (I, J) (padded coordinates)
 // from: an interior cell (i, j) with a sign on the normal momentum, or the
 // inflow constant.
-__device__ __forceinline__ double nan_max_b(double a, double b) {
-  return (a != a || b != b) ? __longlong_as_double(0x7ff8000000000000ll) : fmax(a, b);
-}
-
 struct GhostSrc {
   int i, j;
   bool post;
@@ -168,10 +169,13 @@ __device__ __forceinline__ void tile_gq_side(const T* p, int ks, int ts, T weps,
       a1[k] = ra.v.x, a1[k + 1] = ra.v.y, a2[k] = rb.v.x, a2[k + 1] = rb.v.y;
     }
   } else {
-#pragma unroll
+#pragma unroll(FAST ? 4 : 1)
     for (int k = 0; k < 4; ++k) {
       const T* u = p + k * ks;
-      weno5_gq_pair<T, FAST>(u[0], u[ts], u[2 * ts], u[3 * ts], u[4 * ts], a1[k], a2[k], weps);
+      T a, b;
+      weno5_gq_pair<T, FAST>(u[0], u[ts], u[2 * ts], u[3 * ts], u[4 * ts], a, b, weps);
+      put4(a1, k, a);
+      put4(a2, k, b);
     }
   }
 }
@@ -220,7 +224,7 @@ __global__ void __launch_bounds__(NT) k_stage_tiles(const SolveDesc* __restrict_
   T* FX = P1 + G::P1_ELEMS;
   T* FY = FX;  // the y faces reuse the x faces' buffer
   T* DXF = FX + G::F_ELEMS;
-  __shared__ double red[NT / 32];
+  __shared__ unsigned long long red[NT / 32];
   __shared__ uint64_t bar;
   const int tid = threadIdx.x;
   if (tid == 0) {
@@ -415,7 +419,7 @@ __global__ void __launch_bounds__(NT) k_stage_tiles(const SolveDesc* __restrict_
     const double dt = ctl[tl.x].dt;
     const T* qn = Qn + d.off;
     T* qo = Qo + d.off;
-    double best = 0.0;
+    unsigned long long best = 0;
     for (int e = tid; e < TX * TY; e += NT) {
       const int il = e / TY, jl = e % TY;
       const int i = i0 + il, j = j0 + jl;
@@ -474,21 +478,21 @@ __global__ void __launch_bounds__(NT) k_stage_tiles(const SolveDesc* __restrict_
           uu = v[1] / rho;
           vv = v[2] / rho;
         }
-        const T pp = fmax((gamma - T(1.0)) * (v[3] - T(0.5) * rho * (uu * uu + vv * vv)), T(kEps));
+        const T pp = vmax<T>((gamma - T(1.0)) * (v[3] - T(0.5) * rho * (uu * uu + vv * vv)), T(kEps));
         const T rden = r0 != r0 ? r0 : fmax(r0, T(1e-14));  // np.maximum: a NaN density stays NaN
         const T x = sqrt(qdiv<T, FAST>(gamma * pp, rden)) + sqrt(uu * uu + vv * vv);
-        best = nan_max_b(best, (double)x);
+        best = max_bits(best, speed_bits((double)x));
       }
     }
     if (stage == 3) {
-      for (int off = 16; off > 0; off >>= 1) best = nan_max_b(best, __shfl_xor_sync(0xffffffffu, best, off));
+      for (int off = 16; off > 0; off >>= 1) best = max_bits(best, __shfl_xor_sync(0xffffffffu, best, off));
       if ((tid & 31) == 0) red[tid >> 5] = best;
       __syncthreads();
       if (tid == 0) {
-        double b = 0.0;
-        for (int w = 0; w < NT / 32; ++w) b = nan_max_b(b, red[w]);
-        atomicMax(&ctl[tl.x].cmax_bits, (unsigned long long)__double_as_longlong(b));
-        if (!(b < INFINITY)) atomicOr(&ctl[tl.x].status, 1);
+        unsigned long long b = 0;
+        for (int w = 0; w < NT / 32; ++w) b = max_bits(b, red[w]);
+        atomicMax(&ctl[tl.x].cmax_bits, b);
+        if (b >= 0x7ff0000000000000ull) atomicOr(&ctl[tl.x].status, 1);
       }
     }
     // the next tile's TMA load overwrites U: order this tile's shared-memory
@@ -596,25 +600,25 @@ __global__ void __launch_bounds__(NT) k_staged_pass1(const SolveDesc* __restrict
 // only face A is wanted and the sixth value is not read.  SUM: twice the
 // averages (the Gauss-point sums), for the doubled-state HLLE.
 template <bool Y, bool SUM>
-__device__ __forceinline__ void staged_gq_two(const double* p, long long ks, long long ts, bool two, double gamma,
-                                              double weps, double qA[4], double fA[4], double qB[4], double fB[4]) {
-  double a1A[4], a2A[4], a1B[4], a2B[4];
+__device__ __forceinline__ void staged_gq_two(const f64* p, long long ks, long long ts, bool two, f64 gamma,
+                                              f64 weps, f64 qA[4], f64 fA[4], f64 qB[4], f64 fB[4]) {
+  f64 a1A[4], a2A[4], a1B[4], a2B[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const double* u = p + k * ks;
-    const double v4 = u[4 * ts];
-    weno5_gq_two<double>(u[0], u[ts], u[2 * ts], u[3 * ts], v4, two ? u[5 * ts] : v4, weps, a1A[k], a2A[k], a1B[k],
+    const f64* u = p + k * ks;
+    const f64 v4 = u[4 * ts];
+    weno5_gq_two<f64>(u[0], u[ts], u[2 * ts], u[3 * ts], v4, two ? u[5 * ts] : v4, weps, a1A[k], a2A[k], a1B[k],
                          a2B[k]);
   }
-  double f1[4], f2[4];
-  euler_flux_pair<double, true, Y>(a1A, a2A, gamma, f1, f2);
+  f64 f1[4], f2[4];
+  euler_flux_pair<f64, true, Y>(a1A, a2A, gamma, f1, f2);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     fA[k] = SUM ? f1[k] + f2[k] : 0.5 * (f1[k] + f2[k]);
     qA[k] = SUM ? a1A[k] + a2A[k] : 0.5 * (a1A[k] + a2A[k]);
   }
   if (!two) return;
-  euler_flux_pair<double, true, Y>(a1B, a2B, gamma, f1, f2);
+  euler_flux_pair<f64, true, Y>(a1B, a2B, gamma, f1, f2);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     fB[k] = SUM ? f1[k] + f2[k] : 0.5 * (f1[k] + f2[k]);
@@ -646,11 +650,11 @@ __global__ void __launch_bounds__(NT) k_staged_pass2(const SolveDesc* __restrict
       const int nxp = (nxc + 1) / 2, nxi = (xr1 - i0) * nxp;  // x-face pairs (jj, jj+1)
       const int nyi = ((yr1 - i0 + 1) / 2) * nyc;              // y-face pairs (ii, ii+1)
       for (int e = threadIdx.x; e < nxi + nyi; e += NT) {
-        double qlA[4], flA[4], qlB[4], flB[4], qrA[4], frA[4], qrB[4], frB[4];
+        T qlA[4], flA[4], qlB[4], flB[4], qrA[4], frA[4], qrB[4], frB[4];
         if (e < nxi) {
           const int fi = i0 + e / nxp, jj = j0 + 2 * (e % nxp);
           const bool two = jj + 1 < xc1;
-          const double* p = W + d.w_p1x + (long long)fi * d.l_p1x + jj;
+          const T* p = W + d.w_p1x + (long long)fi * d.l_p1x + jj;
           staged_gq_two<false, SUM>(p, d.s_p1x, 1, two, gamma, weps, qlA, flA, qlB, flB);
           staged_gq_two<false, SUM>(p + 4 * d.s_p1x, d.s_p1x, 1, two, gamma, weps, qrA, frA, qrB, frB);
           tile_face_flux<T, FAST, false, BLEND, S>(qlA, flA, qrA, frA, gamma, W + d.w_fx, (int)d.s_fx,
@@ -662,7 +666,7 @@ __global__ void __launch_bounds__(NT) k_staged_pass2(const SolveDesc* __restrict
           const int e2 = e - nxi;
           const int ii = i0 + 2 * (e2 / nyc), fj = j0 + e2 % nyc;
           const bool two = ii + 1 < yr1;
-          const double* p = W + d.w_p1y + (long long)ii * d.l_p1y + fj;
+          const T* p = W + d.w_p1y + (long long)ii * d.l_p1y + fj;
           staged_gq_two<true, SUM>(p, d.s_p1y, d.l_p1y, two, gamma, weps, qlA, flA, qlB, flB);
           staged_gq_two<true, SUM>(p + 4 * d.s_p1y, d.s_p1y, d.l_p1y, two, gamma, weps, qrA, frA, qrB, frB);
           tile_face_flux<T, FAST, true, BLEND, S>(qlA, flA, qrA, frA, gamma, W + d.w_fy, (int)d.s_fy,
@@ -731,7 +735,7 @@ __global__ void __launch_bounds__(NT) k_staged_residual(const SolveDesc* __restr
                                                          const int4* __restrict__ tiles, int ntiles, const T* W,
                                                          const T* Qs, const T* Qn, T* Qo, int stage, T gamma,
                                                          T jp_lo, T jp_hi) {
-  __shared__ double red[NT / 32];
+  __shared__ unsigned long long red[NT / 32];
   const int tid = threadIdx.x;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int4 tl = tiles[t];
@@ -743,7 +747,7 @@ __global__ void __launch_bounds__(NT) k_staged_residual(const SolveDesc* __restr
     const T* Fy = W + d.w_fy;
     const long long fxs = d.s_fx, fys = d.s_fy;
     const int lx = d.ld, ly = d.l_p1y;
-    double best = 0.0;
+    unsigned long long best = 0;
     for (int e = tid; e < TX * TY; e += NT) {
       const int i = i0 + e / TY, j = j0 + e % TY;
       if (i >= nx || j >= ny) continue;
@@ -807,21 +811,21 @@ __global__ void __launch_bounds__(NT) k_staged_residual(const SolveDesc* __restr
           uu = v[1] / rho;
           vv = v[2] / rho;
         }
-        const T pp = fmax((gamma - T(1.0)) * (v[3] - T(0.5) * rho * (uu * uu + vv * vv)), T(kEps));
+        const T pp = vmax<T>((gamma - T(1.0)) * (v[3] - T(0.5) * rho * (uu * uu + vv * vv)), T(kEps));
         const T rden = r0 != r0 ? r0 : fmax(r0, T(1e-14));  // np.maximum: a NaN density stays NaN
         const T x = sqrt(qdiv<T, FAST>(gamma * pp, rden)) + sqrt(uu * uu + vv * vv);
-        best = nan_max_b(best, (double)x);
+        best = max_bits(best, speed_bits((double)x));
       }
     }
     if (stage == 3) {
-      for (int off = 16; off > 0; off >>= 1) best = nan_max_b(best, __shfl_xor_sync(0xffffffffu, best, off));
+      for (int off = 16; off > 0; off >>= 1) best = max_bits(best, __shfl_xor_sync(0xffffffffu, best, off));
       if ((tid & 31) == 0) red[tid >> 5] = best;
       __syncthreads();
       if (tid == 0) {
-        double b = 0.0;
-        for (int w = 0; w < NT / 32; ++w) b = nan_max_b(b, red[w]);
-        atomicMax(&ctl[tl.x].cmax_bits, (unsigned long long)__double_as_longlong(b));
-        if (!(b < INFINITY)) atomicOr(&ctl[tl.x].status, 1);
+        unsigned long long b = 0;
+        for (int w = 0; w < NT / 32; ++w) b = max_bits(b, red[w]);
+        atomicMax(&ctl[tl.x].cmax_bits, b);
+        if (b >= 0x7ff0000000000000ull) atomicOr(&ctl[tl.x].status, 1);
       }
       __syncthreads();
     }
@@ -833,32 +837,32 @@ template <class T, int NT>
 __global__ void __launch_bounds__(NT) k_cfl_tiles(const SolveDesc* __restrict__ solves, SolveCtl* ctl,
                                                    const int4* __restrict__ tiles, int ntiles, int TX, int TY,
                                                    const T* Q, T gamma) {
-  __shared__ double red[NT / 32];
+  __shared__ unsigned long long red[NT / 32];
   const int tid = threadIdx.x;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int4 tl = tiles[t];
     if (!ctl[tl.x].active) continue;
     const SolveDesc d = solves[tl.x];
-    double best = 0.0;
+    unsigned long long best = 0;
     for (int e = tid; e < TX * TY; e += NT) {
       const int i = tl.y + e / TY, j = tl.z + e % TY;
       if (i >= d.nx || j >= d.ny) continue;
       const long long o = d.off + (long long)i * d.ld + j;
-      const double r0 = (double)Q[o];
-      const double rho = fmax(r0, kEps);
-      const double uu = (double)Q[o + d.ps] / rho, vv = (double)Q[o + 2 * d.ps] / rho;
-      const double pp = fmax(((double)gamma - 1.0) * ((double)Q[o + 3 * d.ps] - 0.5 * rho * (uu * uu + vv * vv)), kEps);
-      const double x = sqrt((double)gamma * pp / (r0 != r0 ? r0 : fmax(r0, 1e-14))) + sqrt(uu * uu + vv * vv);
-      best = nan_max_b(best, x);
+      const f64 g((double)gamma), r0((double)Q[o]);
+      const f64 rho = fmax(r0, f64(kEps));
+      const f64 uu = f64((double)Q[o + d.ps]) / rho, vv = f64((double)Q[o + 2 * d.ps]) / rho;
+      const f64 pp = fmax((g - f64(1.0)) * (f64((double)Q[o + 3 * d.ps]) - f64(0.5) * rho * (uu * uu + vv * vv)), f64(kEps));
+      const f64 x = sqrt(g * pp / (r0 != r0 ? r0 : fmax(r0, f64(1e-14)))) + sqrt(uu * uu + vv * vv);
+      best = max_bits(best, speed_bits(x.v));
     }
-    for (int off = 16; off > 0; off >>= 1) best = nan_max_b(best, __shfl_xor_sync(0xffffffffu, best, off));
+    for (int off = 16; off > 0; off >>= 1) best = max_bits(best, __shfl_xor_sync(0xffffffffu, best, off));
     if ((tid & 31) == 0) red[tid >> 5] = best;
     __syncthreads();
     if (tid == 0) {
-      double b = 0.0;
-      for (int w = 0; w < NT / 32; ++w) b = nan_max_b(b, red[w]);
-      atomicMax(&ctl[tl.x].cmax_bits, (unsigned long long)__double_as_longlong(b));
-      if (!(b < INFINITY)) atomicOr(&ctl[tl.x].status, 1);
+      unsigned long long b = 0;
+      for (int w = 0; w < NT / 32; ++w) b = max_bits(b, red[w]);
+      atomicMax(&ctl[tl.x].cmax_bits, b);
+      if (b >= 0x7ff0000000000000ull) atomicOr(&ctl[tl.x].status, 1);
     }
     __syncthreads();
   }

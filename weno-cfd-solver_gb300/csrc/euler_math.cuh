@@ -20,13 +20,14 @@
 #include <cstdint>
 #include <type_traits>
 
-#include "df64.cuh"
-#include "f32x2.cuh"
-#include "fp64_fast.cuh"
-
 #ifndef WENO_TU_NS
 #error "WENO_TU_NS names the translation unit's inline namespace (tu_exact or tu_fast)"
 #endif
+
+#include "df64.cuh"
+#include "f32x2.cuh"
+#include "f64.cuh"
+#include "fp64_fast.cuh"
 
 namespace weno {
 // Each translation unit compiles its kernels into its own inline namespace, so
@@ -50,7 +51,7 @@ constexpr double kC43 = 13.0 / 3.0;
 // exponent range is ample); float and df64 (float exponent range) take the
 // reciprocal form.
 template <class T>
-constexpr bool is_native_f64 = std::is_same<T, double>::value;
+constexpr bool is_native_f64 = std::is_same<T, f64>::value;
 template <class T>
 constexpr bool is_f32 = std::is_same<T, float>::value;
 
@@ -79,18 +80,39 @@ __device__ __forceinline__ T mul_add(T a, T b, T c) {
 // and equally when held to the FP64 build's 4.
 template <class T, bool FAST>
 __device__ __forceinline__ T cmax(T x, T c) {
-  if constexpr (FAST && is_native_f64<T>) return __double_as_longlong(x) > __double_as_longlong(c) ? x : c;
+  if constexpr (FAST && is_native_f64<T>) return f64_bits(x) > f64_bits(c) ? x : c;
   else return vmax(x, c);
 }
 template <class T, bool FAST>
 __device__ __forceinline__ bool lt_bound(T x, T c) {
-  if constexpr (FAST && is_native_f64<T>) return __double_as_longlong(x) < __double_as_longlong(c);
+  if constexpr (FAST && is_native_f64<T>) return f64_bits(x) < f64_bits(c);
   else return x < c;
 }
 template <class T, bool FAST>
 __device__ __forceinline__ bool gt_zero(T x) {
-  if constexpr (FAST && is_native_f64<T>) return __double_as_longlong(x) > 0;
+  if constexpr (FAST && is_native_f64<T>) return f64_bits(x) > 0;
   else return x > T(0.0);
+}
+
+// x 2^K of the exact forms: an integer operation on an f64's exponent.
+template <int K, class T>
+__device__ __forceinline__ T mul_pow2(T x) {
+  if constexpr (is_native_f64<T>) return T(xscale<K>(x.v));
+  else return x * T(K >= 0 ? (double)(1 << (K >= 0 ? K : 0)) : 1.0 / (double)(1 << (K < 0 ? -K : 0)));
+}
+
+// v[k] and v[k] = x for a run-time k without leaving registers: the exact kernels
+// loop over the four fields (unrolled, their integer divisions would not fit the
+// instruction cache).
+template <class T>
+__device__ __forceinline__ T pick4(const T v[4], int k) {
+  const T a = (k & 1) ? v[1] : v[0], b = (k & 1) ? v[3] : v[2];
+  return (k & 2) ? b : a;
+}
+template <class T>
+__device__ __forceinline__ void put4(T v[4], int k, T x) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = k == i ? x : v[i];
 }
 
 // a / b: the IEEE quotient except in FAST float (the SFU path) and FAST double
@@ -98,18 +120,18 @@ __device__ __forceinline__ bool gt_zero(T x) {
 template <class T, bool FAST>
 __device__ __forceinline__ T qdiv(T a, T b) {
   if constexpr (FAST && is_f32<T>) return __fdividef(a, b);
-  else if constexpr (FAST && is_native_f64<T>) return a * f64fast::rcp(b);
+  else if constexpr (FAST && is_native_f64<T>) return a * T(f64fast::rcp(b.v));
   else return a / b;
 }
 template <class T, bool FAST>
 __device__ __forceinline__ T qrcp(T b) {
   if constexpr (FAST && is_f32<T>) return __fdividef(1.0f, b);
-  else if constexpr (FAST && is_native_f64<T>) return f64fast::rcp(b);
+  else if constexpr (FAST && is_native_f64<T>) return T(f64fast::rcp(b.v));
   else return T(1.0) / b;
 }
 template <class T, bool FAST>
 __device__ __forceinline__ T qsqrt(T x) {
-  if constexpr (FAST && is_native_f64<T>) return f64fast::sqrt(x);
+  if constexpr (FAST && is_native_f64<T>) return T(f64fast::sqrt(x.v));
   else return sqrt(x);
 }
 // 1/sqrt(x) of the FAST forms (x > 0): one reciprocal square root gives sqrt(x)
@@ -118,7 +140,7 @@ __device__ __forceinline__ T qsqrt(T x) {
 // takes 1/sqrt.
 template <class T>
 __device__ __forceinline__ T frsqrt(T x) {
-  if constexpr (is_native_f64<T>) return f64fast::rsqrt(x);
+  if constexpr (is_native_f64<T>) return T(f64fast::rsqrt(x.v));
   else if constexpr (is_f32<T>) return rsqrtf(x);
   else return T(1.0) / sqrt(x);
 }
@@ -133,7 +155,7 @@ __device__ __forceinline__ T frsqrt(T x) {
 // energy has gone negative).
 template <class T>
 __device__ __forceinline__ T sum_prod_rn(T a, T b, T c, T d) {
-  if constexpr (is_native_f64<T>) return __dadd_rn(__dmul_rn(a, b), __dmul_rn(c, d));
+  if constexpr (is_native_f64<T>) return T(xadd(xmul(a.v, b.v), xmul(c.v, d.v)));
   else if constexpr (is_f32<T>) return __fadd_rn(__fmul_rn(a, b), __fmul_rn(c, d));
   else return a * b + c * d;
 }
@@ -147,7 +169,7 @@ __device__ __forceinline__ T sum_prod_rn(T a, T b, T c, T d) {
 template <class T, bool FAST>
 __device__ __forceinline__ T half_rho_speed2(T rho, T m, T n, T u, T v) {
   if constexpr (FAST) return T(0.5) * (m * u + n * v);
-  else return T(0.5) * rho * (u * u + v * v);
+  else return mul_pow2<-1>(rho) * (u * u + v * v);
 }
 
 // Euler flux normal to x (Y = false) or y (Y = true), utils.rs:74-109.  `rinv`
@@ -189,12 +211,12 @@ __device__ __forceinline__ void euler_flux_pair(const T qa[4], const T qb[4], T 
     const T prod = ra * rb;
     T ia, ib;
     if (lt_bound<T, FAST>(prod, T(1e300))) {
-      const T inv = f64fast::rcp2(prod);
+      const T inv = T(f64fast::rcp2(prod.v));
       ia = rb * inv;
       ib = ra * inv;
     } else {
-      ia = f64fast::rcp(ra);
-      ib = f64fast::rcp(rb);
+      ia = T(f64fast::rcp(ra.v));
+      ib = T(f64fast::rcp(rb.v));
     }
     euler_flux<T, FAST, Y>(qa, gamma, fa, ia);
     euler_flux<T, FAST, Y>(qb, gamma, fb, ib);
@@ -218,7 +240,7 @@ __device__ __forceinline__ void con2prim(T q0, T q1, T q2, T q3, T gamma, T& p, 
   } else {
     u = q1 / rho;
     v = q2 / rho;
-    p = vmax((gamma - T(1.0)) * (q3 - T(0.5) * rho * (u * u + v * v)), T(kEps));
+    p = vmax<T>((gamma - T(1.0)) * (q3 - T(0.5) * rho * (u * u + v * v)), T(kEps));
     a = sqrt(gamma * p / rho);
     h = (q3 + p) / rho;
   }
@@ -245,26 +267,28 @@ __device__ __forceinline__ T clamped_pressure(const T q[4], T gamma) {
 // WENO5-JS (weno.rs:214-257) and the 2-point Gauss-quadrature pair
 // (weno.rs:262-303).
 // ---------------------------------------------------------------------------
+// Jiang-Shu indicators of the stencils (u2,u3,u4), (u1,u2,u3), (u0,u1,u2) in the
+// reference's operation order.
 template <class T>
 __device__ __forceinline__ void js_betas(T u0, T u1, T u2, T u3, T u4, T& b0, T& b1, T& b2) {
   T t, s;
-  t = u2 - T(2.0) * u3 + u4;
-  s = T(3.0) * u2 - T(4.0) * u3 + u4;
-  b0 = T(kC13) * (t * t) + T(0.25) * (s * s);
-  t = u1 - T(2.0) * u2 + u3;
+  t = u2 - mul_pow2<1>(u3) + u4;
+  s = T(3.0) * u2 - mul_pow2<2>(u3) + u4;
+  b0 = T(kC13) * (t * t) + mul_pow2<-2>(T(s * s));
+  t = u1 - mul_pow2<1>(u2) + u3;
   s = u1 - u3;
-  b1 = T(kC13) * (t * t) + T(0.25) * (s * s);
-  t = u0 - T(2.0) * u1 + u2;
-  s = u0 - T(4.0) * u1 + T(3.0) * u2;
-  b2 = T(kC13) * (t * t) + T(0.25) * (s * s);
+  b1 = T(kC13) * (t * t) + mul_pow2<-2>(T(s * s));
+  t = u0 - mul_pow2<1>(u1) + u2;
+  s = u0 - mul_pow2<2>(u1) + T(3.0) * u2;
+  b2 = T(kC13) * (t * t) + mul_pow2<-2>(T(s * s));
 }
 
 // Biased exponent of the largest of three positive doubles, from integer
 // operations on the high words (no FP64 slot).
-__device__ __forceinline__ int max_biased_exp3(double a, double b, double c) {
-  const int ea = (__double2hiint(a) >> 20) & 0x7ff;
-  const int eb = (__double2hiint(b) >> 20) & 0x7ff;
-  const int ec = (__double2hiint(c) >> 20) & 0x7ff;
+__device__ __forceinline__ int max_biased_exp3(f64 a, f64 b, f64 c) {
+  const int ea = (__double2hiint(a.v) >> 20) & 0x7ff;
+  const int eb = (__double2hiint(b.v) >> 20) & 0x7ff;
+  const int ec = (__double2hiint(c.v) >> 20) & 0x7ff;
   return max(ea, max(eb, ec));
 }
 
@@ -276,40 +300,51 @@ __device__ __forceinline__ int max_biased_exp3(double a, double b, double c) {
 // the fourth-power products of the WENO5 weights, 120 for the Gauss-point
 // pair, whose shared reciprocal takes an eighth-power product.
 template <int W = 200>
-__device__ __forceinline__ void weno_range(double& e0, double& e1, double& e2) {
+__device__ __forceinline__ void weno_range(f64& e0, f64& e1, f64& e2) {
   const int em = max_biased_exp3(e0, e1, e2);
   if (em >= 1023 - W && em <= 1023 + W) return;
   if (em == 0x7ff || em == 0) return;
   int b = 2045 - em;
   if (b < 1) b = 1;
-  const double sc = __hiloint2double(b << 20, 0);
-  e0 *= sc;
-  e1 *= sc;
-  e2 *= sc;
+  const f64 sc = f64(__hiloint2double(b << 20, 0));
+  e0 = e0 * sc;
+  e1 = e1 * sc;
+  e2 = e2 * sc;
 }
 
-// Non-linear weighting of three candidate values with linear weights d.
-// Exact: the reference's a_k = d_k/(eps+b_k)^2, w_k = a_k/sum.  FAST (float
-// and df64, whose float exponent range rules out products of fourth powers):
-// reciprocals.  FAST native double uses weno_nd instead.
-template <class T, bool FAST>
+// Non-linear weighting of three candidate values with linear weights d in FAST
+// float and df64 (whose float exponent range rules out products of fourth
+// powers): reciprocals.  FAST native double uses weno_nd instead.
+template <class T>
 __device__ __forceinline__ T weno_combine(T e0, T e1, T e2, T d0, T d1, T d2, T p0, T p1, T p2, T scale) {
-  if constexpr (!FAST) {
-    const T a0 = d0 / (e0 * e0);
-    const T a1 = d1 / (e1 * e1);
-    const T a2 = d2 / (e2 * e2);
-    const T sum = a0 + a1 + a2;
-    const T w0 = a0 / sum, w1 = a1 / sum, w2 = a2 / sum;
-    const T r = w0 * p0 + w1 * p1 + w2 * p2;
-    return scale == T(1.0) ? r : r / scale;
-  } else {
-    static_assert(!is_native_f64<T>, "FAST double takes the common-denominator form (weno_nd)");
-    const T a0 = d0 * qrcp<T, FAST>(e0 * e0);
-    const T a1 = d1 * qrcp<T, FAST>(e1 * e1);
-    const T a2 = d2 * qrcp<T, FAST>(e2 * e2);
-    const T num = a0 * p0 + a1 * p1 + a2 * p2;
-    return qdiv<T, FAST>(num, (a0 + a1 + a2) * scale);
+  static_assert(!is_native_f64<T>, "FAST double takes the common-denominator form (weno_nd)");
+  const T a0 = d0 * qrcp<T, true>(e0 * e0);
+  const T a1 = d1 * qrcp<T, true>(e1 * e1);
+  const T a2 = d2 * qrcp<T, true>(e2 * e2);
+  const T num = a0 * p0 + a1 * p1 + a2 * p2;
+  return qdiv<T, true>(num, (a0 + a1 + a2) * scale);
+}
+
+// The exact weights, a_k = d_k/(eps+b_k)^2 and w_k = a_k/sum, applied to the
+// candidates: w0 p0 + w1 p1 + w2 p2.  The three divisions of each kind share
+// one piece of code (a loop): FP64 is the bound, not the latency of one warp,
+// and integer divisions unrolled at every use would not fit the instruction cache.
+template <class T>
+__device__ __forceinline__ T weno_combine_exact(T e0, T e1, T e2, T d0, T d1, T d2, T p0, T p1, T p2) {
+  T a0 = e0 * e0, a1 = e1 * e1, a2 = e2 * e2;
+#pragma unroll 1
+  for (int k = 0; k < 3; ++k) {  // rotates (d, a) so that every k divides the front pair
+    const T q = d0 / a0;
+    a0 = a1, a1 = a2, a2 = q;
+    d0 = d1, d1 = d2;
   }
+  const T sum = a0 + a1 + a2;
+#pragma unroll 1
+  for (int k = 0; k < 3; ++k) {
+    const T w = a0 / sum;
+    a0 = a1, a1 = a2, a2 = w;
+  }
+  return a0 * p0 + a1 * p1 + a2 * p2;
 }
 
 // FAST native double: the weights in a common-denominator form,
@@ -317,10 +352,9 @@ __device__ __forceinline__ T weno_combine(T e0, T e1, T e2, T d0, T d1, T d2, T 
 // a caller can share one divide between two reconstructions; the (eps+b_k)
 // are first brought into a safe range (weno_range), so the products neither
 // overflow nor lose the dominant weight whatever the magnitude of the values.
-__device__ __forceinline__ void weno_nd_products(double e0, double e1, double e2, double& P0, double& P1,
-                                                 double& P2) {
+__device__ __forceinline__ void weno_nd_products(f64 e0, f64 e1, f64 e2, f64& P0, f64& P1, f64& P2) {
   weno_range(e0, e1, e2);
-  const double s0 = e0 * e0, s1 = e1 * e1, s2 = e2 * e2;
+  const f64 s0 = e0 * e0, s1 = e1 * e1, s2 = e2 * e2;
   P0 = s1 * s2;
   P1 = s0 * s2;
   P2 = s0 * s1;
@@ -330,9 +364,9 @@ __device__ __forceinline__ void weno_nd_products(double e0, double e1, double e2
 // operation spelled out: two reconstructions that share the products (the
 // same three stencils seen from both sides of a cell) round exactly as two
 // separate evaluations would.
-__device__ __forceinline__ void weno_nd_combine(double P0, double P1, double P2, double g0, double g1, double g2,
-                                                double& num, double& den) {
-  const double c0 = 3.0 * P0, c1 = 6.0 * P1;
+__device__ __forceinline__ void weno_nd_combine(f64 P0, f64 P1, f64 P2, f64 g0, f64 g1, f64 g2, f64& num,
+                                                f64& den) {
+  const f64 c0 = 3.0 * P0, c1 = 6.0 * P1;
   num = fma(P2, g2, fma(c1, g1, c0 * g0));
   den = (c0 + c1) + P2;
 }
@@ -340,12 +374,11 @@ __device__ __forceinline__ void weno_nd_combine(double P0, double P1, double P2,
 // x = x0 + a/(k b) and y = y0 + c/(k d) with one divide, 1/(k b d), when b d is
 // a normal number well inside the double range (tested on its exponent bits, no
 // FP64 slot); otherwise two divides.
-__device__ __forceinline__ void div_pair(double a, double b, double c, double d, double& x, double& y,
-                                         double k = 1.0, double x0 = 0.0, double y0 = 0.0) {
-  const double bd = b * d;
-  const int e = (__double2hiint(bd) >> 20) & 0x7ff;
+__device__ __forceinline__ void div_pair(f64 a, f64 b, f64 c, f64 d, f64& x, f64& y, f64 k, f64 x0, f64 y0) {
+  const f64 bd = b * d;
+  const int e = (__double2hiint(bd.v) >> 20) & 0x7ff;
   if (e > 64 && e < 1983) {
-    const double inv = f64fast::rcp2(bd * k);  // scales the slopes only
+    const f64 inv = f64(f64fast::rcp2(f64(bd * k).v));  // scales the slopes only
     x = fma(a * d, inv, x0);
     y = fma(c * b, inv, y0);
   } else {
@@ -354,39 +387,32 @@ __device__ __forceinline__ void div_pair(double a, double b, double c, double d,
   }
 }
 
-// weno.rs:214-233 (left-biased, value at the right face of u2)
-template <class T, bool FAST>
-__device__ __forceinline__ T weno5_left(T u0, T u1, T u2, T u3, T u4, T weps) {
-  T b0, b1, b2;
-  js_betas(u0, u1, u2, u3, u4, b0, b1, b2);
-  const T p0 = -u4 + T(5.0) * u3 + T(2.0) * u2;
-  const T p1 = -u1 + T(5.0) * u2 + T(2.0) * u3;
-  const T p2 = T(2.0) * u0 - T(7.0) * u1 + T(11.0) * u2;
-  return weno_combine<T, FAST>(weps + b0, weps + b1, weps + b2, T(0.3), T(0.6), T(0.1), p0, p1, p2, T(6.0));
+// weno.rs:214-257, exact: the left-biased value at the right face of u2 and the
+// right-biased one at the left face of u3, the reference's operations.  The
+// right stencils are the left ones shifted by a cell, so one loop body serves both.
+template <class T>
+__device__ __forceinline__ void weno5_lr_exact(const T u[6], T weps, T& left, T& right) {
+  // candidate polynomials (x6): two are shared by the two sides
+  const T f1 = -u[4] + T(5.0) * u[3] + mul_pow2<1>(u[2]);
+  const T f2 = -u[1] + T(5.0) * u[2] + mul_pow2<1>(u[3]);
+#pragma unroll 1
+  for (int side = 0; side < 2; ++side) {
+    const T v0 = side ? u[1] : u[0], v1 = side ? u[2] : u[1], v2 = side ? u[3] : u[2], v3 = side ? u[4] : u[3],
+            v4 = side ? u[5] : u[4];
+    T b0, b1, b2;
+    js_betas(v0, v1, v2, v3, v4, b0, b1, b2);
+    // 2 u0 - 7 u1 + 11 u2 (left, third candidate), 2 u5 - 7 u4 + 11 u3 (right, first)
+    const T g = mul_pow2<1>(side ? u[5] : u[0]) - T(7.0) * (side ? u[4] : u[1]) + T(11.0) * v2;
+    const T r = weno_combine_exact<T>(weps + b0, weps + b1, weps + b2, side ? T(0.1) : T(0.3), T(0.6),
+                                      side ? T(0.3) : T(0.1), side ? g : f1, side ? f1 : f2, side ? f2 : g) /
+                T(6.0);
+    left = side ? left : r;
+    right = r;
+  }
 }
 
-// weno.rs:238-257 (right-biased, value at the left face of u3)
-template <class T, bool FAST>
-__device__ __forceinline__ T weno5_right(T u1, T u2, T u3, T u4, T u5, T weps) {
-  T b0, b1, b2;
-  T t, s;
-  t = u3 - T(2.0) * u4 + u5;
-  s = T(3.0) * u3 - T(4.0) * u4 + u5;
-  b0 = T(kC13) * (t * t) + T(0.25) * (s * s);
-  t = u2 - T(2.0) * u3 + u4;
-  s = u2 - u4;
-  b1 = T(kC13) * (t * t) + T(0.25) * (s * s);
-  t = u1 - T(2.0) * u2 + u3;
-  s = u1 - T(4.0) * u2 + T(3.0) * u3;
-  b2 = T(kC13) * (t * t) + T(0.25) * (s * s);
-  const T p0 = T(2.0) * u5 - T(7.0) * u4 + T(11.0) * u3;
-  const T p1 = -u4 + T(5.0) * u3 + T(2.0) * u2;
-  const T p2 = -u1 + T(5.0) * u2 + T(2.0) * u3;
-  return weno_combine<T, FAST>(weps + b0, weps + b1, weps + b2, T(0.1), T(0.6), T(0.3), p0, p1, p2, T(6.0));
-}
-
-// weno5_left and weno5_right of one field at one face (the right stencil is
-// the left one shifted by a cell), FAST: native double shares one divide
+// Both reconstructions of one field at one face (the right stencil is the left
+// one shifted by a cell), FAST: native double shares one divide
 // between the two; float and df64 take reciprocal weights.
 template <class T>
 __device__ __forceinline__ void weno5_lr_fast(T u0, T u1, T u2, T u3, T u4, T u5, T weps, T& left, T& right) {
@@ -417,15 +443,15 @@ __device__ __forceinline__ void weno5_lr_fast(T u0, T u1, T u2, T u3, T u4, T u5
   if constexpr (is_native_f64<T>) {
     // linear weights scaled by 10 -- (3, 6, 1) -- and the 1/6 of the candidate
     // polynomials applied once to the shared divide
-    double P0, P1, P2, nl, dl, nr, dr;
+    f64 P0, P1, P2, nl, dl, nr, dr;
     weno_nd_products(el0, el1, el2, P0, P1, P2);
     weno_nd_combine(P0, P1, P2, gl0, gl1, gl2, nl, dl);
     weno_nd_products(er2, er1, er0, P0, P1, P2);
     weno_nd_combine(P0, P1, P2, gr2, gr1, gr0, nr, dr);
     div_pair(nl, dl, nr, dr, left, right, 6.0, u2, u3);
   } else {
-    left = u2 + weno_combine<T, true>(el0, el1, el2, T(0.3), T(0.6), T(0.1), gl0, gl1, gl2, T(6.0));
-    right = u3 + weno_combine<T, true>(er2, er1, er0, T(0.3), T(0.6), T(0.1), gr2, gr1, gr0, T(6.0));
+    left = u2 + weno_combine<T>(el0, el1, el2, T(0.3), T(0.6), T(0.1), gl0, gl1, gl2, T(6.0));
+    right = u3 + weno_combine<T>(er2, er1, er0, T(0.3), T(0.6), T(0.1), gr2, gr1, gr0, T(6.0));
   }
 }
 
@@ -437,27 +463,26 @@ __device__ __forceinline__ void weno5_lr_fast(T u0, T u1, T u2, T u3, T u4, T u5
 // operations weno5_lr_fast performs for each face on its own, so A and B get
 // the bits of two separate calls (the component-wise pass 1 of the FAST
 // double solver).
-__device__ __forceinline__ void weno5_lr_fast_two(double u0, double u1, double u2, double u3, double u4, double u5,
-                                                  double u6, double weps, double& lA, double& rA, double& lB,
-                                                  double& rB) {
-  const double d0 = u1 - u0, d1 = u2 - u1, d2 = u3 - u2, d3 = u4 - u3, d4 = u5 - u4, d5 = u6 - u5;
-  const double D1 = d1 - d0, D2 = d2 - d1, D3 = d3 - d2, D4 = d4 - d3, D5 = d5 - d4;
-  const double w4 = 4.0 * weps;
-  const double C1 = kC43 * D1 * D1 + w4, C2 = kC43 * D2 * D2 + w4, C3 = kC43 * D3 * D3 + w4,
+__device__ __forceinline__ void weno5_lr_fast_two(f64 u0, f64 u1, f64 u2, f64 u3, f64 u4, f64 u5, f64 u6, f64 weps,
+                                                  f64& lA, f64& rA, f64& lB, f64& rB) {
+  const f64 d0 = u1 - u0, d1 = u2 - u1, d2 = u3 - u2, d3 = u4 - u3, d4 = u5 - u4, d5 = u6 - u5;
+  const f64 D1 = d1 - d0, D2 = d2 - d1, D3 = d3 - d2, D4 = d4 - d3, D5 = d5 - d4;
+  const f64 w4 = 4.0 * weps;
+  const f64 C1 = kC43 * D1 * D1 + w4, C2 = kC43 * D2 * D2 + w4, C3 = kC43 * D3 * D3 + w4,
                C4 = kC43 * D4 * D4 + w4, C5 = kC43 * D5 * D5 + w4;
   // face A: as weno5_lr_fast(u0..u5)
-  const double sl0 = d3 - 3.0 * d2, sl1 = d1 + d2, sl2 = 3.0 * d1 - d0;
-  const double sr0 = d4 - 3.0 * d3, sr1 = d2 + d3, sr2 = 3.0 * d2 - d1;
-  const double el0 = sl0 * sl0 + C3, el1 = sl1 * sl1 + C2, el2 = sl2 * sl2 + C1;
-  const double er0 = sr0 * sr0 + C4, er1 = sr1 * sr1 + C3, er2 = sr2 * sr2 + C2;
-  const double gl0 = d2 - sl0, gl1 = sl1 + d2, gl2 = 2.0 * sl2 - d1;
-  const double gr2 = -d2 - sr2, gr1 = -d2 - sr1, gr0 = 2.0 * sr0 + d3;
+  const f64 sl0 = d3 - 3.0 * d2, sl1 = d1 + d2, sl2 = 3.0 * d1 - d0;
+  const f64 sr0 = d4 - 3.0 * d3, sr1 = d2 + d3, sr2 = 3.0 * d2 - d1;
+  const f64 el0 = sl0 * sl0 + C3, el1 = sl1 * sl1 + C2, el2 = sl2 * sl2 + C1;
+  const f64 er0 = sr0 * sr0 + C4, er1 = sr1 * sr1 + C3, er2 = sr2 * sr2 + C2;
+  const f64 gl0 = d2 - sl0, gl1 = sl1 + d2, gl2 = 2.0 * sl2 - d1;
+  const f64 gr2 = -d2 - sr2, gr1 = -d2 - sr1, gr0 = 2.0 * sr0 + d3;
   // face B: as weno5_lr_fast(u1..u6); its left stencils and indicators are A's right ones
-  const double tr0 = d5 - 3.0 * d4, tr1 = d3 + d4, tr2 = 3.0 * d3 - d2;
-  const double fr0 = tr0 * tr0 + C5, fr1 = tr1 * tr1 + C4, fr2 = tr2 * tr2 + C3;
-  const double hl0 = d3 - sr0, hl1 = sr1 + d3, hl2 = 2.0 * sr2 - d2;
-  const double hr2 = -d3 - tr2, hr1 = -d3 - tr1, hr0 = 2.0 * tr0 + d4;
-  double P0, P1, P2, nl, dl, nr, dr;
+  const f64 tr0 = d5 - 3.0 * d4, tr1 = d3 + d4, tr2 = 3.0 * d3 - d2;
+  const f64 fr0 = tr0 * tr0 + C5, fr1 = tr1 * tr1 + C4, fr2 = tr2 * tr2 + C3;
+  const f64 hl0 = d3 - sr0, hl1 = sr1 + d3, hl2 = 2.0 * sr2 - d2;
+  const f64 hr2 = -d3 - tr2, hr1 = -d3 - tr1, hr0 = 2.0 * tr0 + d4;
+  f64 P0, P1, P2, nl, dl, nr, dr;
   weno_nd_products(el0, el1, el2, P0, P1, P2);
   weno_nd_combine(P0, P1, P2, gl0, gl1, gl2, nl, dl);
   weno_nd_products(er2, er1, er0, P0, P1, P2);
@@ -498,14 +523,14 @@ __device__ __forceinline__ void gq_weights(T q2, T h0, T h1, T h2, T f0, T f1, T
   const T S = T(kSqrt3_12);
   if constexpr (is_native_f64<T>) {
     weno_range<120>(f0, f1, f2);
-    const double s0 = f0 * f0, s1 = f1 * f1, s2 = f2 * f2;
-    const double P0 = s1 * s2, P1 = s0 * s2, P2 = s0 * s1;
+    const f64 s0 = f0 * f0, s1 = f1 * f1, s2 = f2 * f2;
+    const f64 P0 = s1 * s2, P1 = s0 * s2, P2 = s0 * s1;
     // linear weights divided by the centre one (a common factor): point a
     // weighs (r0 P0, P1, r2 P2), point b the mirror (r2 P0, P1, r0 P2)
     constexpr double r0 = kGqA0 / kGqA1, r2 = kGqA2 / kGqA1;
-    const double u0 = P0 * h0, u1 = P1 * h1, u2 = P2 * h2;
-    const double sa = fma(r0, P0, fma(r2, P2, P1)), sb = fma(r2, P0, fma(r0, P2, P1));
-    const double t = S * f64fast::rcp2(sa * sb);  // scales the weighted slopes only
+    const f64 u0 = P0 * h0, u1 = P1 * h1, u2 = P2 * h2;
+    const f64 sa = fma(r0, P0, fma(r2, P2, P1)), sb = fma(r2, P0, fma(r0, P2, P1));
+    const f64 t = S * f64(f64fast::rcp2(f64(sa * sb).v));  // scales the weighted slopes only
     // point a: candidates (q2 + S h0, q2 - S h1, q2 - S h2); point b: the mirror
     ra = fma(r0, u0, fma(-r2, u2, -u1)) * (sb * t) + q2;
     rb = fma(r0, u2, fma(-r2, u0, u1)) * (sa * t) + q2;
@@ -555,16 +580,18 @@ __device__ __forceinline__ void weno5_gq_pair(T q0, T q1, T q2, T q3, T q4, T& r
     T b0, b1, b2;
     js_betas(q0, q1, q2, q3, q4, b0, b1, b2);
     const T e0 = weps + b0, e1 = weps + b1, e2 = weps + b2;
-    const T g0 = T(3.0) * q2 - T(4.0) * q3 + q4;
-    const T g2 = T(3.0) * q2 - T(4.0) * q1 + q0;
-    const T pa0 = q2 + g0 * S;
-    const T pa1 = q2 - (-q1 + q3) * S;
-    const T pa2 = q2 - g2 * S;
-    ra = weno_combine<T, FAST>(e0, e1, e2, T(kGqA0), T(kGqA1), T(kGqA2), pa0, pa1, pa2, T(1.0));
-    const T pb0 = q2 - g0 * S;
-    const T pb1 = q2 - (q1 - q3) * S;
-    const T pb2 = q2 + g2 * S;
-    rb = weno_combine<T, FAST>(e0, e1, e2, T(kGqA2), T(kGqA1), T(kGqA0), pb0, pb1, pb2, T(1.0));
+    const T g0 = (T(3.0) * q2 - mul_pow2<2>(q3) + q4) * S;
+    const T g2 = (T(3.0) * q2 - mul_pow2<2>(q1) + q0) * S;
+    // point a: q2 + g0, q2 - (q3 - q1) S, q2 - g2; point b: the mirror (negation
+    // is exact: -q1 + q3 and q1 - q3 are opposite)
+    const T g1 = (-q1 + q3) * S;
+#pragma unroll 1
+    for (int pt = 0; pt < 2; ++pt) {
+      const T r = weno_combine_exact<T>(e0, e1, e2, pt ? T(kGqA2) : T(kGqA0), T(kGqA1), pt ? T(kGqA0) : T(kGqA2),
+                                        q2 + (pt ? -g0 : g0), q2 - (pt ? -g1 : g1), q2 - (pt ? -g2 : g2));
+      ra = pt ? ra : r;
+      rb = r;
+    }
   }
 }
 
@@ -587,7 +614,7 @@ __device__ __forceinline__ RoeSide<T> roe_side(const T u[4], T gamma) {
   s.sq = rho * s.r;
   s.i = s.r * s.r;
   // kinetic energy (m^2 + n^2) / (2 rho): the velocities themselves are not needed
-  const T p = vmax((gamma - T(1.0)) * (u[3] - T(0.5) * ((u[1] * u[1] + u[2] * u[2]) * s.i)), T(kEps));
+  const T p = vmax<T>((gamma - T(1.0)) * (u[3] - T(0.5) * ((u[1] * u[1] + u[2] * u[2]) * s.i)), T(kEps));
   s.a = u[1] * s.r;
   s.b = u[2] * s.r;
   s.ep = u[3] + p;
@@ -601,11 +628,11 @@ template <class T>
 __device__ __forceinline__ void roe_face(const RoeSide<T>& L, const RoeSide<T>& R, T m_l, T n_l, T gamma,
                                          T& rho_roe, T& u_roe, T& v_roe, T& h_roe, T& c_roe, T& ic, T& irho) {
   const T id = qrcp<T, true>(L.sq + R.sq);
-  u_roe = mul_add(m_l, L.r, R.a) * id;
-  v_roe = mul_add(n_l, L.r, R.b) * id;
-  h_roe = mul_add(L.ep, L.r, R.ep * R.r) * id;
+  u_roe = mul_add<T>(m_l, L.r, R.a) * id;
+  v_roe = mul_add<T>(n_l, L.r, R.b) * id;
+  h_roe = mul_add<T>(L.ep, L.r, R.ep * R.r) * id;
   const T kin = T(0.5) * (u_roe * u_roe + v_roe * v_roe);
-  const T c2 = vmax((gamma - T(1.0)) * (h_roe - kin), T(kEps) * vmax(L.i, R.i));
+  const T c2 = vmax<T>((gamma - T(1.0)) * (h_roe - kin), T(kEps) * vmax<T>(L.i, R.i));
   ic = frsqrt(c2);
   c_roe = c2 * ic;
   rho_roe = L.sq * R.sq;
@@ -631,15 +658,15 @@ __device__ __forceinline__ void roe_avg(const T ul[4], const T ur[4], T gamma, T
     const T denom = sqrt_l + sqrt_r;
     const T u_l = ul[1] / rho_l, v_l = ul[2] / rho_l;
     const T u_r = ur[1] / rho_r, v_r = ur[2] / rho_r;
-    const T p_l = vmax((gamma - T(1.0)) * (ul[3] - T(0.5) * rho_l * (u_l * u_l + v_l * v_l)), T(kEps));
-    const T p_r = vmax((gamma - T(1.0)) * (ur[3] - T(0.5) * rho_r * (u_r * u_r + v_r * v_r)), T(kEps));
+    const T p_l = vmax<T>((gamma - T(1.0)) * (ul[3] - T(0.5) * rho_l * (u_l * u_l + v_l * v_l)), T(kEps));
+    const T p_r = vmax<T>((gamma - T(1.0)) * (ur[3] - T(0.5) * rho_r * (u_r * u_r + v_r * v_r)), T(kEps));
     const T h_l = (ul[3] + p_l) / rho_l;
     const T h_r = (ur[3] + p_r) / rho_r;
     u_roe = (sqrt_l * u_l + sqrt_r * u_r) / denom;
     v_roe = (sqrt_l * v_l + sqrt_r * v_r) / denom;
     h_roe = (sqrt_l * h_l + sqrt_r * h_r) / denom;
     const T kin = T(0.5) * (u_roe * u_roe + v_roe * v_roe);
-    const T c2 = vmax((gamma - T(1.0)) * (h_roe - kin), T(kEps) / vmin(rho_l, rho_r));
+    const T c2 = vmax<T>((gamma - T(1.0)) * (h_roe - kin), T(kEps) / vmin(rho_l, rho_r));
     c_roe = sqrt(c2);
     rho_roe = sqrt_l * sqrt_r;
   }
@@ -655,11 +682,11 @@ __device__ __forceinline__ void left_eig(T rho, T u, T v, T c, T gamma, T L[4][4
   const T rc = rho * c;
   const T inv_rc = T(1.0) / rc;
   const T inv_c2 = T(1.0) / (c * c);
-  const T a = g1 * kin / (T(2.0) * c * c);
-  const T b = vn / (T(2.0) * c);
-  const T gu = -g1 * u * inv_c2 / T(2.0);
-  const T gv = -g1 * v * inv_c2 / T(2.0);
-  const T gg = g1 * inv_c2 / T(2.0);
+  const T a = g1 * kin / (mul_pow2<1>(c) * c);
+  const T b = vn / mul_pow2<1>(c);
+  const T gu = mul_pow2<-1>(T(-g1 * u * inv_c2));
+  const T gv = mul_pow2<-1>(T(-g1 * v * inv_c2));
+  const T gg = mul_pow2<-1>(T(g1 * inv_c2));
   const T hr = T(0.5) * inv_rc;
   L[0][0] = a + b;
   L[3][0] = a - b;
@@ -696,15 +723,23 @@ __device__ __forceinline__ void right_eig(T rho, T u, T v, T h, T c, T R[4][4]) 
 
 // weno.rs:197-205 mat4_vec4: every product accumulated from 0.0 in column
 // order, as the reference does (FAST callers use project_left / project_right).
+// 0.0 + x is x except for x = -0, which becomes +0: an integer select.
+template <class T>
+__device__ __forceinline__ T from_zero(T x) {
+  if constexpr (is_native_f64<T>) return f64_bits(x) == (long long)0x8000000000000000ull ? T(0.0) : x;
+  else return T(0.0) + x;
+}
+template <class T>
+__device__ __forceinline__ T row_vec4(const T row[4], const T x[4]) {
+  T acc = from_zero<T>(row[0] * x[0]);
+#pragma unroll
+  for (int c = 1; c < 4; ++c) acc = acc + row[c] * x[c];
+  return acc;
+}
 template <class T>
 __device__ __forceinline__ void mat4_vec4(const T M[4][4], const T x[4], T out[4]) {
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    T acc = T(0.0);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) acc = acc + M[r][c] * x[c];
-    out[r] = acc;
-  }
+  for (int r = 0; r < 4; ++r) out[r] = row_vec4<T>(M[r], x);
 }
 
 // FAST products with the eigenvector matrices of weno.rs:76-189, written from
@@ -759,7 +794,7 @@ template <class T, bool FAST>
 __device__ __forceinline__ void pp_limit(T q[4], const T ub[4], T gamma) {
   if (q[0] < T(kEps)) {
     const T rho_bar = vmax(ub[0], T(kEps));
-    const T theta = vmax(vmin(qdiv<T, FAST>(rho_bar - T(kEps), rho_bar - q[0]), T(1.0)), T(0.0));
+    const T theta = vmax<T>(vmin<T>(qdiv<T, FAST>(rho_bar - T(kEps), rho_bar - q[0]), T(1.0)), T(0.0));
 #pragma unroll
     for (int k = 0; k < 4; ++k) q[k] = theta * (q[k] - ub[k]) + ub[k];
   }
@@ -772,8 +807,8 @@ __device__ __forceinline__ void pp_limit(T q[4], const T ub[4], T gamma) {
   }
   const T p_q = pp_pressure<T, FAST>(q, gamma);
   if (p_q < T(kEps)) {
-    const T p_bar = vmax(pp_pressure<T, FAST>(ub, gamma), T(kEps));
-    const T theta = vmax(vmin(qdiv<T, FAST>(p_bar - T(kEps), p_bar - p_q), T(1.0)), T(0.0));
+    const T p_bar = vmax<T>(pp_pressure<T, FAST>(ub, gamma), T(kEps));
+    const T theta = vmax<T>(vmin<T>(qdiv<T, FAST>(p_bar - T(kEps), p_bar - p_q), T(1.0)), T(0.0));
 #pragma unroll
     for (int k = 0; k < 4; ++k) q[k] = theta * (q[k] - ub[k]) + ub[k];
   }
@@ -788,15 +823,19 @@ template <class T, bool FAST, bool Y, bool CHAR>
 __device__ __forceinline__ void pass1_face(const T c[6][4], T gamma, T ql[4], T qr[4], T weps) {
   if constexpr (!CHAR && FAST && is_f32<T>) {
     weno5_lr_fast_f32_pairs(c, weps, ql, qr, weps);
-  } else if constexpr (!CHAR) {
+  } else if constexpr (!CHAR && FAST) {
 #pragma unroll
+    for (int k = 0; k < 4; ++k)
+      weno5_lr_fast<T>(c[0][k], c[1][k], c[2][k], c[3][k], c[4][k], c[5][k], weps, ql[k], qr[k]);
+  } else if constexpr (!CHAR) {
+#pragma unroll 1
     for (int k = 0; k < 4; ++k) {
-      if constexpr (FAST) {
-        weno5_lr_fast<T>(c[0][k], c[1][k], c[2][k], c[3][k], c[4][k], c[5][k], weps, ql[k], qr[k]);
-      } else {
-        ql[k] = weno5_left<T, FAST>(c[0][k], c[1][k], c[2][k], c[3][k], c[4][k], weps);
-        qr[k] = weno5_right<T, FAST>(c[1][k], c[2][k], c[3][k], c[4][k], c[5][k], weps);
-      }
+      T u[6], l, r;
+#pragma unroll
+      for (int s = 0; s < 6; ++s) u[s] = pick4(c[s], k);
+      weno5_lr_exact<T>(u, weps, l, r);
+      put4(ql, k, l);
+      put4(qr, k, r);
     }
   } else {
     T rho_a, u_a, v_a, h_a, c_a, ic_a = T(0.0), irho_a = T(0.0);
@@ -804,9 +843,9 @@ __device__ __forceinline__ void pass1_face(const T c[6][4], T gamma, T ql[4], T 
     // The reference projects cells 0..4 for the left state and 1..5 for the
     // right state with the same matrix (both faces use the Roe average of
     // cells 2|3), so six projections cover both.
-    T w[6][4];
     T chl[4], chr[4];
     if constexpr (FAST) {
+      T w[6][4];
       CharScalars<T> k;
       k.u = u_a;
       k.v = v_a;
@@ -835,12 +874,19 @@ __device__ __forceinline__ void pass1_face(const T c[6][4], T gamma, T ql[4], T 
     } else {
       T Lm[4][4];
       left_eig<T, Y>(rho_a, u_a, v_a, c_a, gamma, Lm);
-#pragma unroll
-      for (int s = 0; s < 6; ++s) mat4_vec4<T>(Lm, c[s], w[s]);
-#pragma unroll
+#pragma unroll 1
       for (int f = 0; f < 4; ++f) {
-        chl[f] = weno5_left<T, FAST>(w[0][f], w[1][f], w[2][f], w[3][f], w[4][f], weps);
-        chr[f] = weno5_right<T, FAST>(w[1][f], w[2][f], w[3][f], w[4][f], w[5][f], weps);
+        // characteristic field f of the six cells: row f of L times the cells
+        const T row[4] = {f < 2 ? (f == 0 ? Lm[0][0] : Lm[1][0]) : (f == 2 ? Lm[2][0] : Lm[3][0]),
+                          f < 2 ? (f == 0 ? Lm[0][1] : Lm[1][1]) : (f == 2 ? Lm[2][1] : Lm[3][1]),
+                          f < 2 ? (f == 0 ? Lm[0][2] : Lm[1][2]) : (f == 2 ? Lm[2][2] : Lm[3][2]),
+                          f < 2 ? (f == 0 ? Lm[0][3] : Lm[1][3]) : (f == 2 ? Lm[2][3] : Lm[3][3])};
+        T w[6], l, r;
+#pragma unroll
+        for (int s = 0; s < 6; ++s) w[s] = row_vec4<T>(row, c[s]);
+        weno5_lr_exact<T>(w, weps, l, r);
+        put4(chl, f, l);
+        put4(chr, f, r);
       }
       T Rm[4][4];
       right_eig<T, Y>(rho_a, u_a, v_a, h_a, c_a, Rm);
@@ -923,7 +969,7 @@ template <class T, bool FAST>
 __device__ __forceinline__ T guard_denom(T d) {
   bool small;
   if constexpr (FAST && is_native_f64<T>)
-    small = (__double_as_longlong(d) & 0x7fffffffffffffffLL) < __double_as_longlong(kEps);
+    small = (f64_bits(d) & 0x7fffffffffffffffLL) < __double_as_longlong(kEps);
   else
     small = fabs(d) < T(kEps);
   if (small) d = copysign(T(kEps), d) + T(kEps);
@@ -948,7 +994,12 @@ __device__ __forceinline__ void hlle_flux(const RiemannPre<T, FAST, Y>& r, const
     const T srsl = r.s_r * r.s_l;
     if constexpr (!FAST) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) F[k] = (r.s_r * fl[k] - r.s_l * fr[k] + srsl * (qrv[k] - qlv[k])) / denom;
+      for (int k = 0; k < 4; ++k) F[k] = r.s_r * fl[k] - r.s_l * fr[k] + srsl * (qrv[k] - qlv[k]);
+#pragma unroll 1
+      for (int k = 0; k < 4; ++k) {  // one division in the code, F rotating past it
+        const T f = F[0] / denom;
+        F[0] = F[1], F[1] = F[2], F[2] = F[3], F[3] = f;
+      }
     } else {
       const T id = qrcp<T, FAST>(S == 1 ? denom : T(S) * denom);
 #pragma unroll

@@ -33,6 +33,8 @@
 
 #include <cuda_runtime.h>
 
+#include "opaque64.cuh"
+
 namespace weno {
 namespace f64fast {
 
@@ -92,8 +94,8 @@ __device__ __forceinline__ double rsqrt_core(int hi, int lo) {
   const int odd = e2 & 1;
   const double m = __hiloint2double((hi & 0x000fffff) | ((1023 + odd) << 20), lo);
   const double y0 = widen(rsqrt_approx(narrow(hi, lo, 127u + (unsigned)odd)));
-  const double e = fma(-m, y0 * y0, 1.0);
-  const double y = fma(y0 * e, fma(0.375, e, 0.5), y0);  // in [0.5, 1]
+  const double e = fma(-m, xmul(y0, y0), 1.0);
+  const double y = fma(xmul(y0, e), fma(0.375, e, 0.5), y0);  // in [0.5, 1]
   const int yh = __double2hiint(y) - ((e2 - odd) / 2) * (1 << 20);
   return __hiloint2double(yh, __double2loint(y));
 }
@@ -123,7 +125,7 @@ __device__ __forceinline__ double sqrt(double x) {
   const int hi = __double2hiint(x), lo = __double2loint(x);
   const int ex = biased_exp(hi);
   if (hi < 0 || ex < kExpLo || ex > kExpHi) return ::sqrt(x);
-  return x * rsqrt_core(hi, lo);
+  return xmul(x, rsqrt_core(hi, lo));
 }
 
 }  // namespace f64fast

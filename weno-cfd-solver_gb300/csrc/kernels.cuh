@@ -68,16 +68,16 @@ __global__ void __launch_bounds__(128) k_pass1(CView<T> u, int64_t rows, int64_t
     if (safe) {
       pass1_face<T, FAST, Y, CHAR>(c, gamma, ql, qr, weps);
     } else {
-      double cd[6][4], l[4], r[4];
+      f64 cd[6][4], l[4], r[4];
 #pragma unroll
       for (int s = 0; s < 6; ++s)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) cd[s][k] = (double)c[s][k];
-      pass1_face<double, FAST, Y, CHAR>(cd, (double)gamma, l, r, (double)weps);
+        for (int k = 0; k < 4; ++k) cd[s][k] = f64((double)c[s][k]);
+      pass1_face<f64, FAST, Y, CHAR>(cd, f64((double)gamma), l, r, f64((double)weps));
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        ql[k] = T(l[k]);
-        qr[k] = T(r[k]);
+        ql[k] = T(l[k].v);
+        qr[k] = T(r[k].v);
       }
     }
   } else {
@@ -95,8 +95,8 @@ __global__ void __launch_bounds__(128) k_pass1(CView<T> u, int64_t rows, int64_t
 // reconstructions about the middle cell serve both (weno5_lr_fast_two; the
 // same bits as one face per thread).
 template <bool Y>
-__global__ void __launch_bounds__(128) k_pass1_cons2(CView<double> u, int64_t rows, int64_t cols,
-                                                      Planes<double> PL, Planes<double> PR, double weps) {
+__global__ void __launch_bounds__(128) k_pass1_cons2(CView<f64> u, int64_t rows, int64_t cols, Planes<f64> PL,
+                                                      Planes<f64> PR, f64 weps) {
   int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t row = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;
   if constexpr (Y) col *= 2;
@@ -106,12 +106,12 @@ __global__ void __launch_bounds__(128) k_pass1_cons2(CView<double> u, int64_t ro
   const int64_t rowB = Y ? row : row + 1, colB = Y ? col + 1 : col;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    double v[7];
+    f64 v[7];
 #pragma unroll
     for (int s = 0; s < 6; ++s) v[s] = Y ? u.at(row, col + s, k) : u.at(row + s, col, k);
     // the seventh cell exists only when face B does
     v[6] = two ? (Y ? u.at(row, col + 6, k) : u.at(row + 6, col, k)) : v[5];
-    double lA, rA, lB, rB;
+    f64 lA, rA, lB, rB;
     weno5_lr_fast_two(v[0], v[1], v[2], v[3], v[4], v[5], v[6], weps, lA, rA, lB, rB);
     PL.at(k, row, col) = lA;
     PR.at(k, row, col) = rA;
@@ -141,12 +141,14 @@ struct Pass2Dst {
 
 template <class T, bool FAST, bool Y>
 __device__ __forceinline__ void gq_face(const Planes<T>& P, int64_t row, int64_t col, T q1[4], T q2[4], T weps) {
-#pragma unroll
+#pragma unroll(FAST ? 4 : 1)
   for (int k = 0; k < 4; ++k) {
-    T s[5];
+    T s[5], a, b;
 #pragma unroll
     for (int t = 0; t < 5; ++t) s[t] = Y ? P.at(k, row + 1 + t, col) : P.at(k, row, col + 1 + t);
-    weno5_gq_pair<T, FAST>(s[0], s[1], s[2], s[3], s[4], q1[k], q2[k], weps);
+    weno5_gq_pair<T, FAST>(s[0], s[1], s[2], s[3], s[4], a, b, weps);
+    put4(q1, k, a);
+    put4(q2, k, b);
   }
 }
 
@@ -195,21 +197,19 @@ __global__ void __launch_bounds__(128) k_pass2(Planes<T> PL, Planes<T> PR, int64
   const int64_t row = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;
   if (row >= rows || col >= cols) return;
   T ql[4], qr[4], fl[4], fr[4];
-  {
+#pragma unroll(FAST ? 2 : 1)
+  for (int side = 0; side < 2; ++side) {
     T a1[4], a2[4], f1[4], f2[4];
-    gq_face<T, FAST, Y>(PL, row, col, a1, a2, weps);
+    const Planes<T> P{side ? PR.p : PL.p, PL.ps, PL.ld};
+    gq_face<T, FAST, Y>(P, row, col, a1, a2, weps);
     euler_flux_pair<T, FAST, Y>(a1, a2, gamma, f1, f2);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      fl[k] = T(0.5) * (f1[k] + f2[k]);
-      ql[k] = T(0.5) * (a1[k] + a2[k]);
-    }
-    gq_face<T, FAST, Y>(PR, row, col, a1, a2, weps);
-    euler_flux_pair<T, FAST, Y>(a1, a2, gamma, f1, f2);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      fr[k] = T(0.5) * (f2[k] + f1[k]);
-      qr[k] = T(0.5) * (a1[k] + a2[k]);
+      const T f = mul_pow2<-1>(T(f1[k] + f2[k])), q = mul_pow2<-1>(T(a1[k] + a2[k]));
+      fl[k] = side ? fl[k] : f;
+      ql[k] = side ? ql[k] : q;
+      fr[k] = f;
+      qr[k] = q;
     }
   }
   pass2_emit<T, FAST, Y, OUT>(ql, fl, qr, fr, gamma, dst, row, col, cols);
@@ -509,24 +509,22 @@ __global__ void k_bc_dmr(S3<T> Q, int64_t nx, int64_t ny, int64_t bound, Post8<T
 // AOS = true reads the primitives from channels 5, 6, 7 of a (M, N, C>=8)
 // array instead (the first step of a run starting from the driver's array).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void atomic_max_nonneg(unsigned long long* a, double x) {
-  atomicMax(a, (unsigned long long)__double_as_longlong(x));
-}
-
 // np.maximum(rho, 1e-14) of the driver's CFL (Rie_prob_2d_rs.py:314): NaN in,
 // NaN out (fmax would return the bound).
 template <class T>
 __device__ __forceinline__ T np_maximum(T x, T c) { return x != x ? x : fmax(x, c); }
 
 // np.max propagates NaN (and inf dominates), so a non-finite wave speed makes
-// the maximum non-finite and dt follows, as in the driver; NaN's bit pattern
-// orders above +inf under the unsigned atomicMax.
-__device__ __forceinline__ double nan_max(double a, double b) { return (a != a || b != b) ? __longlong_as_double(0x7ff8000000000000ll) : fmax(a, b); }
+// the maximum non-finite and dt follows, as in the driver.  The speeds are
+// non-negative or NaN (of either sign), so the maximum is one of unsigned
+// integers: NaN's bits order above +inf's.
+__device__ __forceinline__ unsigned long long max_bits(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
+__device__ __forceinline__ unsigned long long speed_bits(double x) { return (unsigned long long)__double_as_longlong(x); }
 
 template <class T, bool AOS>
 __global__ void __launch_bounds__(256) k_cfl_max(CView<T> q, int64_t nx, int64_t ny, T gamma, StepCtl* ctl) {
   if (!ctl->active || ctl->cmax_preset) return;
-  double best = 0.0;
+  unsigned long long best = 0;
   bool nonpos = false;  // FP64 positivity check of the recovered density and pressure
   const int64_t total = nx * ny;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
@@ -543,38 +541,38 @@ __global__ void __launch_bounds__(256) k_cfl_max(CView<T> q, int64_t nx, int64_t
       const float uu = m1 * ir, vv = m2 * ir;
       const float pp = fmaxf(((float)gamma - 1.0f) * (E - 0.5f * rho * (uu * uu + vv * vv)), float(kEps));
       const float w = sqrtf(uu * uu + vv * vv) + sqrtf((float)gamma * pp * __fdividef(1.0f, np_maximum(r0, 1e-14f)));
-      best = nan_max(best, (double)w);
+      best = max_bits(best, speed_bits((double)w));
     } else {
-      double uu, vv, pp;
-      const double r0 = (double)q.at(i, j, 0);
+      const f64 g((double)gamma), r0((double)q.at(i, j, 0));
+      f64 uu, vv, pp;
       if constexpr (AOS) {
-        uu = (double)q.at(i, j, 5);
-        vv = (double)q.at(i, j, 6);
-        pp = (double)q.at(i, j, 7);
+        uu = f64((double)q.at(i, j, 5));
+        vv = f64((double)q.at(i, j, 6));
+        pp = f64((double)q.at(i, j, 7));
       } else {
-        const double rho = fmax(r0, kEps);
-        uu = (double)q.at(i, j, 1) / rho;
-        vv = (double)q.at(i, j, 2) / rho;
-        const double praw = ((double)gamma - 1.0) * ((double)q.at(i, j, 3) - 0.5 * rho * (uu * uu + vv * vv));
-        pp = fmax(praw, kEps);
-        if (!(r0 > 0.0) || !(praw > 0.0)) nonpos = true;
+        const f64 rho = fmax(r0, f64(kEps));
+        uu = f64((double)q.at(i, j, 1)) / rho;
+        vv = f64((double)q.at(i, j, 2)) / rho;
+        const f64 praw = (g - f64(1.0)) * (f64((double)q.at(i, j, 3)) - f64(0.5) * rho * (uu * uu + vv * vv));
+        pp = fmax(praw, f64(kEps));
+        if (!(r0 > f64(0.0)) || !(praw > f64(0.0))) nonpos = true;
       }
-      const double speed = sqrt(uu * uu + vv * vv);
-      const double c = sqrt((double)gamma * pp / np_maximum(r0, 1e-14));
-      best = nan_max(best, c + speed);
+      const f64 speed = sqrt(uu * uu + vv * vv);
+      const f64 c = sqrt(g * pp / np_maximum(r0, f64(1e-14)));
+      best = max_bits(best, speed_bits((c + speed).v));
     }
   }
   nonpos = __any_sync(0xffffffffu, nonpos);
   if (nonpos && (threadIdx.x & 31) == 0) atomicOr(&ctl->status, 2);
-  for (int off = 16; off > 0; off >>= 1) best = nan_max(best, __shfl_xor_sync(0xffffffffu, best, off));
-  __shared__ double sm[8];
+  for (int off = 16; off > 0; off >>= 1) best = max_bits(best, __shfl_xor_sync(0xffffffffu, best, off));
+  __shared__ unsigned long long sm[8];
   if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = best;
   __syncthreads();
   if (threadIdx.x == 0) {
-    double b = sm[0];
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) b = nan_max(b, sm[w]);
-    atomic_max_nonneg(&ctl->cmax_bits, b);
-    if (!(b < INFINITY)) atomicOr(&ctl->status, 1);
+    unsigned long long b = sm[0];
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) b = max_bits(b, sm[w]);
+    atomicMax(&ctl->cmax_bits, b);
+    if (b >= 0x7ff0000000000000ull) atomicOr(&ctl->status, 1);
   }
 }
 

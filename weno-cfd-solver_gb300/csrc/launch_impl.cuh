@@ -32,15 +32,16 @@ const dim3 kBlk(32, 4, 1);
 }  // namespace detail
 }  // inline namespace WENO_TU_NS
 
-template <class T, bool FAST>
-cudaError_t Launch<T, FAST>::pass1(HostView u, int64_t rows, int64_t cols, double gamma, bool ydir, bool chr,
+template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::pass1(HostView u, int64_t rows, int64_t cols, double gamma, bool ydir, bool chr,
                                    HostPlanes PL, HostPlanes PR, double weps, cudaStream_t st) {
+  using T = dev_t<H>;
   using namespace detail;
   if (rows <= 0 || cols <= 0) return cudaSuccess;
   const dim3 g = grid2d(rows, cols, kBlk);
   auto U = cview<T>(u);
   auto L = planes<T>(PL), R = planes<T>(PR);
-  if constexpr (FAST && std::is_same<T, double>::value) {
+  if constexpr (FAST && is_native_f64<T>) {
     if (!chr) {  // component-wise: two faces per thread along the sweep
       const dim3 g2 = ydir ? grid2d(rows, (cols + 1) / 2, kBlk) : grid2d((rows + 1) / 2, cols, kBlk);
       if (!ydir) k_pass1_cons2<false><<<g2, kBlk, 0, st>>>(U, rows, cols, L, R, weps);
@@ -55,10 +56,11 @@ cudaError_t Launch<T, FAST>::pass1(HostView u, int64_t rows, int64_t cols, doubl
   return cudaGetLastError();
 }
 
-template <class T, bool FAST>
-cudaError_t Launch<T, FAST>::pass2(HostPlanes PL, HostPlanes PR, int64_t rows, int64_t cols, double gamma, bool ydir,
+template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::pass2(HostPlanes PL, HostPlanes PR, int64_t rows, int64_t cols, double gamma, bool ydir,
                                    int kind, void* a, void* b, void* c, void* d, int64_t ps, int64_t ld, double weps,
                                    cudaStream_t st) {
+  using T = dev_t<H>;
   using namespace detail;
   if (rows <= 0 || cols <= 0) return cudaSuccess;
   const dim3 g = grid2d(rows, cols, kBlk);
@@ -80,26 +82,27 @@ cudaError_t Launch<T, FAST>::pass2(HostPlanes PL, HostPlanes PR, int64_t rows, i
       else WENO_P2T(true, P2_BLEND);
     }
 #undef WENO_P2T
-    return cudaGetLastError();
-  }
-#define WENO_P2(Y, K) k_pass2<T, FAST, Y, K><<<g, kBlk, 0, st>>>(L, R, rows, cols, gm, dst, (T)weps)
-  if (!ydir) {
-    if (kind == 0) WENO_P2(false, P2_STATES);
-    else if (kind == 1) WENO_P2(false, P2_HLLE);
-    else WENO_P2(false, P2_BLEND);
   } else {
-    if (kind == 0) WENO_P2(true, P2_STATES);
-    else if (kind == 1) WENO_P2(true, P2_HLLE);
-    else WENO_P2(true, P2_BLEND);
-  }
+#define WENO_P2(Y, K) k_pass2<T, FAST, Y, K><<<g, kBlk, 0, st>>>(L, R, rows, cols, gm, dst, (T)weps)
+    if (!ydir) {
+      if (kind == 0) WENO_P2(false, P2_STATES);
+      else if (kind == 1) WENO_P2(false, P2_HLLE);
+      else WENO_P2(false, P2_BLEND);
+    } else {
+      if (kind == 0) WENO_P2(true, P2_STATES);
+      else if (kind == 1) WENO_P2(true, P2_HLLE);
+      else WENO_P2(true, P2_BLEND);
+    }
 #undef WENO_P2
+  }
   return cudaGetLastError();
 }
 
-template <class T, bool FAST>
-cudaError_t Launch<T, FAST>::riemann(const void* ql, const void* fl, const void* qr, const void* fr, int64_t rows,
+template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::riemann(const void* ql, const void* fl, const void* qr, const void* fr, int64_t rows,
                                      int64_t cols, double gamma, bool ydir, int kind, void* out, void* a, void* b,
                                      void* c, int64_t ps, int64_t ld, cudaStream_t st) {
+  using T = dev_t<H>;
   using namespace detail;
   if (rows <= 0 || cols <= 0) return cudaSuccess;
   const dim3 g = grid2d(rows, cols, kBlk);
@@ -122,9 +125,10 @@ cudaError_t Launch<T, FAST>::riemann(const void* ql, const void* fl, const void*
   return cudaGetLastError();
 }
 
-template <class T, bool FAST>
-cudaError_t Launch<T, FAST>::blend(HostPlanes Fc, HostPlanes Fe, HostPlanes Pbar, int64_t rows, int64_t cols,
+template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::blend(HostPlanes Fc, HostPlanes Fe, HostPlanes Pbar, int64_t rows, int64_t cols,
                                    double jp_lo, double jp_hi, void* out, cudaStream_t st) {
+  using T = dev_t<H>;
   using namespace detail;
   if (rows <= 0 || cols <= 0) return cudaSuccess;
   const dim3 g = grid2d(rows, cols, kBlk);
@@ -134,10 +138,11 @@ cudaError_t Launch<T, FAST>::blend(HostPlanes Fc, HostPlanes Fe, HostPlanes Pbar
   return cudaGetLastError();
 }
 
-template <class T, bool FAST>
-cudaError_t Launch<T, FAST>::residual(HostPlanes Fx, HostPlanes Fy, int64_t rows, int64_t cols, double dx, int stage,
+template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::residual(HostPlanes Fx, HostPlanes Fy, int64_t rows, int64_t cols, double dx, int stage,
                                       void* out, HostPlanes Qn, HostPlanes Qs, HostPlanes Qo, const StepCtl* ctl,
                                       cudaStream_t st) {
+  using T = dev_t<H>;
   using namespace detail;
   if (rows <= 0 || cols <= 0) return cudaSuccess;
   const dim3 g = grid2d(rows, cols, kBlk);
@@ -152,9 +157,10 @@ cudaError_t Launch<T, FAST>::residual(HostPlanes Fx, HostPlanes Fy, int64_t rows
   return cudaGetLastError();
 }
 
-template <class T, bool FAST>
-cudaError_t Launch<T, FAST>::flux(HostView q, int64_t rows, int64_t cols, double gamma, bool ydir, void* out,
+template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::flux(HostView q, int64_t rows, int64_t cols, double gamma, bool ydir, void* out,
                                   cudaStream_t st) {
+  using T = dev_t<H>;
   using namespace detail;
   if (rows <= 0 || cols <= 0) return cudaSuccess;
   const dim3 g = grid2d(rows, cols, kBlk);
@@ -163,9 +169,10 @@ cudaError_t Launch<T, FAST>::flux(HostView q, int64_t rows, int64_t cols, double
   return cudaGetLastError();
 }
 
-template <class T, bool FAST>
-cudaError_t Launch<T, FAST>::con2primi(HostView q, int64_t rows, int64_t cols, double gamma, void* p, void* a,
+template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::con2primi(HostView q, int64_t rows, int64_t cols, double gamma, void* p, void* a,
                                        void* rho, void* u, void* v, void* h, cudaStream_t st) {
+  using T = dev_t<H>;
   using namespace detail;
   if (rows <= 0 || cols <= 0) return cudaSuccess;
   const dim3 g = grid2d(rows, cols, kBlk);
@@ -175,9 +182,10 @@ cudaError_t Launch<T, FAST>::con2primi(HostView q, int64_t rows, int64_t cols, d
   return cudaGetLastError();
 }
 
-template <class T, bool FAST>
-cudaError_t Launch<T, FAST>::bc_transmissive(HostView q, int nc, int64_t M, int64_t N, const StepCtl* ctl,
+template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::bc_transmissive(HostView q, int nc, int64_t M, int64_t N, const StepCtl* ctl,
                                              cudaStream_t st) {
+  using T = dev_t<H>;
   using namespace detail;
   const dim3 g = grid2d(M, N, kBlk);
   if (nc == 8) k_bc_transmissive<T, 8><<<g, kBlk, 0, st>>>(s3<T>(q), M, N, ctl);
@@ -185,21 +193,23 @@ cudaError_t Launch<T, FAST>::bc_transmissive(HostView q, int nc, int64_t M, int6
   return cudaGetLastError();
 }
 
-template <class T, bool FAST>
-cudaError_t Launch<T, FAST>::bc_dmr(HostView q, int nc, int64_t nx, int64_t ny, int64_t bound, const double* post8,
+template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::bc_dmr(HostView q, int nc, int64_t nx, int64_t ny, int64_t bound, const double* post8,
                                     const StepCtl* ctl, cudaStream_t st) {
+  using T = dev_t<H>;
   using namespace detail;
   const dim3 g = grid2d(nx + 6, ny + 6, kBlk);
   Post8<T> post;
-  for (int k = 0; k < 8; ++k) post.v[k] = (T)post8[k];
+  for (int k = 0; k < 8; ++k) post.v[k] = T(post8[k]);
   if (nc == 8) k_bc_dmr<T, 8><<<g, kBlk, 0, st>>>(s3<T>(q), nx, ny, bound, post, ctl);
   else k_bc_dmr<T, 4><<<g, kBlk, 0, st>>>(s3<T>(q), nx, ny, bound, post, ctl);
   return cudaGetLastError();
 }
 
-template <class T, bool FAST>
-cudaError_t Launch<T, FAST>::cfl_max(HostView q, bool aos, int64_t nx, int64_t ny, double gamma, StepCtl* ctl,
+template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::cfl_max(HostView q, bool aos, int64_t nx, int64_t ny, double gamma, StepCtl* ctl,
                                      int sm_count, cudaStream_t st) {
+  using T = dev_t<H>;
   const int64_t total = nx * ny;
   int64_t blocks = (total + 255) / 256;
   const int64_t cap = (int64_t)sm_count * 8;
@@ -210,17 +220,19 @@ cudaError_t Launch<T, FAST>::cfl_max(HostView q, bool aos, int64_t nx, int64_t n
   return cudaGetLastError();
 }
 
-template <class T, bool FAST>
-cudaError_t Launch<T, FAST>::export_aos8(HostPlanes Q, int64_t M, int64_t N, double gamma, double* out,
+template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::export_aos8(HostPlanes Q, int64_t M, int64_t N, double gamma, double* out,
                                          cudaStream_t st) {
+  using T = dev_t<H>;
   using namespace detail;
   const dim3 g = grid2d(M, N, kBlk);
   k_export_aos8<T, FAST><<<g, kBlk, 0, st>>>(planes<T>(Q), M, N, (T)gamma, out);
   return cudaGetLastError();
 }
 
-template <class T, bool FAST>
-cudaError_t Launch<T, FAST>::totals(HostView q, int64_t nx, int64_t ny, double* out4, int sm_count, cudaStream_t st) {
+template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::totals(HostView q, int64_t nx, int64_t ny, double* out4, int sm_count, cudaStream_t st) {
+  using T = dev_t<H>;
   int64_t blocks = (nx * ny + 255) / 256;
   if (blocks > (int64_t)sm_count * 4) blocks = (int64_t)sm_count * 4;
   if (blocks < 1) blocks = 1;
@@ -230,8 +242,9 @@ cudaError_t Launch<T, FAST>::totals(HostView q, int64_t nx, int64_t ny, double* 
   return cudaGetLastError();
 }
 
-template <class T, bool FAST>
-cudaError_t Launch<T, FAST>::import_planes(HostView q, int64_t M, int64_t N, HostPlanes Q, cudaStream_t st) {
+template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::import_planes(HostView q, int64_t M, int64_t N, HostPlanes Q, cudaStream_t st) {
+  using T = dev_t<H>;
   using namespace detail;
   const dim3 g = grid2d(M, N, kBlk);
   k_import_planes<T><<<g, kBlk, 0, st>>>(cview<double>(q), M, N, planes<T>(Q));
