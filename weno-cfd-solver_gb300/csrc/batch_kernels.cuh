@@ -169,7 +169,7 @@ __device__ __forceinline__ void tile_gq_side(const T* p, int ks, int ts, T weps,
       a1[k] = ra.v.x, a1[k + 1] = ra.v.y, a2[k] = rb.v.x, a2[k + 1] = rb.v.y;
     }
   } else {
-#pragma unroll(FAST ? 4 : 1)
+#pragma unroll(kFieldUnroll<T>)
     for (int k = 0; k < 4; ++k) {
       const T* u = p + k * ks;
       T a, b;
@@ -603,12 +603,16 @@ template <bool Y, bool SUM>
 __device__ __forceinline__ void staged_gq_two(const f64* p, long long ks, long long ts, bool two, f64 gamma,
                                               f64 weps, f64 qA[4], f64 fA[4], f64 qB[4], f64 fB[4]) {
   f64 a1A[4], a2A[4], a1B[4], a2B[4];
-#pragma unroll
+#pragma unroll 1
   for (int k = 0; k < 4; ++k) {
     const f64* u = p + k * ks;
     const f64 v4 = u[4 * ts];
-    weno5_gq_two<f64>(u[0], u[ts], u[2 * ts], u[3 * ts], v4, two ? u[5 * ts] : v4, weps, a1A[k], a2A[k], a1B[k],
-                         a2B[k]);
+    f64 pA, mA, pB, mB;
+    weno5_gq_two<f64>(u[0], u[ts], u[2 * ts], u[3 * ts], v4, two ? u[5 * ts] : v4, weps, pA, mA, pB, mB);
+    put4(a1A, k, pA);
+    put4(a2A, k, mA);
+    put4(a1B, k, pB);
+    put4(a2B, k, mB);
   }
   f64 f1[4], f2[4];
   euler_flux_pair<f64, true, Y>(a1A, a2A, gamma, f1, f2);

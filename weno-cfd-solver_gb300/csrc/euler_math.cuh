@@ -27,6 +27,7 @@
 #include "df64.cuh"
 #include "f32x2.cuh"
 #include "f64.cuh"
+#include "ffw.cuh"
 #include "fp64_fast.cuh"
 
 namespace weno {
@@ -101,9 +102,12 @@ __device__ __forceinline__ T mul_pow2(T x) {
   else return x * T(K >= 0 ? (double)(1 << (K >= 0 ? K : 0)) : 1.0 / (double)(1 << (K < 0 ? -K : 0)));
 }
 
-// v[k] and v[k] = x for a run-time k without leaving registers: the exact kernels
-// loop over the four fields (unrolled, their integer divisions would not fit the
-// instruction cache).
+// v[k] and v[k] = x for a run-time k without leaving registers.  The FP64 kernels
+// loop over the four fields: unrolled, their integer divisions (exact) or
+// float-pair weights (FAST) would not fit the instruction cache, and FP64 is
+// their bound, not the latency of one warp.
+template <class T>
+constexpr int kFieldUnroll = is_native_f64<T> ? 1 : 4;
 template <class T>
 __device__ __forceinline__ T pick4(const T v[4], int k) {
   const T a = (k & 1) ? v[1] : v[0], b = (k & 1) ? v[3] : v[2];
@@ -411,6 +415,35 @@ __device__ __forceinline__ void weno5_lr_exact(const T u[6], T weps, T& left, T&
   }
 }
 
+// Largest high word (sign cleared) of differences, for ffw::covers.
+__device__ __forceinline__ uint32_t max_magnitude(f64 a, f64 b) { return max(ffw::magnitude(a.v), ffw::magnitude(b.v)); }
+__device__ __forceinline__ uint32_t max_magnitude(uint32_t a, uint32_t b, f64 c) {
+  return max(max(a, b), ffw::magnitude(c.v));
+}
+
+// u plus (sg = 1) or minus the weighted slope of a cell's face state: near and
+// mid differences dn (across the face), dm and far ones df (behind the cell), fn
+// (beyond the face).
+__device__ __forceinline__ f64 face_slope(f64 dn, f64 fn, f64 dm, f64 df, double c_near, double c_mid, double c_far) {
+  // candidates less the cell's value (x6): 4 dn - fn, 2 dn + dm, 5 dm - 2 df
+  return fma(f64(c_near), fma(f64(4.0), dn, -fn),
+             fma(f64(c_mid), fma(f64(2.0), dn, dm), f64(xmul(ffw::twice(c_far), fma(f64(2.5), dm, -df).v))));
+}
+
+// Both states of one field at the face between u2 and u3 with float-pair weights
+// (ffw.cuh): 21 FP64 operations, where the FP64 weights below take 69.
+__device__ __forceinline__ void weno5_lr_ffw(f64 u2, f64 u3, f64 d0, f64 d1, f64 d2, f64 d3, f64 d4, f64 weps,
+                                             f64& left, f64& right) {
+  const ffw::ff w = ffw::eps75(weps.v);
+  const ffw::ff f0 = ffw::from_double(d0.v), f1 = ffw::from_double(d1.v), f2 = ffw::from_double(d2.v),
+                f3 = ffw::from_double(d3.v), f4 = ffw::from_double(d4.v);
+  double cn, cm, cf;
+  ffw::face_weights(ffw::side(f2, f3, w), ffw::centre(f1, f2, w), ffw::side(f1, f0, w), cn, cm, cf);
+  left = u2 + face_slope(d2, d3, d1, d0, cn, cm, cf);
+  ffw::face_weights(ffw::side(f2, f1, w), ffw::centre(f2, f3, w), ffw::side(f3, f4, w), cn, cm, cf);
+  right = u3 - face_slope(d2, d1, d3, d4, cn, cm, cf);
+}
+
 // Both reconstructions of one field at one face (the right stencil is the left
 // one shifted by a cell), FAST: native double shares one divide
 // between the two; float and df64 take reciprocal weights.
@@ -420,6 +453,12 @@ __device__ __forceinline__ void weno5_lr_fast(T u0, T u1, T u2, T u3, T u4, T u5
   // (centred on u_m), shared by the two stencils; each Jiang-Shu indicator is
   // 13/12 D^2 + 1/4 s^2 with s a combination of two first differences.
   const T d0 = u1 - u0, d1 = u2 - u1, d2 = u3 - u2, d3 = u4 - u3, d4 = u5 - u4;
+  if constexpr (is_native_f64<T>) {
+    if (ffw::covers(max_magnitude(max_magnitude(d0, d1), max_magnitude(d2, d3), d4), weps.v)) {
+      weno5_lr_ffw(u2, u3, d0, d1, d2, d3, d4, weps, left, right);
+      return;
+    }
+  }
   const T D1 = d1 - d0, D2 = d2 - d1, D3 = d3 - d2, D4 = d4 - d3;
   // indicators scaled by 4 (see kC43): 4 eps + (13/3) D^2 + s^2
   const T w4 = T(4.0) * weps;
@@ -543,12 +582,36 @@ __device__ __forceinline__ void gq_weights(T q2, T h0, T h1, T h2, T f0, T f1, T
   }
 }
 
+// The Gauss-point pair of one cell with first differences d0, d1 | d2, d3 (their
+// float pairs f), float-pair weights.
+__device__ __forceinline__ void gq_ffw(f64 q, f64 d0, f64 d1, f64 d2, f64 d3, ffw::ff f0, ffw::ff f1, ffw::ff f2,
+                                       ffw::ff f3, ffw::ff w, f64& ra, f64& rb) {
+  constexpr ffw::ff r0 = ffw::constant(kGqA0 / kGqA1), r2 = ffw::constant(kGqA2 / kGqA1), S = ffw::constant(kSqrt3_12);
+  const ffw::ff qr = ffw::side(f2, f3, w), qm = ffw::centre(f1, f2, w), ql = ffw::side(f1, f0, w);
+  const f64 hr = fma(f64(-3.0), d2, d3), hm = d1 + d2, hl = fma(f64(3.0), d1, -d0);
+  double cr, cm, cl;
+  ffw::gauss_weights(qr, qm, ql, r0, r2, S, cr, cm, cl);
+  ra = q + fma(f64(cr), hr, fma(f64(-cm), hm, f64(xmul(-cl, hl.v))));
+  ffw::gauss_weights(qr, qm, ql, r2, r0, S, cr, cm, cl);
+  rb = q + fma(f64(-cr), hr, fma(f64(cm), hm, f64(xmul(cl, hl.v))));
+}
+
 // Two neighbouring 5-cell stencils (q0..q4 and q1..q5), FAST: both
 // Gauss-point pairs, sharing the first and second differences.
 template <class T>
 __device__ __forceinline__ void weno5_gq_two(T q0, T q1, T q2, T q3, T q4, T q5, T weps, T& raA, T& rbA, T& raB,
                                              T& rbB) {
   const T d0 = q1 - q0, d1 = q2 - q1, d2 = q3 - q2, d3 = q4 - q3, d4 = q5 - q4;
+  if constexpr (is_native_f64<T>) {
+    if (ffw::covers(max_magnitude(max_magnitude(d0, d1), max_magnitude(d2, d3), d4), weps.v)) {
+      const ffw::ff w = ffw::eps75(weps.v);
+      const ffw::ff f0 = ffw::from_double(d0.v), f1 = ffw::from_double(d1.v), f2 = ffw::from_double(d2.v),
+                    f3 = ffw::from_double(d3.v), f4 = ffw::from_double(d4.v);
+      gq_ffw(q2, d0, d1, d2, d3, f0, f1, f2, f3, w, raA, rbA);
+      gq_ffw(q3, d1, d2, d3, d4, f1, f2, f3, f4, w, raB, rbB);
+      return;
+    }
+  }
   const T D1 = d1 - d0, D2 = d2 - d1, D3 = d3 - d2, D4 = d4 - d3;
   const T w4 = T(4.0) * weps;
   const T C1 = T(kC43) * D1 * D1 + w4, C2 = T(kC43) * D2 * D2 + w4, C3 = T(kC43) * D3 * D3 + w4,
@@ -566,6 +629,13 @@ __device__ __forceinline__ void weno5_gq_pair(T q0, T q1, T q2, T q3, T q4, T& r
     // difference form (as in weno5_lr_fast): the one-sided indicator terms are
     // the polynomial slopes g0, g2 and the centred one is g1/S
     const T d0 = q1 - q0, d1 = q2 - q1, d2 = q3 - q2, d3 = q4 - q3;
+    if constexpr (is_native_f64<T>) {
+      if (ffw::covers(max(max_magnitude(d0, d1), max_magnitude(d2, d3)), weps.v)) {
+        gq_ffw(q2, d0, d1, d2, d3, ffw::from_double(d0.v), ffw::from_double(d1.v), ffw::from_double(d2.v),
+               ffw::from_double(d3.v), ffw::eps75(weps.v), ra, rb);
+        return;
+      }
+    }
     const T D1 = d1 - d0, D2 = d2 - d1, D3 = d3 - d2;
     const T h0 = d3 - T(3.0) * d2;  // 3 q2 - 4 q3 + q4
     const T h1 = d1 + d2;           // q3 - q1
@@ -759,10 +829,15 @@ struct CharScalars {
 };
 
 template <class T, bool Y>
+__device__ __forceinline__ void project_parts(const CharScalars<T>& k, const T q[4], T& Z, T& Yv) {
+  Z = (k.kin * q[0] + q[3]) - k.u * q[1] - k.v * q[2];
+  Yv = k.b * q[0] - k.hr * q[Y ? 2 : 1];
+}
+template <class T, bool Y>
 __device__ __forceinline__ void project_left(const CharScalars<T>& k, const T q[4], T w[4]) {
   // Z from q3 upwards and G Z / 2 +- Yv as one FMA each: nine operations
-  const T Z = (k.kin * q[0] + q[3]) - k.u * q[1] - k.v * q[2];
-  const T Yv = k.b * q[0] - k.hr * q[Y ? 2 : 1];
+  T Z, Yv;
+  project_parts<T, Y>(k, q, Z, Yv);
   w[0] = k.G2 * Z + Yv;
   w[1] = q[0] - k.G * Z;
   w[2] = q[Y ? 1 : 2] - (Y ? k.u : k.v) * q[0];  // rho w2
@@ -823,17 +898,14 @@ template <class T, bool FAST, bool Y, bool CHAR>
 __device__ __forceinline__ void pass1_face(const T c[6][4], T gamma, T ql[4], T qr[4], T weps) {
   if constexpr (!CHAR && FAST && is_f32<T>) {
     weno5_lr_fast_f32_pairs(c, weps, ql, qr, weps);
-  } else if constexpr (!CHAR && FAST) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      weno5_lr_fast<T>(c[0][k], c[1][k], c[2][k], c[3][k], c[4][k], c[5][k], weps, ql[k], qr[k]);
   } else if constexpr (!CHAR) {
-#pragma unroll 1
+#pragma unroll(kFieldUnroll<T>)
     for (int k = 0; k < 4; ++k) {
       T u[6], l, r;
 #pragma unroll
       for (int s = 0; s < 6; ++s) u[s] = pick4(c[s], k);
-      weno5_lr_exact<T>(u, weps, l, r);
+      if constexpr (FAST) weno5_lr_fast<T>(u[0], u[1], u[2], u[3], u[4], u[5], weps, l, r);
+      else weno5_lr_exact<T>(u, weps, l, r);
       put4(ql, k, l);
       put4(qr, k, r);
     }
@@ -845,7 +917,6 @@ __device__ __forceinline__ void pass1_face(const T c[6][4], T gamma, T ql[4], T 
     // cells 2|3), so six projections cover both.
     T chl[4], chr[4];
     if constexpr (FAST) {
-      T w[6][4];
       CharScalars<T> k;
       k.u = u_a;
       k.v = v_a;
@@ -858,16 +929,40 @@ __device__ __forceinline__ void pass1_face(const T c[6][4], T gamma, T ql[4], T 
       const T ich = T(0.5) * ic_a;
       k.b = (Y ? v_a : u_a) * ich;
       k.hr = ich * irho_a;
-#pragma unroll
-      for (int s = 0; s < 6; ++s) project_left<T, Y>(k, c[s], w[s]);
       const T weps2 = weps * (rho_a * rho_a);  // epsilon of the shear field rho w2
-      if constexpr (is_f32<T>) {
-        weno5_lr_fast_f32_pairs(w, weps, chl, chr, weps2);
-      } else {
+      if constexpr (is_native_f64<T>) {
+        // the fields are G2 Z + Yv, q0 - G Z, q_t - u_t q0, G2 Z - Yv (project_left):
+        // one product and one addend per cell, selected by field
+        T Z[6], Yv[6];
 #pragma unroll
-        for (int f = 0; f < 4; ++f)
-          weno5_lr_fast<T>(w[0][f], w[1][f], w[2][f], w[3][f], w[4][f], w[5][f], f == 2 ? weps2 : weps, chl[f],
-                           chr[f]);
+        for (int s = 0; s < 6; ++s) project_parts<T, Y>(k, c[s], Z[s], Yv[s]);
+        const T ut = Y ? k.u : k.v;
+#pragma unroll 1
+        for (int f = 0; f < 4; ++f) {
+          const T A = f == 1 ? -k.G : (f == 2 ? -ut : k.G2);
+          T w[6], l, r;
+#pragma unroll
+          for (int s = 0; s < 6; ++s) {
+            const T X = f == 2 ? c[s][0] : Z[s];
+            const T B = f == 0 ? Yv[s] : (f == 1 ? c[s][0] : (f == 2 ? c[s][Y ? 1 : 2] : -Yv[s]));
+            w[s] = fma(A, X, B);
+          }
+          weno5_lr_fast<T>(w[0], w[1], w[2], w[3], w[4], w[5], f == 2 ? weps2 : weps, l, r);
+          put4(chl, f, l);
+          put4(chr, f, r);
+        }
+      } else {
+        T w[6][4];
+#pragma unroll
+        for (int s = 0; s < 6; ++s) project_left<T, Y>(k, c[s], w[s]);
+        if constexpr (is_f32<T>) {
+          weno5_lr_fast_f32_pairs(w, weps, chl, chr, weps2);
+        } else {
+#pragma unroll
+          for (int f = 0; f < 4; ++f)
+            weno5_lr_fast<T>(w[0][f], w[1][f], w[2][f], w[3][f], w[4][f], w[5][f], f == 2 ? weps2 : weps, chl[f],
+                             chr[f]);
+        }
       }
       project_right<T, Y>(k, chl, ql);
       project_right<T, Y>(k, chr, qr);

@@ -141,7 +141,7 @@ struct Pass2Dst {
 
 template <class T, bool FAST, bool Y>
 __device__ __forceinline__ void gq_face(const Planes<T>& P, int64_t row, int64_t col, T q1[4], T q2[4], T weps) {
-#pragma unroll(FAST ? 4 : 1)
+#pragma unroll(kFieldUnroll<T>)
   for (int k = 0; k < 4; ++k) {
     T s[5], a, b;
 #pragma unroll
@@ -237,12 +237,16 @@ __device__ __forceinline__ void gq_side_two(const Planes<T>& P, int64_t row, int
       a1B[k] = raB.v.x, a1B[k + 1] = raB.v.y, a2B[k] = rbB.v.x, a2B[k + 1] = rbB.v.y;
     }
   } else {
-#pragma unroll
+#pragma unroll(kFieldUnroll<T>)
     for (int k = 0; k < 4; ++k) {
-      T v[6];
+      T v[6], pA, mA, pB, mB;
 #pragma unroll
       for (int t = 0; t < 6; ++t) v[t] = Y ? P.at(k, row + 1 + t, col) : P.at(k, row, col + 1 + t);
-      weno5_gq_two<T>(v[0], v[1], v[2], v[3], v[4], v[5], weps, a1A[k], a2A[k], a1B[k], a2B[k]);
+      weno5_gq_two<T>(v[0], v[1], v[2], v[3], v[4], v[5], weps, pA, mA, pB, mB);
+      put4(a1A, k, pA);
+      put4(a2A, k, mA);
+      put4(a1B, k, pB);
+      put4(a2B, k, mB);
     }
   }
   const T h = SUM ? T(1.0) : T(0.5);
@@ -278,8 +282,23 @@ __global__ void __launch_bounds__(128) k_pass2_two(Planes<T> PL, Planes<T> PR, i
   constexpr bool SUM = OUT == P2_HLLE;
   constexpr int S = SUM ? 2 : 1;
   T qlA[4], flA[4], qlB[4], flB[4], qrA[4], frA[4], qrB[4], frB[4];
-  gq_side_two<T, Y, SUM>(PL, row, col, gamma, weps, qlA, flA, qlB, flB);
-  gq_side_two<T, Y, SUM>(PR, row, col, gamma, weps, qrA, frA, qrB, frB);
+  if constexpr (is_native_f64<T>) {
+#pragma unroll 1
+    for (int side = 0; side < 2; ++side) {  // one copy of the code, left then right
+      const Planes<T> P{side ? PR.p : PL.p, PL.ps, PL.ld};
+      gq_side_two<T, Y, SUM>(P, row, col, gamma, weps, qrA, frA, qrB, frB);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        qlA[k] = side ? qlA[k] : qrA[k];
+        flA[k] = side ? flA[k] : frA[k];
+        qlB[k] = side ? qlB[k] : qrB[k];
+        flB[k] = side ? flB[k] : frB[k];
+      }
+    }
+  } else {
+    gq_side_two<T, Y, SUM>(PL, row, col, gamma, weps, qlA, flA, qlB, flB);
+    gq_side_two<T, Y, SUM>(PR, row, col, gamma, weps, qrA, frA, qrB, frB);
+  }
   pass2_emit<T, true, Y, OUT, S>(qlA, flA, qrA, frA, gamma, dst, row, col, cols);
   if (two)
     pass2_emit<T, true, Y, OUT, S>(qlB, flB, qrB, frB, gamma, dst, Y ? row + 1 : row, Y ? col : col + 1, cols);
