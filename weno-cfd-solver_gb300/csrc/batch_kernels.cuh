@@ -614,19 +614,21 @@ __device__ __forceinline__ void staged_gq_two(const f64* p, long long ks, long l
     put4(a1B, k, pB);
     put4(a2B, k, mB);
   }
-  f64 f1[4], f2[4];
-  euler_flux_pair<f64, true, Y>(a1A, a2A, gamma, f1, f2);
+  euler_flux_sum<f64, Y>(a1A, a2A, gamma, fA);
+  if (two) euler_flux_sum<f64, Y>(a1B, a2B, gamma, fB);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    fA[k] = SUM ? f1[k] + f2[k] : 0.5 * (f1[k] + f2[k]);
-    qA[k] = SUM ? a1A[k] + a2A[k] : 0.5 * (a1A[k] + a2A[k]);
-  }
-  if (!two) return;
-  euler_flux_pair<f64, true, Y>(a1B, a2B, gamma, f1, f2);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    fB[k] = SUM ? f1[k] + f2[k] : 0.5 * (f1[k] + f2[k]);
-    qB[k] = SUM ? a1B[k] + a2B[k] : 0.5 * (a1B[k] + a2B[k]);
+    qA[k] = a1A[k] + a2A[k];
+    if constexpr (!SUM) {
+      fA[k] = half(fA[k]);
+      qA[k] = half(qA[k]);
+    }
+    if (!two) continue;
+    qB[k] = a1B[k] + a2B[k];
+    if constexpr (!SUM) {
+      fB[k] = half(fB[k]);
+      qB[k] = half(qB[k]);
+    }
   }
 }
 

@@ -84,23 +84,15 @@ __device__ __forceinline__ T cmax(T x, T c) {
   if constexpr (FAST && is_native_f64<T>) return f64_bits(x) > f64_bits(c) ? x : c;
   else return vmax(x, c);
 }
-template <class T, bool FAST>
-__device__ __forceinline__ bool lt_bound(T x, T c) {
-  if constexpr (FAST && is_native_f64<T>) return f64_bits(x) < f64_bits(c);
-  else return x < c;
-}
-template <class T, bool FAST>
-__device__ __forceinline__ bool gt_zero(T x) {
-  if constexpr (FAST && is_native_f64<T>) return f64_bits(x) > 0;
-  else return x > T(0.0);
-}
-
 // x 2^K of the exact forms: an integer operation on an f64's exponent.
 template <int K, class T>
 __device__ __forceinline__ T mul_pow2(T x) {
   if constexpr (is_native_f64<T>) return T(xscale<K>(x.v));
   else return x * T(K >= 0 ? (double)(1 << (K >= 0 ? K : 0)) : 1.0 / (double)(1 << (K < 0 ? -K : 0)));
 }
+
+template <class T>
+__device__ __forceinline__ T half(T x) { return mul_pow2<-1>(x); }
 
 // v[k] and v[k] = x for a run-time k without leaving registers.  The FP64 kernels
 // loop over the four fields: unrolled, their integer divisions (exact) or
@@ -119,34 +111,34 @@ __device__ __forceinline__ void put4(T v[4], int k, T x) {
   for (int i = 0; i < 4; ++i) v[i] = k == i ? x : v[i];
 }
 
-// a / b: the IEEE quotient except in FAST float (the SFU path) and FAST double
-// (a times the three-FMA reciprocal of fp64_fast.cuh).
+// a / b: the IEEE quotient except in FAST float (the SFU path).  For an f64 the
+// correctly rounded integer forms of rn64.cuh: no FP64 slot, where the seeded
+// Newton forms of fp64_fast.cuh take three to six (64 issue slots each).
 template <class T, bool FAST>
 __device__ __forceinline__ T qdiv(T a, T b) {
   if constexpr (FAST && is_f32<T>) return __fdividef(a, b);
-  else if constexpr (FAST && is_native_f64<T>) return a * T(f64fast::rcp(b.v));
   else return a / b;
 }
 template <class T, bool FAST>
 __device__ __forceinline__ T qrcp(T b) {
   if constexpr (FAST && is_f32<T>) return __fdividef(1.0f, b);
-  else if constexpr (FAST && is_native_f64<T>) return T(f64fast::rcp(b.v));
   else return T(1.0) / b;
 }
-template <class T, bool FAST>
-__device__ __forceinline__ T qsqrt(T x) {
-  if constexpr (FAST && is_native_f64<T>) return T(f64fast::sqrt(x.v));
-  else return sqrt(x);
-}
-// 1/sqrt(x) of the FAST forms (x > 0): one reciprocal square root gives sqrt(x)
-// = x * r and 1/x = r * r, replacing a square root and two divisions.  Double:
-// fp64_fast.cuh (within 1 ulp); float: CUDA's rsqrtf (within 2 ulp); df64
-// takes 1/sqrt.
+// sqrt(x), 1/sqrt(x) and 1/x of the FAST forms (x > 0).  An f64 takes the integer
+// root and reciprocal and one product; float (CUDA's rsqrtf, within 2 ulp) and
+// df64 one reciprocal square root r, x r and r r.
 template <class T>
-__device__ __forceinline__ T frsqrt(T x) {
-  if constexpr (is_native_f64<T>) return T(f64fast::rsqrt(x.v));
-  else if constexpr (is_f32<T>) return rsqrtf(x);
-  else return T(1.0) / sqrt(x);
+__device__ __forceinline__ void roots(T x, T& root, T& inv_root, T& inv) {
+  if constexpr (is_native_f64<T>) {
+    root = sqrt(x);
+    inv = T(1.0) / x;
+    inv_root = root * inv;
+  } else {
+    if constexpr (is_f32<T>) inv_root = rsqrtf(x);
+    else inv_root = T(1.0) / sqrt(x);
+    root = x * inv_root;
+    inv = inv_root * inv_root;
+  }
 }
 
 // a*b + c*d with both products rounded on their own (never contracted into an
@@ -176,14 +168,13 @@ __device__ __forceinline__ T half_rho_speed2(T rho, T m, T n, T u, T v) {
   else return mul_pow2<-1>(rho) * (u * u + v * v);
 }
 
-// Euler flux normal to x (Y = false) or y (Y = true), utils.rs:74-109.  `rinv`
-// (FAST only, when > 0) is 1/max(q[0], eps) computed by the caller.
+// Euler flux normal to x (Y = false) or y (Y = true), utils.rs:74-109.
 template <class T, bool FAST, bool Y>
-__device__ __forceinline__ void euler_flux(const T q[4], T gamma, T f[4], T rinv = T(0.0)) {
+__device__ __forceinline__ void euler_flux(const T q[4], T gamma, T f[4]) {
   const T rho = cmax<T, FAST>(q[0], T(kEps));
   T u, v;
   if constexpr (FAST) {
-    const T r = gt_zero<T, FAST>(rinv) ? rinv : qrcp<T, FAST>(rho);
+    const T r = qrcp<T, FAST>(rho);
     u = q[1] * r;
     v = q[2] * r;
   } else {
@@ -204,29 +195,33 @@ __device__ __forceinline__ void euler_flux(const T q[4], T gamma, T f[4], T rinv
   }
 }
 
-// Two Euler fluxes (utils.rs:74-109).  FAST native double shares one division
-// between the two densities: 1/(rho_a rho_b) (f64fast::rcp2, relative error
-// below 2^-41), whose product stays in range for any clamped density below
-// 1e150 (otherwise two divisions).
+// Two Euler fluxes (utils.rs:74-109).
 template <class T, bool FAST, bool Y>
 __device__ __forceinline__ void euler_flux_pair(const T qa[4], const T qb[4], T gamma, T fa[4], T fb[4]) {
-  if constexpr (FAST && is_native_f64<T>) {
-    const T ra = cmax<T, FAST>(qa[0], T(kEps)), rb = cmax<T, FAST>(qb[0], T(kEps));
-    const T prod = ra * rb;
-    T ia, ib;
-    if (lt_bound<T, FAST>(prod, T(1e300))) {
-      const T inv = T(f64fast::rcp2(prod.v));
-      ia = rb * inv;
-      ib = ra * inv;
-    } else {
-      ia = T(f64fast::rcp(ra.v));
-      ib = T(f64fast::rcp(rb.v));
-    }
-    euler_flux<T, FAST, Y>(qa, gamma, fa, ia);
-    euler_flux<T, FAST, Y>(qb, gamma, fb, ib);
+  euler_flux<T, FAST, Y>(qa, gamma, fa);
+  euler_flux<T, FAST, Y>(qb, gamma, fb);
+}
+
+// The sum of the two fluxes of a Gauss pair (FAST).  An f64 adds the products as
+// FMAs: with m, n the momenta along and across the face normal,
+// sum (m, m u + p, n u, u (E + p)).
+template <class T, bool Y>
+__device__ __forceinline__ void euler_flux_sum(const T qa[4], const T qb[4], T gamma, T f[4]) {
+  if constexpr (is_native_f64<T>) {
+    constexpr int M = Y ? 2 : 1, N = Y ? 1 : 2;
+    const T ia = T(1.0) / cmax<T, true>(qa[0], T(kEps)), ib = T(1.0) / cmax<T, true>(qb[0], T(kEps));
+    const T ua = qa[M] * ia, ub = qb[M] * ib, va = qa[N] * ia, vb = qb[N] * ib;
+    const T g = gamma - T(1.0);
+    const T pa = g * (qa[3] - T(0.5) * (qa[M] * ua + qa[N] * va)), pb = g * (qb[3] - T(0.5) * (qb[M] * ub + qb[N] * vb));
+    f[0] = qa[M] + qb[M];
+    f[M] = qa[M] * ua + (qb[M] * ub + (pa + pb));
+    f[N] = qa[N] * ua + qb[N] * ub;
+    f[3] = ua * (qa[3] + pa) + ub * (qb[3] + pb);
   } else {
-    euler_flux<T, FAST, Y>(qa, gamma, fa);
-    euler_flux<T, FAST, Y>(qb, gamma, fb);
+    T f1[4], f2[4];
+    euler_flux_pair<T, true, Y>(qa, qb, gamma, f1, f2);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) f[k] = f1[k] + f2[k];
   }
 }
 
@@ -239,7 +234,7 @@ __device__ __forceinline__ void con2prim(T q0, T q1, T q2, T q3, T gamma, T& p, 
     u = q1 * r;
     v = q2 * r;
     p = cmax<T, FAST>((gamma - T(1.0)) * (q3 - half_rho_speed2<T, FAST>(rho, q1, q2, u, v)), T(kEps));
-    a = qsqrt<T, FAST>(gamma * p * r);
+    a = sqrt(T(gamma * p * r));
     h = (q3 + p) * r;
   } else {
     u = q1 / rho;
@@ -679,10 +674,7 @@ struct RoeSide {
 template <class T>
 __device__ __forceinline__ RoeSide<T> roe_side(const T u[4], T gamma) {
   RoeSide<T> s;
-  const T rho = vmax(u[0], T(kEps));
-  s.r = frsqrt(rho);
-  s.sq = rho * s.r;
-  s.i = s.r * s.r;
+  roots(vmax(u[0], T(kEps)), s.sq, s.r, s.i);
   // kinetic energy (m^2 + n^2) / (2 rho): the velocities themselves are not needed
   const T p = vmax<T>((gamma - T(1.0)) * (u[3] - T(0.5) * ((u[1] * u[1] + u[2] * u[2]) * s.i)), T(kEps));
   s.a = u[1] * s.r;
@@ -703,8 +695,13 @@ __device__ __forceinline__ void roe_face(const RoeSide<T>& L, const RoeSide<T>& 
   h_roe = mul_add<T>(L.ep, L.r, R.ep * R.r) * id;
   const T kin = T(0.5) * (u_roe * u_roe + v_roe * v_roe);
   const T c2 = vmax<T>((gamma - T(1.0)) * (h_roe - kin), T(kEps) * vmax<T>(L.i, R.i));
-  ic = frsqrt(c2);
-  c_roe = c2 * ic;
+  if constexpr (is_native_f64<T>) {
+    c_roe = sqrt(c2);
+    ic = T(1.0) / c_roe;
+  } else {
+    T i;
+    roots(c2, c_roe, ic, i);
+  }
   rho_roe = L.sq * R.sq;
   irho = L.r * R.r;
 }
@@ -859,6 +856,23 @@ __device__ __forceinline__ void project_right(const CharScalars<T>& k, const T w
   out[3] = (k.h - un * k.c) * w[0] + k.kin * w[1] + (Y ? k.u : k.v) * w[2] + (k.h + un * k.c) * w[3];
 }
 
+// A double as the nearest-below float for a screening test: zero below the float
+// range, NaN (which fails every comparison) above it.
+__device__ __forceinline__ float screen_float(f64 x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x.v), e = hi & 0x7ff00000u;
+  const uint32_t m = (__funnelshift_l((uint32_t)__double2loint(x.v), hi, 3) & 0x7fffffffu) ^ 0x40000000u;
+  const float f = __uint_as_float(m | (hi & 0x80000000u));
+  return e < (897u << 20) ? 0.0f : (e > (1150u << 20) ? __uint_as_float(0x7fffffffu) : f);
+}
+// Whether the density is positive and the pressure test E rho - |m|^2/2 >=
+// eps rho / (gamma - 1) passes by 4e-6 of E rho (the float forms are within
+// 5e-7 of it, and 3e-6 E rho exceeds the bound): the limiter has nothing to do.
+__device__ __forceinline__ bool clearly_positive(const f64 q[4], f64 gamma) {
+  const float r = screen_float(q[0]), m = screen_float(q[1]), n = screen_float(q[2]), e = screen_float(q[3]);
+  const float er = e * r;
+  return r > 1e-9f && e > 1e-3f && er - 0.5f * (m * m + n * n) > 4e-6f * er && gamma > f64(1.001);
+}
+
 // weno.rs:312-315 pressure ; weno.rs:327-352 Zhang-Shu limiter toward `ub`.
 template <class T, bool FAST>
 __device__ __forceinline__ T pp_pressure(const T q[4], T gamma) {
@@ -867,6 +881,10 @@ __device__ __forceinline__ T pp_pressure(const T q[4], T gamma) {
 }
 template <class T, bool FAST>
 __device__ __forceinline__ void pp_limit(T q[4], const T ub[4], T gamma) {
+  // FAST native double: a float test, off the FP64 pipe, settles nearly every face
+  if constexpr (FAST && is_native_f64<T>) {
+    if (clearly_positive(q, gamma)) return;
+  }
   if (q[0] < T(kEps)) {
     const T rho_bar = vmax(ub[0], T(kEps));
     const T theta = vmax<T>(vmin<T>(qdiv<T, FAST>(rho_bar - T(kEps), rho_bar - q[0]), T(1.0)), T(0.0));
@@ -1013,14 +1031,13 @@ __device__ __forceinline__ RiemannPre<T, FAST, Y> riemann_pre(const T ql[4], con
   r.ql0 = cmax<T, FAST>(ql[0], T(kEps * S));
   r.qr0 = cmax<T, FAST>(qr[0], T(kEps * S));
   T h_l, h_r, u_t, v_t, h_t;
-  T rsl = T(0.0), rsr = T(0.0);  // FAST: 1/sqrt(rho) per side
+  T sl = T(0.0), sr = T(0.0), rsl = T(0.0), rsr = T(0.0), il = T(0.0), ir = T(0.0);  // FAST: sqrt(rho), 1/sqrt(rho), 1/rho
   if constexpr (!FAST) {
     r.u_l = ql[1] / r.ql0; r.v_l = ql[2] / r.ql0;
     r.u_r = qr[1] / r.qr0; r.v_r = qr[2] / r.qr0;
   } else {
-    rsl = frsqrt(r.ql0);
-    rsr = frsqrt(r.qr0);
-    const T il = rsl * rsl, ir = rsr * rsr;
+    roots(r.ql0, sl, rsl, il);
+    roots(r.qr0, sr, rsr, ir);
     r.u_l = ql[1] * il; r.v_l = ql[2] * il;
     r.u_r = qr[1] * ir; r.v_r = qr[2] * ir;
   }
@@ -1030,8 +1047,8 @@ __device__ __forceinline__ RiemannPre<T, FAST, Y> riemann_pre(const T ql[4], con
     r.p_l = (gamma - T(1.0)) * (ql[3] - half_rho_speed2<T, FAST>(r.ql0, ql[1], ql[2], r.u_l, r.v_l));
     r.p_r = (gamma - T(1.0)) * (qr[3] - half_rho_speed2<T, FAST>(r.qr0, qr[1], qr[2], r.u_r, r.v_r));
   } else {
-    r.p_l = (gamma - T(1.0)) * (ql[3] - T(0.5) * ((ql[1] * ql[1] + ql[2] * ql[2]) * (rsl * rsl)));
-    r.p_r = (gamma - T(1.0)) * (qr[3] - T(0.5) * ((qr[1] * qr[1] + qr[2] * qr[2]) * (rsr * rsr)));
+    r.p_l = (gamma - T(1.0)) * (ql[3] - T(0.5) * ((ql[1] * ql[1] + ql[2] * ql[2]) * il));
+    r.p_r = (gamma - T(1.0)) * (qr[3] - T(0.5) * ((qr[1] * qr[1] + qr[2] * qr[2]) * ir));
   }
   r.p_l = cmax<T, FAST>(r.p_l, T(kEps * S));
   r.p_r = cmax<T, FAST>(r.p_r, T(kEps * S));
@@ -1045,13 +1062,13 @@ __device__ __forceinline__ RiemannPre<T, FAST, Y> riemann_pre(const T ql[4], con
     h_t = (srl * h_l + srr * h_r) / denom_r;
   } else {
     // sqrt(rho) = rho r and sqrt(rho)*h = (E+p) r with r = 1/sqrt(rho) per side.
-    const T id = qrcp<T, FAST>(r.ql0 * rsl + r.qr0 * rsr);
+    const T id = qrcp<T, FAST>(sl + sr);
     u_t = sum_prod_rn<T>(ql[1], rsl, qr[1], rsr) * id;
     v_t = sum_prod_rn<T>(ql[2], rsl, qr[2], rsr) * id;
     h_t = ((ql[3] + r.p_l) * rsl + (qr[3] + r.p_r) * rsr) * id;
   }
   const T tmp = h_t - T(0.5) * (u_t * u_t + v_t * v_t);
-  const T a_t = qsqrt<T, FAST>(cmax<T, FAST>((gamma - T(1.0)) * tmp, T(0.0)));
+  const T a_t = sqrt(cmax<T, FAST>((gamma - T(1.0)) * tmp, T(0.0)));
   const T un_t = Y ? v_t : u_t;
   r.un_l = Y ? r.v_l : r.u_l;
   r.un_r = Y ? r.v_r : r.u_r;
@@ -1155,7 +1172,7 @@ __device__ __forceinline__ void hllc_flux(const RiemannPre<T, FAST, Y>& r, const
 // riemann.rs:394-405: blend weight from the normalised pressure gradient.
 template <class T, bool FAST>
 __device__ __forceinline__ T sensor_weight(T dpdx, T dpdy, T p, T jp_lo, T jp_hi) {
-  const T grad = qsqrt<T, FAST>(dpdx * dpdx + dpdy * dpdy);
+  const T grad = sqrt(T(dpdx * dpdx + dpdy * dpdy));
   const T jp = qdiv<T, FAST>(grad, vmax(p, T(kEps)));
   if (jp <= jp_lo) return T(1.0);
   if (jp >= jp_hi) return T(0.0);

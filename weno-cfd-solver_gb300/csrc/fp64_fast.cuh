@@ -1,9 +1,10 @@
 // FAST FP64 reciprocal, reciprocal square root and square root.
 //
-// GB300 runs FP64 at 1/64 of the FP32 rate, and CUDA's correctly rounded FP64
-// divide costs about ten FP64 pipe slots.  These forms take three
-// (reciprocal) or five (reciprocal square root) FP64 operations; the rest is
-// integer and FP32 work on pipes that the FP64-bound kernels leave idle.
+// Three FP64 operations (reciprocal) or five (reciprocal square root), the rest
+// integer and FP32 work.  The FP64 WENO weights, taken where the float pairs of
+// ffw.cuh do not reach, normalise with rcp2; the averages, fluxes and Riemann
+// solvers take the correctly rounded integer forms of rn64.cuh, which need no
+// FP64 slot at all.
 //
 // Method (Newton's iteration raised to third order, i.e. Householder's method
 // of order 2, on a hardware seed):
@@ -22,18 +23,17 @@
 // The reciprocal and the reciprocal square root are within 1 ulp, the square
 // root (x times its reciprocal square root) within 2 ulp.  Arguments whose
 // exponent lies outside [-1000, 1000] (zero, subnormals, infinities, NaN) and
-// negative arguments of the square roots take CUDA's IEEE operations.
+// negative arguments of the square roots take the correctly rounded operations.
 //
 // rcp2 stops the series after e (Newton's step, two FP64 operations): relative
-// error below 2^-41 (the seed's error squared).  It serves quotients whose
-// relative error only scales a small correction -- the normalisation of the
-// WENO weights, which multiplies the weighted slope added to a centre value,
-// and the shared 1/(rho_a rho_b) of two Euler fluxes.
+// error below 2^-41 (the seed's error squared), which in the normalisation of the
+// WENO weights only scales the weighted slope added to a centre value.
 #pragma once
 
 #include <cuda_runtime.h>
 
 #include "opaque64.cuh"
+#include "rn64.cuh"
 
 namespace weno {
 namespace f64fast {
@@ -63,6 +63,16 @@ __device__ __forceinline__ double widen(float f) {
 // exponent fexp.
 __device__ __forceinline__ float narrow(int hi, int lo, unsigned fexp) {
   return __uint_as_float((fexp << 23) | (((unsigned)hi & 0xfffffu) << 3) | ((unsigned)lo >> 29));
+}
+
+// The correctly rounded forms outside the fast range.
+__device__ __forceinline__ double rcp_rn(double x) {
+  return __longlong_as_double((long long)rn64::div(0x3ff0000000000000ull, (uint64_t)__double_as_longlong(x),
+                                                   [](float v) { return rcp_approx(v); }));
+}
+__device__ __forceinline__ double sqrt_rn(double x) {
+  return __longlong_as_double(
+      (long long)rn64::sqrt((uint64_t)__double_as_longlong(x), [](float v) { return rsqrt_approx(v); }));
 }
 
 __device__ __forceinline__ int biased_exp(int hi) { return (hi >> 20) & 0x7ff; }
@@ -103,14 +113,14 @@ __device__ __forceinline__ double rsqrt_core(int hi, int lo) {
 __device__ __forceinline__ double rcp(double x) {
   const int hi = __double2hiint(x), lo = __double2loint(x);
   const int ex = biased_exp(hi);
-  if (ex < kExpLo || ex > kExpHi) return 1.0 / x;
+  if (ex < kExpLo || ex > kExpHi) return rcp_rn(x);
   return rcp_core(hi, lo);
 }
 
 __device__ __forceinline__ double rcp2(double x) {
   const int hi = __double2hiint(x), lo = __double2loint(x);
   const int ex = biased_exp(hi);
-  if (ex < kExpLo || ex > kExpHi) return 1.0 / x;
+  if (ex < kExpLo || ex > kExpHi) return rcp_rn(x);
   return rcp2_core(hi, lo);
 }
 
@@ -124,7 +134,7 @@ __device__ __forceinline__ double rsqrt(double x) {
 __device__ __forceinline__ double sqrt(double x) {
   const int hi = __double2hiint(x), lo = __double2loint(x);
   const int ex = biased_exp(hi);
-  if (hi < 0 || ex < kExpLo || ex > kExpHi) return ::sqrt(x);
+  if (hi < 0 || ex < kExpLo || ex > kExpHi) return sqrt_rn(x);
   return xmul(x, rsqrt_core(hi, lo));
 }
 

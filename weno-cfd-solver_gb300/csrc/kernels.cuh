@@ -249,19 +249,18 @@ __device__ __forceinline__ void gq_side_two(const Planes<T>& P, int64_t row, int
       put4(a2B, k, mB);
     }
   }
-  const T h = SUM ? T(1.0) : T(0.5);
-  T f1[4], f2[4];
-  euler_flux_pair<T, true, Y>(a1A, a2A, gamma, f1, f2);
+  euler_flux_sum<T, Y>(a1A, a2A, gamma, fA);
+  euler_flux_sum<T, Y>(a1B, a2B, gamma, fB);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    fA[k] = SUM ? f1[k] + f2[k] : h * (f1[k] + f2[k]);
-    qA[k] = SUM ? a1A[k] + a2A[k] : h * (a1A[k] + a2A[k]);
-  }
-  euler_flux_pair<T, true, Y>(a1B, a2B, gamma, f1, f2);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    fB[k] = SUM ? f1[k] + f2[k] : h * (f1[k] + f2[k]);
-    qB[k] = SUM ? a1B[k] + a2B[k] : h * (a1B[k] + a2B[k]);
+    qA[k] = a1A[k] + a2A[k];
+    qB[k] = a1B[k] + a2B[k];
+    if constexpr (!SUM) {
+      fA[k] = half(fA[k]);
+      qA[k] = half(qA[k]);
+      fB[k] = half(fB[k]);
+      qB[k] = half(qB[k]);
+    }
   }
 }
 
@@ -299,9 +298,18 @@ __global__ void __launch_bounds__(128) k_pass2_two(Planes<T> PL, Planes<T> PR, i
     gq_side_two<T, Y, SUM>(PL, row, col, gamma, weps, qlA, flA, qlB, flB);
     gq_side_two<T, Y, SUM>(PR, row, col, gamma, weps, qrA, frA, qrB, frB);
   }
-  pass2_emit<T, true, Y, OUT, S>(qlA, flA, qrA, frA, gamma, dst, row, col, cols);
-  if (two)
-    pass2_emit<T, true, Y, OUT, S>(qlB, flB, qrB, frB, gamma, dst, Y ? row + 1 : row, Y ? col : col + 1, cols);
+  if constexpr (is_native_f64<T>) {
+#pragma unroll 1
+    for (int face = 0; face < (two ? 2 : 1); ++face) {
+      pass2_emit<T, true, Y, OUT, S>(qlA, flA, qrA, frA, gamma, dst, Y ? row + face : row, Y ? col : col + face, cols);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) qlA[k] = qlB[k], flA[k] = flB[k], qrA[k] = qrB[k], frA[k] = frB[k];
+    }
+  } else {
+    pass2_emit<T, true, Y, OUT, S>(qlA, flA, qrA, frA, gamma, dst, row, col, cols);
+    if (two)
+      pass2_emit<T, true, Y, OUT, S>(qlB, flB, qrB, frB, gamma, dst, Y ? row + 1 : row, Y ? col : col + 1, cols);
+  }
 }
 
 // Riemann solver on caller-provided dense (rows, cols, 4) face arrays
