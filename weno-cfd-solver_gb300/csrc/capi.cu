@@ -390,6 +390,10 @@ struct weno_solver {
 
 namespace {
 
+// pass 1 and 2 of both sweeps and the residual; two sensor blends; df64: the marked
+// faces of the two pass 1
+int launches_per_residual(const weno_solver* s) { return 5 + (s->force_hlle ? 0 : 2) + (s->prec == 48 ? 2 : 0); }
+
 HostPlanes state_planes(weno_solver* s, void* base) { return HostPlanes{base, s->PS, s->N}; }
 
 // Kernel classes of the timing report.
@@ -439,7 +443,7 @@ cudaError_t enqueue_step_t(weno_solver* s, int* launches) {
     if ((e = tm(TC_BC, false))) return e;
     nl += 1;
   }
-  const int per_residual = s->force_hlle ? 5 : 7;
+  const int per_residual = launches_per_residual(s);
   struct StageIO {
     void* in;
     HostPlanes qs, qo;
@@ -709,7 +713,7 @@ int weno_solver_launches_per_step(weno_solver* s) {
   if (!s) return 0;
   if (!s->launches) {
     // Count without enqueuing: the structure is fixed by the configuration.
-    const int per_residual = s->force_hlle ? 5 : 7;
+    const int per_residual = launches_per_residual(s);
     s->launches = 2 + (s->bc_kind == WENO_BC_TRANSMISSIVE ? 1 : 0) + 3 * (per_residual + 1) + 1;
   }
   return s->launches;

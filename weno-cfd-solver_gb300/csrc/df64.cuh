@@ -73,13 +73,27 @@ __device__ __forceinline__ df64 operator*(df64 a, df64 b) {
   return df64(p, e);
 }
 // Division: q1 = a.hi / b.hi (float), r = a - q1 * b, q2 = r.hi / b.hi, q1 + q2.
+// The float quotients are products with one hardware reciprocal after a Newton
+// step (within a unit in the last place of the IEEE quotient, whose own code is
+// several times longer); a power of two keeps that reciprocal normal at the ends
+// of the range.
 __device__ __forceinline__ df64 operator/(df64 a, df64 b) {
-  const float q1 = __fdiv_rn(a.hi, b.hi);
+  const float m = ::fabsf(b.hi);
+  const float s = m > 0x1p100f ? 0x1p-60f : (m < 0x1p-100f ? 0x1p60f : 1.0f);
+  const float bs = __fmul_rn(b.hi, s);
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(bs));
+  const float e = __fmaf_rn(-bs, y, 1.0f);
+  y = e == e ? __fmaf_rn(y, e, y) : y;
+  const float q1 = __fmul_rn(__fmul_rn(a.hi, s), y);
   const df64 r = a - b * df64(q1, 0.f);
-  const float q2 = __fdiv_rn(r.hi, b.hi);
-  float s, e;
-  dfd::quick_two_sum(q1, q2, s, e);
-  return df64(s, e);
+  float q2 = __fmul_rn(__fmul_rn(r.hi, s), y);
+  // what is left of r after q2, low parts included, rounds q2 correctly but for 2^-48
+  const float t = __fadd_rn(__fmaf_rn(-b.hi, q2, r.hi), __fmaf_rn(-b.lo, q2, r.lo));
+  q2 = t == t ? __fmaf_rn(__fmul_rn(t, s), y, q2) : q2;
+  float h, l;
+  dfd::quick_two_sum(q1, q2, h, l);
+  return df64(h, l);
 }
 __device__ __forceinline__ df64& operator+=(df64& a, df64 b) { return a = a + b; }
 
@@ -111,11 +125,21 @@ __device__ __forceinline__ df64 copysign(df64 mag, df64 sgn) {
 // s = x + (a - x*x) / (2x) in double-float arithmetic.
 __device__ __forceinline__ df64 sqrt(df64 a) {
   if (!(a.hi > 0.f)) return df64(sqrtf(a.hi), 0.f);  // 0, negative (NaN) or NaN
-  const float x = sqrtf(a.hi);
+  // the float root and the division by it come from one hardware reciprocal
+  // square root after a Newton step, scaled by a power of two at the ends of the range
+  const float k = a.hi > 0x1p100f ? 0x1p-60f : (a.hi < 0x1p-100f ? 0x1p60f : 1.0f);
+  const float g = k < 1.0f ? 0x1p30f : (k > 1.0f ? 0x1p-30f : 1.0f);  // 1 / sqrt(k)
+  const float as = __fmul_rn(a.hi, k);
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(as));
+  y = __fmaf_rn(__fmul_rn(0.5f, y), __fmaf_rn(-__fmul_rn(as, y), y, 1.0f), y);
+  const float x = __fmul_rn(__fmul_rn(as, y), g);
   float p, e;
   dfd::two_prod(x, x, p, e);
   const df64 r = a - df64(p, e);
-  const float corr = __fdiv_rn(r.hi, 2.f * x);
+  const float z = __fmul_rn(__fmul_rn(0.5f, y), __fmul_rn(k, g));  // 1 / (2 sqrt(a))
+  float corr = __fmul_rn(r.hi, z);
+  corr = __fmaf_rn(__fadd_rn(__fmaf_rn(-2.f * x, corr, r.hi), __fmaf_rn(-corr, corr, r.lo)), z, corr);
   float s, t;
   dfd::quick_two_sum(x, corr, s, t);
   return df64(s, t);

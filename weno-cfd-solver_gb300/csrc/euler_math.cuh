@@ -94,12 +94,12 @@ __device__ __forceinline__ T mul_pow2(T x) {
 template <class T>
 __device__ __forceinline__ T half(T x) { return mul_pow2<-1>(x); }
 
-// v[k] and v[k] = x for a run-time k without leaving registers.  The FP64 kernels
-// loop over the four fields: unrolled, their integer divisions (exact) or
-// float-pair weights (FAST) would not fit the instruction cache, and FP64 is
-// their bound, not the latency of one warp.
+// v[k] and v[k] = x for a run-time k without leaving registers.  The FP64 and df64
+// kernels loop over the four fields: unrolled, their integer divisions (exact) or
+// float-pair weights (FAST) would not fit the instruction cache, and FP64 or issue
+// slots are their bound, not the latency of one warp.
 template <class T>
-constexpr int kFieldUnroll = is_native_f64<T> ? 1 : 4;
+constexpr int kFieldUnroll = is_f32<T> ? 4 : 1;
 template <class T>
 __device__ __forceinline__ T pick4(const T v[4], int k) {
   const T a = (k & 1) ? v[1] : v[0], b = (k & 1) ? v[3] : v[2];
@@ -439,6 +439,29 @@ __device__ __forceinline__ void weno5_lr_ffw(f64 u2, f64 u3, f64 d0, f64 d1, f64
   right = u3 - face_slope(d2, d1, d3, d4, cn, cm, cf);
 }
 
+// The same in df64, whose values already are float pairs.
+__device__ __forceinline__ ffw::ff as_pair(df64 a) { return ffw::ff{a.hi, a.lo}; }
+__device__ __forceinline__ df64 from_pair(ffw::ff a) { return df64(a.h, a.l); }
+__device__ __forceinline__ df64 scaled(float c, df64 a) { return df64(c * a.hi, c * a.lo); }  // c a power of two
+__device__ __forceinline__ float max_head(df64 a, df64 b, df64 c, df64 d) {
+  return fmaxf(fmaxf(fabsf(a.hi), fabsf(b.hi)), fmaxf(fabsf(c.hi), fabsf(d.hi)));
+}
+__device__ __forceinline__ df64 face_slope(df64 dn, df64 fn, df64 dm, df64 df, ffw::ff c_near, ffw::ff c_mid,
+                                           ffw::ff c_far) {
+  return from_pair(c_near) * (scaled(4.0f, dn) - fn) +
+         (from_pair(c_mid) * (scaled(2.0f, dn) + dm) + from_pair(ffw::pow2(2.0f, c_far)) * (df64(2.5f, 0.0f) * dm - df));
+}
+__device__ __forceinline__ void weno5_lr_ffw(df64 u2, df64 u3, df64 d0, df64 d1, df64 d2, df64 d3, df64 d4, df64 weps,
+                                             df64& left, df64& right) {
+  const ffw::ff w = ffw::scale(0.75f, as_pair(weps));
+  const ffw::ff f0 = as_pair(d0), f1 = as_pair(d1), f2 = as_pair(d2), f3 = as_pair(d3), f4 = as_pair(d4);
+  ffw::ff cn, cm, cf;
+  ffw::face_weights(ffw::side(f2, f3, w), ffw::centre(f1, f2, w), ffw::side(f1, f0, w), cn, cm, cf);
+  left = u2 + face_slope(d2, d3, d1, d0, cn, cm, cf);
+  ffw::face_weights(ffw::side(f2, f1, w), ffw::centre(f2, f3, w), ffw::side(f3, f4, w), cn, cm, cf);
+  right = u3 - face_slope(d2, d1, d3, d4, cn, cm, cf);
+}
+
 // Both reconstructions of one field at one face (the right stencil is the left
 // one shifted by a cell), FAST: native double shares one divide
 // between the two; float and df64 take reciprocal weights.
@@ -450,6 +473,12 @@ __device__ __forceinline__ void weno5_lr_fast(T u0, T u1, T u2, T u3, T u4, T u5
   const T d0 = u1 - u0, d1 = u2 - u1, d2 = u3 - u2, d3 = u4 - u3, d4 = u5 - u4;
   if constexpr (is_native_f64<T>) {
     if (ffw::covers(max_magnitude(max_magnitude(d0, d1), max_magnitude(d2, d3), d4), weps.v)) {
+      weno5_lr_ffw(u2, u3, d0, d1, d2, d3, d4, weps, left, right);
+      return;
+    }
+  }
+  if constexpr (std::is_same<T, df64>::value) {
+    if (ffw::covers_pair(fmaxf(max_head(d0, d1, d2, d3), fabsf(d4.hi)), weps.hi)) {
       weno5_lr_ffw(u2, u3, d0, d1, d2, d3, d4, weps, left, right);
       return;
     }
@@ -591,6 +620,18 @@ __device__ __forceinline__ void gq_ffw(f64 q, f64 d0, f64 d1, f64 d2, f64 d3, ff
   rb = q + fma(f64(-cr), hr, fma(f64(cm), hm, f64(xmul(cl, hl.v))));
 }
 
+__device__ __forceinline__ void gq_ffw(df64 q, df64 d0, df64 d1, df64 d2, df64 d3, df64 weps, df64& ra, df64& rb) {
+  constexpr ffw::ff r0 = ffw::constant(kGqA0 / kGqA1), r2 = ffw::constant(kGqA2 / kGqA1), S = ffw::constant(kSqrt3_12);
+  const ffw::ff w = ffw::scale(0.75f, as_pair(weps)), f0 = as_pair(d0), f1 = as_pair(d1), f2 = as_pair(d2), f3 = as_pair(d3);
+  const ffw::ff qr = ffw::side(f2, f3, w), qm = ffw::centre(f1, f2, w), ql = ffw::side(f1, f0, w);
+  const df64 three(3.0f, 0.0f), hr = d3 - three * d2, hm = d1 + d2, hl = three * d1 - d0;
+  ffw::ff cr, cm, cl;
+  ffw::gauss_weights(qr, qm, ql, r0, r2, S, cr, cm, cl);
+  ra = q + (from_pair(cr) * hr - (from_pair(cm) * hm + from_pair(cl) * hl));
+  ffw::gauss_weights(qr, qm, ql, r2, r0, S, cr, cm, cl);
+  rb = q - (from_pair(cr) * hr - (from_pair(cm) * hm + from_pair(cl) * hl));
+}
+
 // Two neighbouring 5-cell stencils (q0..q4 and q1..q5), FAST: both
 // Gauss-point pairs, sharing the first and second differences.
 template <class T>
@@ -628,6 +669,12 @@ __device__ __forceinline__ void weno5_gq_pair(T q0, T q1, T q2, T q3, T q4, T& r
       if (ffw::covers(max(max_magnitude(d0, d1), max_magnitude(d2, d3)), weps.v)) {
         gq_ffw(q2, d0, d1, d2, d3, ffw::from_double(d0.v), ffw::from_double(d1.v), ffw::from_double(d2.v),
                ffw::from_double(d3.v), ffw::eps75(weps.v), ra, rb);
+        return;
+      }
+    }
+    if constexpr (std::is_same<T, df64>::value) {
+      if (ffw::covers_pair(max_head(d0, d1, d2, d3), weps.hi)) {
+        gq_ffw(q2, d0, d1, d2, d3, weps, ra, rb);
         return;
       }
     }
@@ -948,7 +995,7 @@ __device__ __forceinline__ void pass1_face(const T c[6][4], T gamma, T ql[4], T 
       k.b = (Y ? v_a : u_a) * ich;
       k.hr = ich * irho_a;
       const T weps2 = weps * (rho_a * rho_a);  // epsilon of the shear field rho w2
-      if constexpr (is_native_f64<T>) {
+      if constexpr (!is_f32<T>) {
         // the fields are G2 Z + Yv, q0 - G Z, q_t - u_t q0, G2 Z - Yv (project_left):
         // one product and one addend per cell, selected by field
         T Z[6], Yv[6];
@@ -963,7 +1010,7 @@ __device__ __forceinline__ void pass1_face(const T c[6][4], T gamma, T ql[4], T 
           for (int s = 0; s < 6; ++s) {
             const T X = f == 2 ? c[s][0] : Z[s];
             const T B = f == 0 ? Yv[s] : (f == 1 ? c[s][0] : (f == 2 ? c[s][Y ? 1 : 2] : -Yv[s]));
-            w[s] = fma(A, X, B);
+            w[s] = mul_add<T>(A, X, B);
           }
           weno5_lr_fast<T>(w[0], w[1], w[2], w[3], w[4], w[5], f == 2 ? weps2 : weps, l, r);
           put4(chl, f, l);
@@ -973,14 +1020,7 @@ __device__ __forceinline__ void pass1_face(const T c[6][4], T gamma, T ql[4], T 
         T w[6][4];
 #pragma unroll
         for (int s = 0; s < 6; ++s) project_left<T, Y>(k, c[s], w[s]);
-        if constexpr (is_f32<T>) {
-          weno5_lr_fast_f32_pairs(w, weps, chl, chr, weps2);
-        } else {
-#pragma unroll
-          for (int f = 0; f < 4; ++f)
-            weno5_lr_fast<T>(w[0][f], w[1][f], w[2][f], w[3][f], w[4][f], w[5][f], f == 2 ? weps2 : weps, chl[f],
-                             chr[f]);
-        }
+        weno5_lr_fast_f32_pairs(w, weps, chl, chr, weps2);
       }
       project_right<T, Y>(k, chl, ql);
       project_right<T, Y>(k, chr, qr);

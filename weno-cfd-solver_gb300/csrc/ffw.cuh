@@ -110,6 +110,11 @@ __device__ __forceinline__ bool covers(uint32_t dmax, double eps) {
          (uint32_t)__double2hiint(eps) - ((1023u - 58u) << 20) < ((58u + 40u) << 20);
 }
 
+// The same for float pairs.
+__device__ __forceinline__ bool covers_pair(float dmax, float eps) {
+  return dmax < 0x1p22f && eps >= 0x1p-58f && eps <= 0x1p40f;
+}
+
 // 0.75 eps.
 __device__ __forceinline__ ff eps75(double eps) { return scale(0.75f, from_double(eps)); }
 
@@ -128,11 +133,17 @@ __device__ __forceinline__ ff centre(ff a, ff b, ff w) {
 // largest formed as k less the other two: the weights then sum to k to 2^-50 and
 // an error of the two smaller ones only multiplies the difference of their
 // candidates to the largest one's.
-__device__ __forceinline__ void normalised(ff a0, ff a1, ff a2, ff r, ff k, double& c0, double& c1, double& c2) {
+__device__ __forceinline__ void take(ff a, double& c) { c = to_double(a); }
+__device__ __forceinline__ void take(ff a, ff& c) { c = a; }
+template <class C>  // double, or ff for the df64 kernels
+__device__ __forceinline__ void normalised(ff a0, ff a1, ff a2, ff r, ff k, C& c0, C& c1, C& c2) {
   const bool m0 = a0.h > a1.h && a0.h > a2.h, m2 = !m0 && a2.h > a1.h;  // largest: 0, 2 or else 1
   const ff x = mul(ff{m0 ? a1.h : a0.h, m0 ? a1.l : a0.l}, r);  // a1 where 0 is the largest, else a0
   const ff y = mul(ff{m2 ? a1.h : a2.h, m2 ? a1.l : a2.l}, r);  // a1 where 2 is the largest, else a2
-  const double cx = to_double(x), cy = to_double(y), cm = to_double(add(add(k, neg(x)), neg(y)));
+  C cx, cy, cm;
+  take(x, cx);
+  take(y, cy);
+  take(add(add(k, neg(x)), neg(y)), cm);
   c0 = m0 ? cm : cx;
   c1 = m0 ? cx : (m2 ? cy : cm);
   c2 = m2 ? cm : cy;
@@ -145,8 +156,8 @@ __device__ __forceinline__ double twice(double c) {
 
 // w/6 of a face state from the inverse squares of the stencil reaching over the
 // face (linear weight .3), the central one (.6) and the one on the other side (.1).
-__device__ __forceinline__ void face_weights(ff q_near, ff q_mid, ff q_far, double& c_near, double& c_mid,
-                                             double& c_far) {
+template <class C>
+__device__ __forceinline__ void face_weights(ff q_near, ff q_mid, ff q_far, C& c_near, C& c_mid, C& c_far) {
   constexpr ff sixth = constant(1.0 / 6.0);
   const ff a0 = scale(3.0f, q_near), a1 = pow2(2.0f, scale(3.0f, q_mid));
   const ff r = mul(sixth, rcp(add(add(a0, a1), q_far)));
@@ -155,8 +166,8 @@ __device__ __forceinline__ void face_weights(ff q_near, ff q_mid, ff q_far, doub
 
 // S w of one Gauss point from the inverse squares of the stencils on its side, in the
 // middle and on the other side; r0, r2 are the outer linear weights over the central one.
-__device__ __forceinline__ void gauss_weights(ff q0, ff q1, ff q2, ff r0, ff r2, ff S, double& c0, double& c1,
-                                              double& c2) {
+template <class C>
+__device__ __forceinline__ void gauss_weights(ff q0, ff q1, ff q2, ff r0, ff r2, ff S, C& c0, C& c1, C& c2) {
   const ff a0 = mul(r0, q0), a2 = mul(r2, q2);
   const ff r = mul(S, rcp(add(add(a0, a2), q1)));
   normalised(a0, q1, a2, r, S, c0, c1, c2);

@@ -42,6 +42,10 @@ struct Planes {
 // ---------------------------------------------------------------------------
 // Pass 1 (weno.rs:390-454 characteristic, weno.rs:654-717 component-wise)
 // ---------------------------------------------------------------------------
+// What the df64 pass 1 leaves in plane 0 of q_l for a face that k_pass1_marked has
+// to reconstruct: a NaN no arithmetic produces.
+constexpr uint32_t kDf64Marker = 0x7fc0df64u;
+
 template <class T, bool FAST, bool Y, bool CHAR>
 __global__ void __launch_bounds__(128) k_pass1(CView<T> u, int64_t rows, int64_t cols, T gamma, Planes<T> PL,
                                                 Planes<T> PR, T weps) {
@@ -57,7 +61,8 @@ __global__ void __launch_bounds__(128) k_pass1(CView<T> u, int64_t rows, int64_t
   if constexpr (std::is_same<T, df64>::value) {
     // df64 has the float exponent range: a face whose stencil holds a tiny
     // density or a huge value (near vacuum the characteristic projection scales
-    // by 1/(rho*c)) is reconstructed in native double instead.
+    // by 1/(rho*c)) is left to k_pass1_marked, in native double: with that code
+    // in this kernel its registers (168 against 96) would bind every face.
     bool safe = true;
 #pragma unroll
     for (int s = 0; s < 6; ++s) {
@@ -65,21 +70,11 @@ __global__ void __launch_bounds__(128) k_pass1(CView<T> u, int64_t rows, int64_t
 #pragma unroll
       for (int k = 0; k < 4; ++k) safe = safe && fabsf(c[s][k].hi) < 1e15f;
     }
-    if (safe) {
-      pass1_face<T, FAST, Y, CHAR>(c, gamma, ql, qr, weps);
-    } else {
-      f64 cd[6][4], l[4], r[4];
-#pragma unroll
-      for (int s = 0; s < 6; ++s)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) cd[s][k] = f64((double)c[s][k]);
-      pass1_face<f64, FAST, Y, CHAR>(cd, f64((double)gamma), l, r, f64((double)weps));
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        ql[k] = T(l[k].v);
-        qr[k] = T(r[k].v);
-      }
+    if (!safe) {
+      PL.at(0, row, col) = df64(__uint_as_float(kDf64Marker), 0.0f);
+      return;
     }
+    pass1_face<T, FAST, Y, CHAR>(c, gamma, ql, qr, weps);
   } else {
     pass1_face<T, FAST, Y, CHAR>(c, gamma, ql, qr, weps);
   }
@@ -87,6 +82,27 @@ __global__ void __launch_bounds__(128) k_pass1(CView<T> u, int64_t rows, int64_t
   for (int k = 0; k < 4; ++k) {
     PL.at(k, row, col) = ql[k];
     PR.at(k, row, col) = qr[k];
+  }
+}
+
+// The faces k_pass1<df64> marked, in native double.
+template <bool Y, bool CHAR>
+__global__ void __launch_bounds__(128) k_pass1_marked(CView<df64> u, int64_t rows, int64_t cols, df64 gamma,
+                                                       Planes<df64> PL, Planes<df64> PR, df64 weps) {
+  const int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t row = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;
+  if (row >= rows || col >= cols) return;
+  if (__float_as_uint(PL.at(0, row, col).hi) != kDf64Marker) return;
+  f64 c[6][4], l[4], r[4];
+#pragma unroll
+  for (int s = 0; s < 6; ++s)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c[s][k] = f64((double)(Y ? u.at(row, col + s, k) : u.at(row + s, col, k)));
+  pass1_face<f64, true, Y, CHAR>(c, f64((double)gamma), l, r, f64((double)weps));
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    PL.at(k, row, col) = df64(l[k].v);
+    PR.at(k, row, col) = df64(r[k].v);
   }
 }
 
@@ -197,7 +213,7 @@ __global__ void __launch_bounds__(128) k_pass2(Planes<T> PL, Planes<T> PR, int64
   const int64_t row = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;
   if (row >= rows || col >= cols) return;
   T ql[4], qr[4], fl[4], fr[4];
-#pragma unroll(FAST ? 2 : 1)
+#pragma unroll(is_f32<T> ? 2 : 1)
   for (int side = 0; side < 2; ++side) {
     T a1[4], a2[4], f1[4], f2[4];
     const Planes<T> P{side ? PR.p : PL.p, PL.ps, PL.ld};

@@ -53,6 +53,13 @@ cudaError_t Launch<H, FAST>::pass1(HostView u, int64_t rows, int64_t cols, doubl
   else if (!ydir) k_pass1<T, FAST, false, false><<<g, kBlk, 0, st>>>(U, rows, cols, (T)gamma, L, R, (T)weps);
   else if (chr) k_pass1<T, FAST, true, true><<<g, kBlk, 0, st>>>(U, rows, cols, (T)gamma, L, R, (T)weps);
   else k_pass1<T, FAST, true, false><<<g, kBlk, 0, st>>>(U, rows, cols, (T)gamma, L, R, (T)weps);
+  if constexpr (std::is_same<T, df64>::value) {  // reads one plane: 1 % of the pass
+    const T gm = (T)gamma, we = (T)weps;
+    if (!ydir && chr) k_pass1_marked<false, true><<<g, kBlk, 0, st>>>(U, rows, cols, gm, L, R, we);
+    else if (!ydir) k_pass1_marked<false, false><<<g, kBlk, 0, st>>>(U, rows, cols, gm, L, R, we);
+    else if (chr) k_pass1_marked<true, true><<<g, kBlk, 0, st>>>(U, rows, cols, gm, L, R, we);
+    else k_pass1_marked<true, false><<<g, kBlk, 0, st>>>(U, rows, cols, gm, L, R, we);
+  }
   return cudaGetLastError();
 }
 
