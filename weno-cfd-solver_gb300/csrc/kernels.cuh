@@ -39,6 +39,28 @@ struct Planes {
   __device__ __forceinline__ T& at(int k, int64_t r, int64_t c) const { return p[k * ps + r * ld + c]; }
 };
 
+// The (row, column) of this thread in a rows x cols index space: of a 2-D grid of
+// (32, 4) blocks, or with one-row blocks of the flattened space (launch_impl.cuh
+// says which is launched when).  False past the end.
+__device__ __forceinline__ bool locate(int64_t rows, int64_t cols, int64_t& row, int64_t& col) {
+  if (blockDim.y == 1) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= rows * cols) return false;
+    if (rows * cols < ((int64_t)1 << 32)) {
+      const uint32_t q = (uint32_t)e / (uint32_t)cols;
+      row = q;
+      col = (uint32_t)e - q * (uint32_t)cols;
+    } else {
+      row = e / cols;
+      col = e - row * cols;
+    }
+    return true;
+  }
+  col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  row = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;
+  return row < rows && col < cols;
+}
+
 // ---------------------------------------------------------------------------
 // Pass 1 (weno.rs:390-454 characteristic, weno.rs:654-717 component-wise)
 // ---------------------------------------------------------------------------
@@ -49,9 +71,8 @@ constexpr uint32_t kDf64Marker = 0x7fc0df64u;
 template <class T, bool FAST, bool Y, bool CHAR>
 __global__ void __launch_bounds__(128) k_pass1(CView<T> u, int64_t rows, int64_t cols, T gamma, Planes<T> PL,
                                                 Planes<T> PR, T weps) {
-  const int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t row = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;
-  if (row >= rows || col >= cols) return;
+  int64_t row, col;
+  if (!locate(rows, cols, row, col)) return;
   T c[6][4];
 #pragma unroll
   for (int s = 0; s < 6; ++s)
@@ -89,9 +110,8 @@ __global__ void __launch_bounds__(128) k_pass1(CView<T> u, int64_t rows, int64_t
 template <bool Y, bool CHAR>
 __global__ void __launch_bounds__(128) k_pass1_marked(CView<df64> u, int64_t rows, int64_t cols, df64 gamma,
                                                        Planes<df64> PL, Planes<df64> PR, df64 weps) {
-  const int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t row = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;
-  if (row >= rows || col >= cols) return;
+  int64_t row, col;
+  if (!locate(rows, cols, row, col)) return;
   if (__float_as_uint(PL.at(0, row, col).hi) != kDf64Marker) return;
   f64 c[6][4], l[4], r[4];
 #pragma unroll
@@ -113,11 +133,10 @@ __global__ void __launch_bounds__(128) k_pass1_marked(CView<df64> u, int64_t row
 template <bool Y>
 __global__ void __launch_bounds__(128) k_pass1_cons2(CView<f64> u, int64_t rows, int64_t cols, Planes<f64> PL,
                                                       Planes<f64> PR, f64 weps) {
-  int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int64_t row = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;
+  int64_t row, col;
+  if (!locate(Y ? rows : (rows + 1) / 2, Y ? (cols + 1) / 2 : cols, row, col)) return;
   if constexpr (Y) col *= 2;
   else row *= 2;
-  if (row >= rows || col >= cols) return;
   const bool two = Y ? (col + 1 < cols) : (row + 1 < rows);
   const int64_t rowB = Y ? row : row + 1, colB = Y ? col + 1 : col;
 #pragma unroll
@@ -209,9 +228,8 @@ __device__ __forceinline__ void pass2_emit(const T ql[4], const T fl[4], const T
 template <class T, bool FAST, bool Y, int OUT>
 __global__ void __launch_bounds__(128) k_pass2(Planes<T> PL, Planes<T> PR, int64_t rows, int64_t cols, T gamma,
                                                 Pass2Dst dst, T weps) {
-  const int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t row = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;
-  if (row >= rows || col >= cols) return;
+  int64_t row, col;
+  if (!locate(rows, cols, row, col)) return;
   T ql[4], qr[4], fl[4], fr[4];
 #pragma unroll(is_f32<T> ? 2 : 1)
   for (int side = 0; side < 2; ++side) {
@@ -287,11 +305,10 @@ __device__ __forceinline__ void gq_side_two(const Planes<T>& P, int64_t row, int
 template <class T, bool Y, int OUT>
 __global__ void __launch_bounds__(128) k_pass2_two(Planes<T> PL, Planes<T> PR, int64_t rows, int64_t cols, T gamma,
                                                     Pass2Dst dst, T weps) {
-  int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int64_t row = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;
+  int64_t row, col;
+  if (!locate(Y ? (rows + 1) / 2 : rows, Y ? cols : (cols + 1) / 2, row, col)) return;
   if constexpr (Y) row *= 2;
   else col *= 2;
-  if (row >= rows || col >= cols) return;
   const bool two = Y ? (row + 1 < rows) : (col + 1 < cols);
   // the HLLE flux takes the Gauss-point sums (twice the face averages)
   constexpr bool SUM = OUT == P2_HLLE;
@@ -336,9 +353,8 @@ template <class T, bool FAST, bool Y, int KIND>
 __global__ void __launch_bounds__(128) k_riemann(const T* QL, const T* FL, const T* QR, const T* FR, int64_t rows,
                                                   int64_t cols, T gamma, T* out, Planes<T> Fc, Planes<T> Fe,
                                                   Planes<T> Pbar) {
-  const int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t row = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;
-  if (row >= rows || col >= cols) return;
+  int64_t row, col;
+  if (!locate(rows, cols, row, col)) return;
   const int64_t o = (row * cols + col) * 4;
   T ql[4], qr[4], fl[4], fr[4];
 #pragma unroll
@@ -377,9 +393,8 @@ __global__ void __launch_bounds__(128) k_riemann(const T* QL, const T* FL, const
 template <class T, bool FAST, bool DENSE>
 __global__ void __launch_bounds__(128) k_blend(Planes<T> Fc, Planes<T> Fe, Planes<T> Pbar, int64_t rows,
                                                 int64_t cols, T jp_lo, T jp_hi, T* out, Planes<T> Fout) {
-  const int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t row = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;
-  if (row >= rows || col >= cols) return;
+  int64_t row, col;
+  if (!locate(rows, cols, row, col)) return;
   const int64_t min_dim = rows < cols ? rows : cols;
   const T dx = T(1.0) / T((double)min_dim);
   const T two_dx = T(2.0) * dx;
@@ -413,9 +428,8 @@ template <class T, bool FAST, int STAGE>
 __global__ void __launch_bounds__(128) k_residual(Planes<T> Fx, Planes<T> Fy, int64_t rows, int64_t cols, T dx,
                                                    T* out, Planes<T> Qn, Planes<T> Qs, Planes<T> Qo,
                                                    const StepCtl* ctl) {
-  const int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t row = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;
-  if (row >= rows || col >= cols) return;
+  int64_t row, col;
+  if (!locate(rows, cols, row, col)) return;
   if constexpr (STAGE > 0) {
     if (!ctl->active) return;
   }
@@ -676,9 +690,8 @@ __global__ void k_step_end(StepCtl* ctl) {
 // ---------------------------------------------------------------------------
 template <class T, bool FAST, bool Y>
 __global__ void k_flux(CView<T> q, int64_t rows, int64_t cols, T gamma, T* out) {
-  const int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t row = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;
-  if (row >= rows || col >= cols) return;
+  int64_t row, col;
+  if (!locate(rows, cols, row, col)) return;
   T s[4], f[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) s[k] = q.at(row, col, k);
@@ -689,9 +702,8 @@ __global__ void k_flux(CView<T> q, int64_t rows, int64_t cols, T gamma, T* out) 
 
 template <class T, bool FAST>
 __global__ void k_con2primi(CView<T> q, int64_t rows, int64_t cols, T gamma, T* p, T* a, T* rho, T* u, T* v, T* h) {
-  const int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t row = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;
-  if (row >= rows || col >= cols) return;
+  int64_t row, col;
+  if (!locate(rows, cols, row, col)) return;
   const int64_t e = row * cols + col;
   con2prim<T, FAST>(q.at(row, col, 0), q.at(row, col, 1), q.at(row, col, 2), q.at(row, col, 3), gamma, p[e], a[e],
                     rho[e], u[e], v[e], h[e]);

@@ -29,6 +29,25 @@ inline S3<T> s3(HostView v) {
 
 const dim3 kBlk(32, 4, 1);
 
+// Launch shape of a face or cell kernel over rows x cols threads.  FP64 and df64
+// kernels are bound by a pipe that serves one warp at a time, so what counts is
+// that no lane is idle and every SM has the same number of warps: the flattened
+// index space, in blocks of one warp while there are fewer than 32 warps per SM
+// (blocks of four would fill a part of the SMs, or leave a last wave).  FP32
+// kernels are issue bound and keep the 2-D blocks (no division for the index)
+// unless rounding the columns up to warps would idle more than 1 lane in 16.
+struct Shape {
+  dim3 grid, block;
+};
+template <class T>
+inline Shape shape(int64_t rows, int64_t cols) {
+  const int64_t padded = (cols + 31) / 32 * 32;
+  if (is_f32<T> && (padded - cols) * 16 <= padded) return Shape{grid2d(rows, cols, kBlk), kBlk};
+  const int64_t warps = (rows * cols + 31) / 32;
+  const unsigned block = warps < 152 * 32 ? 32 : 128;
+  return Shape{dim3((unsigned)((rows * cols + block - 1) / block), 1, 1), dim3(block, 1, 1)};
+}
+
 }  // namespace detail
 }  // inline namespace WENO_TU_NS
 
@@ -38,27 +57,27 @@ cudaError_t Launch<H, FAST>::pass1(HostView u, int64_t rows, int64_t cols, doubl
   using T = dev_t<H>;
   using namespace detail;
   if (rows <= 0 || cols <= 0) return cudaSuccess;
-  const dim3 g = grid2d(rows, cols, kBlk);
+  const Shape g = shape<T>(rows, cols);
   auto U = cview<T>(u);
   auto L = planes<T>(PL), R = planes<T>(PR);
   if constexpr (FAST && is_native_f64<T>) {
     if (!chr) {  // component-wise: two faces per thread along the sweep
-      const dim3 g2 = ydir ? grid2d(rows, (cols + 1) / 2, kBlk) : grid2d((rows + 1) / 2, cols, kBlk);
-      if (!ydir) k_pass1_cons2<false><<<g2, kBlk, 0, st>>>(U, rows, cols, L, R, weps);
-      else k_pass1_cons2<true><<<g2, kBlk, 0, st>>>(U, rows, cols, L, R, weps);
+      const Shape g2 = ydir ? shape<T>(rows, (cols + 1) / 2) : shape<T>((rows + 1) / 2, cols);
+      if (!ydir) k_pass1_cons2<false><<<g2.grid, g2.block, 0, st>>>(U, rows, cols, L, R, weps);
+      else k_pass1_cons2<true><<<g2.grid, g2.block, 0, st>>>(U, rows, cols, L, R, weps);
       return cudaGetLastError();
     }
   }
-  if (!ydir && chr) k_pass1<T, FAST, false, true><<<g, kBlk, 0, st>>>(U, rows, cols, (T)gamma, L, R, (T)weps);
-  else if (!ydir) k_pass1<T, FAST, false, false><<<g, kBlk, 0, st>>>(U, rows, cols, (T)gamma, L, R, (T)weps);
-  else if (chr) k_pass1<T, FAST, true, true><<<g, kBlk, 0, st>>>(U, rows, cols, (T)gamma, L, R, (T)weps);
-  else k_pass1<T, FAST, true, false><<<g, kBlk, 0, st>>>(U, rows, cols, (T)gamma, L, R, (T)weps);
+  if (!ydir && chr) k_pass1<T, FAST, false, true><<<g.grid, g.block, 0, st>>>(U, rows, cols, (T)gamma, L, R, (T)weps);
+  else if (!ydir) k_pass1<T, FAST, false, false><<<g.grid, g.block, 0, st>>>(U, rows, cols, (T)gamma, L, R, (T)weps);
+  else if (chr) k_pass1<T, FAST, true, true><<<g.grid, g.block, 0, st>>>(U, rows, cols, (T)gamma, L, R, (T)weps);
+  else k_pass1<T, FAST, true, false><<<g.grid, g.block, 0, st>>>(U, rows, cols, (T)gamma, L, R, (T)weps);
   if constexpr (std::is_same<T, df64>::value) {  // reads one plane: 1 % of the pass
     const T gm = (T)gamma, we = (T)weps;
-    if (!ydir && chr) k_pass1_marked<false, true><<<g, kBlk, 0, st>>>(U, rows, cols, gm, L, R, we);
-    else if (!ydir) k_pass1_marked<false, false><<<g, kBlk, 0, st>>>(U, rows, cols, gm, L, R, we);
-    else if (chr) k_pass1_marked<true, true><<<g, kBlk, 0, st>>>(U, rows, cols, gm, L, R, we);
-    else k_pass1_marked<true, false><<<g, kBlk, 0, st>>>(U, rows, cols, gm, L, R, we);
+    if (!ydir && chr) k_pass1_marked<false, true><<<g.grid, g.block, 0, st>>>(U, rows, cols, gm, L, R, we);
+    else if (!ydir) k_pass1_marked<false, false><<<g.grid, g.block, 0, st>>>(U, rows, cols, gm, L, R, we);
+    else if (chr) k_pass1_marked<true, true><<<g.grid, g.block, 0, st>>>(U, rows, cols, gm, L, R, we);
+    else k_pass1_marked<true, false><<<g.grid, g.block, 0, st>>>(U, rows, cols, gm, L, R, we);
   }
   return cudaGetLastError();
 }
@@ -70,15 +89,15 @@ cudaError_t Launch<H, FAST>::pass2(HostPlanes PL, HostPlanes PR, int64_t rows, i
   using T = dev_t<H>;
   using namespace detail;
   if (rows <= 0 || cols <= 0) return cudaSuccess;
-  const dim3 g = grid2d(rows, cols, kBlk);
+  const Shape g = shape<T>(rows, cols);
   auto L = planes<T>(PL), R = planes<T>(PR);
   Pass2Dst dst{a, b, c, d, ps, ld};
   const T gm = (T)gamma;
   if constexpr (FAST && !std::is_same<T, df64>::value) {
     // two faces per thread along the transverse direction (df64 keeps one:
     // its larger per-face register footprint outweighs the shared differences)
-    const dim3 g2 = ydir ? grid2d((rows + 1) / 2, cols, kBlk) : grid2d(rows, (cols + 1) / 2, kBlk);
-#define WENO_P2T(Y, K) k_pass2_two<T, Y, K><<<g2, kBlk, 0, st>>>(L, R, rows, cols, gm, dst, (T)weps)
+    const Shape g2 = ydir ? shape<T>((rows + 1) / 2, cols) : shape<T>(rows, (cols + 1) / 2);
+#define WENO_P2T(Y, K) k_pass2_two<T, Y, K><<<g2.grid, g2.block, 0, st>>>(L, R, rows, cols, gm, dst, (T)weps)
     if (!ydir) {
       if (kind == 0) WENO_P2T(false, P2_STATES);
       else if (kind == 1) WENO_P2T(false, P2_HLLE);
@@ -90,7 +109,7 @@ cudaError_t Launch<H, FAST>::pass2(HostPlanes PL, HostPlanes PR, int64_t rows, i
     }
 #undef WENO_P2T
   } else {
-#define WENO_P2(Y, K) k_pass2<T, FAST, Y, K><<<g, kBlk, 0, st>>>(L, R, rows, cols, gm, dst, (T)weps)
+#define WENO_P2(Y, K) k_pass2<T, FAST, Y, K><<<g.grid, g.block, 0, st>>>(L, R, rows, cols, gm, dst, (T)weps)
     if (!ydir) {
       if (kind == 0) WENO_P2(false, P2_STATES);
       else if (kind == 1) WENO_P2(false, P2_HLLE);
@@ -112,13 +131,13 @@ cudaError_t Launch<H, FAST>::riemann(const void* ql, const void* fl, const void*
   using T = dev_t<H>;
   using namespace detail;
   if (rows <= 0 || cols <= 0) return cudaSuccess;
-  const dim3 g = grid2d(rows, cols, kBlk);
+  const Shape g = shape<T>(rows, cols);
   const T *QL = static_cast<const T*>(ql), *FL = static_cast<const T*>(fl);
   const T *QR = static_cast<const T*>(qr), *FR = static_cast<const T*>(fr);
   Planes<T> A{static_cast<T*>(a), ps, ld}, B{static_cast<T*>(b), ps, ld}, C{static_cast<T*>(c), ps, ld};
   T* o = static_cast<T*>(out);
   const T gm = (T)gamma;
-#define WENO_RS(Y, K) k_riemann<T, FAST, Y, K><<<g, kBlk, 0, st>>>(QL, FL, QR, FR, rows, cols, gm, o, A, B, C)
+#define WENO_RS(Y, K) k_riemann<T, FAST, Y, K><<<g.grid, g.block, 0, st>>>(QL, FL, QR, FR, rows, cols, gm, o, A, B, C)
   if (!ydir) {
     if (kind == 0) WENO_RS(false, 0);
     else if (kind == 1) WENO_RS(false, 1);
@@ -138,10 +157,10 @@ cudaError_t Launch<H, FAST>::blend(HostPlanes Fc, HostPlanes Fe, HostPlanes Pbar
   using T = dev_t<H>;
   using namespace detail;
   if (rows <= 0 || cols <= 0) return cudaSuccess;
-  const dim3 g = grid2d(rows, cols, kBlk);
+  const Shape g = shape<T>(rows, cols);
   auto C = planes<T>(Fc), E = planes<T>(Fe), P = planes<T>(Pbar);
-  if (out) k_blend<T, FAST, true><<<g, kBlk, 0, st>>>(C, E, P, rows, cols, (T)jp_lo, (T)jp_hi, static_cast<T*>(out), C);
-  else k_blend<T, FAST, false><<<g, kBlk, 0, st>>>(C, E, P, rows, cols, (T)jp_lo, (T)jp_hi, nullptr, C);
+  if (out) k_blend<T, FAST, true><<<g.grid, g.block, 0, st>>>(C, E, P, rows, cols, (T)jp_lo, (T)jp_hi, static_cast<T*>(out), C);
+  else k_blend<T, FAST, false><<<g.grid, g.block, 0, st>>>(C, E, P, rows, cols, (T)jp_lo, (T)jp_hi, nullptr, C);
   return cudaGetLastError();
 }
 
@@ -152,14 +171,14 @@ cudaError_t Launch<H, FAST>::residual(HostPlanes Fx, HostPlanes Fy, int64_t rows
   using T = dev_t<H>;
   using namespace detail;
   if (rows <= 0 || cols <= 0) return cudaSuccess;
-  const dim3 g = grid2d(rows, cols, kBlk);
+  const Shape g = shape<T>(rows, cols);
   auto X = planes<T>(Fx), Yp = planes<T>(Fy), N = planes<T>(Qn), S = planes<T>(Qs), O = planes<T>(Qo);
   T* o = static_cast<T*>(out);
   switch (stage) {
-    case 0: k_residual<T, FAST, 0><<<g, kBlk, 0, st>>>(X, Yp, rows, cols, (T)dx, o, N, S, O, ctl); break;
-    case 1: k_residual<T, FAST, 1><<<g, kBlk, 0, st>>>(X, Yp, rows, cols, (T)dx, o, N, S, O, ctl); break;
-    case 2: k_residual<T, FAST, 2><<<g, kBlk, 0, st>>>(X, Yp, rows, cols, (T)dx, o, N, S, O, ctl); break;
-    default: k_residual<T, FAST, 3><<<g, kBlk, 0, st>>>(X, Yp, rows, cols, (T)dx, o, N, S, O, ctl); break;
+    case 0: k_residual<T, FAST, 0><<<g.grid, g.block, 0, st>>>(X, Yp, rows, cols, (T)dx, o, N, S, O, ctl); break;
+    case 1: k_residual<T, FAST, 1><<<g.grid, g.block, 0, st>>>(X, Yp, rows, cols, (T)dx, o, N, S, O, ctl); break;
+    case 2: k_residual<T, FAST, 2><<<g.grid, g.block, 0, st>>>(X, Yp, rows, cols, (T)dx, o, N, S, O, ctl); break;
+    default: k_residual<T, FAST, 3><<<g.grid, g.block, 0, st>>>(X, Yp, rows, cols, (T)dx, o, N, S, O, ctl); break;
   }
   return cudaGetLastError();
 }
@@ -170,9 +189,9 @@ cudaError_t Launch<H, FAST>::flux(HostView q, int64_t rows, int64_t cols, double
   using T = dev_t<H>;
   using namespace detail;
   if (rows <= 0 || cols <= 0) return cudaSuccess;
-  const dim3 g = grid2d(rows, cols, kBlk);
-  if (ydir) k_flux<T, FAST, true><<<g, kBlk, 0, st>>>(cview<T>(q), rows, cols, (T)gamma, static_cast<T*>(out));
-  else k_flux<T, FAST, false><<<g, kBlk, 0, st>>>(cview<T>(q), rows, cols, (T)gamma, static_cast<T*>(out));
+  const Shape g = shape<T>(rows, cols);
+  if (ydir) k_flux<T, FAST, true><<<g.grid, g.block, 0, st>>>(cview<T>(q), rows, cols, (T)gamma, static_cast<T*>(out));
+  else k_flux<T, FAST, false><<<g.grid, g.block, 0, st>>>(cview<T>(q), rows, cols, (T)gamma, static_cast<T*>(out));
   return cudaGetLastError();
 }
 
@@ -182,8 +201,8 @@ cudaError_t Launch<H, FAST>::con2primi(HostView q, int64_t rows, int64_t cols, d
   using T = dev_t<H>;
   using namespace detail;
   if (rows <= 0 || cols <= 0) return cudaSuccess;
-  const dim3 g = grid2d(rows, cols, kBlk);
-  k_con2primi<T, FAST><<<g, kBlk, 0, st>>>(cview<T>(q), rows, cols, (T)gamma, static_cast<T*>(p),
+  const Shape g = shape<T>(rows, cols);
+  k_con2primi<T, FAST><<<g.grid, g.block, 0, st>>>(cview<T>(q), rows, cols, (T)gamma, static_cast<T*>(p),
                                            static_cast<T*>(a), static_cast<T*>(rho), static_cast<T*>(u),
                                            static_cast<T*>(v), static_cast<T*>(h));
   return cudaGetLastError();
