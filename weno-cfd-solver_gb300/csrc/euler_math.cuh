@@ -106,6 +106,14 @@ __device__ __forceinline__ T pick4(const T v[4], int k) {
   return (k & 2) ? b : a;
 }
 template <class T>
+__device__ __forceinline__ void pick_row(const T M[4][4], int r, T row[4]) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const T col[4] = {M[0][c], M[1][c], M[2][c], M[3][c]};
+    row[c] = pick4(col, r);
+  }
+}
+template <class T>
 __device__ __forceinline__ void put4(T v[4], int k, T x) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) v[i] = k == i ? x : v[i];
@@ -878,6 +886,31 @@ __device__ __forceinline__ void project_parts(const CharScalars<T>& k, const T q
   Yv = k.b * q[0] - k.hr * q[Y ? 2 : 1];
 }
 template <class T, bool Y>
+__device__ __forceinline__ CharScalars<T> char_scalars(T rho, T u, T v, T h, T c, T ic, T irho, T gamma) {
+  CharScalars<T> k;
+  k.u = u;
+  k.v = v;
+  k.c = c;
+  k.rho = rho;
+  k.h = h;
+  k.kin = T(0.5) * (u * u + v * v);
+  k.G = (gamma - T(1.0)) * (ic * ic);
+  k.G2 = T(0.5) * k.G;
+  const T ich = T(0.5) * ic;
+  k.b = (Y ? v : u) * ich;
+  k.hr = ich * irho;
+  return k;
+}
+// Field f of a cell from its parts: G2 Z + Yv, q0 - G Z, q_t - u_t q0, G2 Z - Yv
+// as one product and one addend.
+template <class T, bool Y>
+__device__ __forceinline__ T char_field(const CharScalars<T>& k, const T q[4], T Z, T Yv, int f) {
+  const T A = f == 1 ? -k.G : (f == 2 ? -(Y ? k.u : k.v) : k.G2);
+  const T X = f == 2 ? q[0] : Z;
+  const T B = f == 0 ? Yv : (f == 1 ? q[0] : (f == 2 ? q[Y ? 1 : 2] : -Yv));
+  return mul_add<T>(A, X, B);
+}
+template <class T, bool Y>
 __device__ __forceinline__ void project_left(const CharScalars<T>& k, const T q[4], T w[4]) {
   // Z from q3 upwards and G Z / 2 +- Yv as one FMA each: nine operations
   T Z, Yv;
@@ -982,36 +1015,17 @@ __device__ __forceinline__ void pass1_face(const T c[6][4], T gamma, T ql[4], T 
     // cells 2|3), so six projections cover both.
     T chl[4], chr[4];
     if constexpr (FAST) {
-      CharScalars<T> k;
-      k.u = u_a;
-      k.v = v_a;
-      k.c = c_a;
-      k.rho = rho_a;
-      k.h = h_a;
-      k.kin = T(0.5) * (u_a * u_a + v_a * v_a);
-      k.G = (gamma - T(1.0)) * (ic_a * ic_a);
-      k.G2 = T(0.5) * k.G;
-      const T ich = T(0.5) * ic_a;
-      k.b = (Y ? v_a : u_a) * ich;
-      k.hr = ich * irho_a;
+      const CharScalars<T> k = char_scalars<T, Y>(rho_a, u_a, v_a, h_a, c_a, ic_a, irho_a, gamma);
       const T weps2 = weps * (rho_a * rho_a);  // epsilon of the shear field rho w2
       if constexpr (!is_f32<T>) {
-        // the fields are G2 Z + Yv, q0 - G Z, q_t - u_t q0, G2 Z - Yv (project_left):
-        // one product and one addend per cell, selected by field
         T Z[6], Yv[6];
 #pragma unroll
         for (int s = 0; s < 6; ++s) project_parts<T, Y>(k, c[s], Z[s], Yv[s]);
-        const T ut = Y ? k.u : k.v;
 #pragma unroll 1
         for (int f = 0; f < 4; ++f) {
-          const T A = f == 1 ? -k.G : (f == 2 ? -ut : k.G2);
           T w[6], l, r;
 #pragma unroll
-          for (int s = 0; s < 6; ++s) {
-            const T X = f == 2 ? c[s][0] : Z[s];
-            const T B = f == 0 ? Yv[s] : (f == 1 ? c[s][0] : (f == 2 ? c[s][Y ? 1 : 2] : -Yv[s]));
-            w[s] = mul_add<T>(A, X, B);
-          }
+          for (int s = 0; s < 6; ++s) w[s] = char_field<T, Y>(k, c[s], Z[s], Yv[s], f);
           weno5_lr_fast<T>(w[0], w[1], w[2], w[3], w[4], w[5], f == 2 ? weps2 : weps, l, r);
           put4(chl, f, l);
           put4(chr, f, r);
@@ -1030,11 +1044,8 @@ __device__ __forceinline__ void pass1_face(const T c[6][4], T gamma, T ql[4], T 
 #pragma unroll 1
       for (int f = 0; f < 4; ++f) {
         // characteristic field f of the six cells: row f of L times the cells
-        const T row[4] = {f < 2 ? (f == 0 ? Lm[0][0] : Lm[1][0]) : (f == 2 ? Lm[2][0] : Lm[3][0]),
-                          f < 2 ? (f == 0 ? Lm[0][1] : Lm[1][1]) : (f == 2 ? Lm[2][1] : Lm[3][1]),
-                          f < 2 ? (f == 0 ? Lm[0][2] : Lm[1][2]) : (f == 2 ? Lm[2][2] : Lm[3][2]),
-                          f < 2 ? (f == 0 ? Lm[0][3] : Lm[1][3]) : (f == 2 ? Lm[2][3] : Lm[3][3])};
-        T w[6], l, r;
+        T row[4], w[6], l, r;
+        pick_row(Lm, f, row);
 #pragma unroll
         for (int s = 0; s < 6; ++s) w[s] = row_vec4<T>(row, c[s]);
         weno5_lr_exact<T>(w, weps, l, r);
@@ -1048,6 +1059,65 @@ __device__ __forceinline__ void pass1_face(const T c[6][4], T gamma, T ql[4], T 
     }
     pp_limit<T, FAST>(ql, c[2], gamma);
     pp_limit<T, FAST>(qr, c[3], gamma);
+  }
+}
+
+// Pass 1 of one face by the four lanes of a quad, lane f reconstructing field f:
+// the operations of pass1_face, each on one lane only (the Roe average on all
+// four), and the fields exchanged by shuffles.  Returns component f of q_l and
+// q_r.  All 32 lanes of the warp call it.
+template <class T>
+__device__ __forceinline__ T quad_get(T x, int lane) {
+  return T(__shfl_sync(0xffffffffu, x.v, lane, 4));
+}
+template <class T>
+__device__ __forceinline__ void quad_gather(T x, T v[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v[k] = quad_get(x, k);
+}
+template <class T, bool FAST, bool Y, bool CHAR>
+__device__ __forceinline__ void pass1_face_quad(const T c[6][4], int f, T gamma, T& ql_f, T& qr_f, T weps) {
+  T w[6];
+  if constexpr (!CHAR) {
+#pragma unroll
+    for (int s = 0; s < 6; ++s) w[s] = pick4(c[s], f);
+    if constexpr (FAST) weno5_lr_fast<T>(w[0], w[1], w[2], w[3], w[4], w[5], weps, ql_f, qr_f);
+    else weno5_lr_exact<T>(w, weps, ql_f, qr_f);
+  } else {
+    T rho_a, u_a, v_a, h_a, c_a, ic_a = T(0.0), irho_a = T(0.0);
+    roe_avg<T, FAST>(c[2], c[3], gamma, rho_a, u_a, v_a, h_a, c_a, ic_a, irho_a);
+    T l, r, chl[4], chr[4], ql[4], qr[4];
+    if constexpr (FAST) {
+      const CharScalars<T> k = char_scalars<T, Y>(rho_a, u_a, v_a, h_a, c_a, ic_a, irho_a, gamma);
+#pragma unroll
+      for (int s = 0; s < 6; ++s) {
+        T Z, Yv;
+        project_parts<T, Y>(k, c[s], Z, Yv);
+        w[s] = char_field<T, Y>(k, c[s], Z, Yv, f);
+      }
+      weno5_lr_fast<T>(w[0], w[1], w[2], w[3], w[4], w[5], f == 2 ? T(weps * (rho_a * rho_a)) : weps, l, r);
+      quad_gather(l, chl);
+      quad_gather(r, chr);
+      project_right<T, Y>(k, chl, ql);
+      project_right<T, Y>(k, chr, qr);
+    } else {
+      T M[4][4], row[4];
+      left_eig<T, Y>(rho_a, u_a, v_a, c_a, gamma, M);
+      pick_row(M, f, row);
+#pragma unroll
+      for (int s = 0; s < 6; ++s) w[s] = row_vec4<T>(row, c[s]);
+      weno5_lr_exact<T>(w, weps, l, r);
+      quad_gather(l, chl);
+      quad_gather(r, chr);
+      right_eig<T, Y>(rho_a, u_a, v_a, h_a, c_a, M);
+      pick_row(M, f, row);
+      quad_gather(row_vec4<T>(row, chl), ql);
+      quad_gather(row_vec4<T>(row, chr), qr);
+    }
+    pp_limit<T, FAST>(ql, c[2], gamma);
+    pp_limit<T, FAST>(qr, c[3], gamma);
+    ql_f = pick4(ql, f);
+    qr_f = pick4(qr, f);
   }
 }
 

@@ -345,6 +345,106 @@ __global__ void __launch_bounds__(128) k_pass2_two(Planes<T> PL, Planes<T> PR, i
   }
 }
 
+// ---------------------------------------------------------------------------
+// Small FP64 grids: four lanes per face.  With fewer than about six warps per SM
+// the one-thread-per-face kernels wait for their own chain of dependent
+// operations (an FP64 one takes 64 cycles: a 64 x 64 residual spent 50 us in each
+// pass); a quad shares the fields of a face among its lanes, which costs a third
+// more FP64 instructions (the averages, repeated on four lanes) and leaves a
+// chain about a sixth as long.  The faces' values are those of k_pass1 / k_pass2 /
+// k_pass2_two operation by operation.
+// ---------------------------------------------------------------------------
+// The face (row, col) and component of this lane; lanes past the end work on the
+// last face and store nothing.
+__device__ __forceinline__ bool locate_quad(int64_t rows, int64_t cols, int64_t& row, int64_t& col, int& k) {
+  int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+  k = threadIdx.x & 3;
+  const bool in = e < rows * cols;
+  if (!in) e = rows * cols - 1;
+  row = e / cols;
+  col = e - row * cols;
+  return in;
+}
+
+template <bool FAST, bool Y, bool CHAR>
+__global__ void __launch_bounds__(32) k_pass1_quad(CView<f64> u, int64_t rows, int64_t cols, f64 gamma,
+                                                    Planes<f64> PL, Planes<f64> PR, f64 weps) {
+  int64_t row, col;
+  int k;
+  const bool in = locate_quad(rows, cols, row, col, k);
+  f64 c[6][4], l, r;
+#pragma unroll
+  for (int s = 0; s < 6; ++s)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) c[s][j] = Y ? u.at(row, col + s, j) : u.at(row + s, col, j);
+  pass1_face_quad<f64, FAST, Y, CHAR>(c, k, gamma, l, r, weps);
+  if (!in) return;
+  PL.at(k, row, col) = l;
+  PR.at(k, row, col) = r;
+}
+
+template <bool FAST, bool Y, int OUT>
+__global__ void __launch_bounds__(32) k_pass2_quad(Planes<f64> PL, Planes<f64> PR, int64_t rows, int64_t cols,
+                                                    f64 gamma, Pass2Dst dst, f64 weps) {
+  int64_t row, col;
+  int k;
+  const bool in = locate_quad(rows, cols, row, col, k);
+  constexpr bool SUM = FAST && OUT == P2_HLLE;
+  constexpr int S = SUM ? 2 : 1;
+  f64 ql[4], fl[4], qr[4], fr[4];
+#pragma unroll 1
+  for (int side = 0; side < 2; ++side) {
+    const Planes<f64> P{side ? PR.p : PL.p, PL.ps, PL.ld};
+    f64 s[5], a, b, a1[4], a2[4];
+#pragma unroll
+    for (int t = 0; t < 5; ++t) s[t] = Y ? P.at(k, row + 1 + t, col) : P.at(k, row, col + 1 + t);
+    weno5_gq_pair<f64, FAST>(s[0], s[1], s[2], s[3], s[4], a, b, weps);
+    quad_gather(a, a1);
+    quad_gather(b, a2);
+    f64 f[4];
+    if constexpr (FAST) {
+      euler_flux_sum<f64, Y>(a1, a2, gamma, f);
+    } else {
+      f64 f1[4], f2[4];
+      euler_flux_pair<f64, false, Y>(a1, a2, gamma, f1, f2);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) f[j] = f1[j] + f2[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const f64 q = SUM ? a1[j] + a2[j] : half(a1[j] + a2[j]);
+      const f64 g = SUM ? f[j] : half(f[j]);
+      ql[j] = side ? ql[j] : q;
+      fl[j] = side ? fl[j] : g;
+      qr[j] = q;
+      fr[j] = g;
+    }
+  }
+  const int64_t e = row * dst.ld + col;
+  if constexpr (OUT == P2_STATES) {
+    if (!in) return;
+    const int64_t o = (row * cols + col) * 4 + k;
+    static_cast<f64*>(dst.a)[o] = pick4(ql, k);
+    static_cast<f64*>(dst.b)[o] = pick4(fl, k);
+    static_cast<f64*>(dst.c)[o] = pick4(qr, k);
+    static_cast<f64*>(dst.d)[o] = pick4(fr, k);
+  } else {
+    const RiemannPre<f64, FAST, Y> r = riemann_pre<f64, FAST, Y, S>(ql, qr, gamma);
+    f64 F[4];
+    hlle_flux<f64, FAST, Y, S>(r, ql, fl, qr, fr, F);
+    if constexpr (OUT == P2_HLLE) {
+      if (in) static_cast<f64*>(dst.a)[k * dst.ps + e] = pick4(F, k);
+    } else {
+      f64 G[4];
+      hllc_flux<f64, FAST, Y>(r, ql, fl, qr, fr, G);
+      if (!in) return;
+      static_cast<f64*>(dst.a)[k * dst.ps + e] = pick4(G, k);
+      static_cast<f64*>(dst.b)[k * dst.ps + e] = pick4(F, k);
+      if (k == 0) static_cast<f64*>(dst.c)[e] = f64(0.5) * (r.p_l + r.p_r);
+    }
+  }
+}
+
 // Riemann solver on caller-provided dense (rows, cols, 4) face arrays
 // (hllc_x_rs_py & co, lib.rs:54-132).  KIND 0: HLLC -> out dense;
 // KIND 1: HLLE -> out dense; KIND 2: HLLC, HLLE and mean pressure -> planes
