@@ -54,20 +54,25 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 inline int64_t align_elems(int64_t x) { return (x + 63) / 64 * 64; }  // 256 B for f32, 512 B for f64
 
 // Workspace of the residual pipeline for an (m, n) array: pass-1 planes
-// (reused by both directions) and the face planes of x and y.
+// (reused by both directions, except by small FP64 grids, which run both at once)
+// and the face planes of x and y.
 struct ResidualLayout {
   int64_t m, n, P1, FX, FY;
   int nf;
   size_t es;
-  size_t off_pl, off_pr, off_fx, off_fy, total;
-  ResidualLayout(int64_t m_, int64_t n_, bool force_hlle, size_t es_) : m(m_), n(n_), es(es_) {
+  bool quads;
+  size_t off_pl, off_pr, off_ply, off_pry, off_fx, off_fy, total;
+  ResidualLayout(int64_t m_, int64_t n_, bool force_hlle, size_t es_, bool native_f64)
+      : m(m_), n(n_), es(es_), quads(native_f64 && quad_faces(m_, n_)) {
     P1 = align_elems(std::max((m - 5) * n, m * (n - 5)));
     FX = align_elems(std::max<int64_t>((m - 5) * (n - 6), 0));
     FY = align_elems(std::max<int64_t>((m - 6) * (n - 5), 0));
     nf = force_hlle ? 4 : 9;
     off_pl = 0;
     off_pr = off_pl + align_up(4 * P1 * es, 256);
-    off_fx = off_pr + align_up(4 * P1 * es, 256);
+    off_ply = quads ? off_pr + align_up(4 * P1 * es, 256) : off_pl;
+    off_pry = quads ? off_ply + align_up(4 * P1 * es, 256) : off_pr;
+    off_fx = off_pry + align_up(4 * P1 * es, 256);
     off_fy = off_fx + align_up(nf * FX * es, 256);
     total = off_fy + align_up(nf * FY * es, 256);
   }
@@ -93,7 +98,6 @@ cudaError_t residual_pipeline(HostView u, int64_t m, int64_t n, const ResidualLa
   T* fx = static_cast<T*>(at(ws, Lo.off_fx));
   T* fy = static_cast<T*>(at(ws, Lo.off_fy));
   cudaError_t e;
-  // x sweep
   HostPlanes PL{at(ws, Lo.off_pl), Lo.P1, n}, PR{at(ws, Lo.off_pr), Lo.P1, n};
 #define WENO_TIMED(cls, call)                              \
   do {                                                     \
@@ -101,19 +105,26 @@ cudaError_t residual_pipeline(HostView u, int64_t m, int64_t n, const ResidualLa
     if ((e = (call)) != cudaSuccess) return e;             \
     if ((e = tm(cls, false)) != cudaSuccess) return e;     \
   } while (0)
-  WENO_TIMED(HC_PASS1_X, Lx::pass1(u, m - 5, n, gamma, false, !cons, PL, PR, weps, st));
-  WENO_TIMED(HC_PASS2_X, Lx::pass2(PL, PR, m - 5, n - 6, gamma, false, kind, fx, fx + 4 * Lo.FX, fx + 8 * Lo.FX,
-                                   nullptr, Lo.FX, n - 6, weps, st));
+  if (Lo.quads) {
+    const HostPlanes P[4] = {PL, PR, {at(ws, Lo.off_ply), Lo.P1, n - 5}, {at(ws, Lo.off_pry), Lo.P1, n - 5}};
+    const FaceDst X{fx, fx + 4 * Lo.FX, fx + 8 * Lo.FX, nullptr, Lo.FX, n - 6};
+    const FaceDst Y{fy, fy + 4 * Lo.FY, fy + 8 * Lo.FY, nullptr, Lo.FY, n - 5};
+    WENO_TIMED(HC_PASS1_X, Lx::pass1_quads(u, m, n, 3, gamma, !cons, P, weps, st));
+    WENO_TIMED(HC_PASS2_X, Lx::pass2_quads(P, m, n, 3, gamma, kind, X, Y, weps, st));
+  } else {
+    WENO_TIMED(HC_PASS1_X, Lx::pass1(u, m - 5, n, gamma, false, !cons, PL, PR, weps, st));
+    WENO_TIMED(HC_PASS2_X, Lx::pass2(PL, PR, m - 5, n - 6, gamma, false, kind, fx, fx + 4 * Lo.FX, fx + 8 * Lo.FX,
+                                     nullptr, Lo.FX, n - 6, weps, st));
+    PL.ld = n - 5;
+    PR.ld = n - 5;
+    WENO_TIMED(HC_PASS1_Y, Lx::pass1(u, m, n - 5, gamma, true, !cons, PL, PR, weps, st));
+    WENO_TIMED(HC_PASS2_Y, Lx::pass2(PL, PR, m - 6, n - 5, gamma, true, kind, fy, fy + 4 * Lo.FY, fy + 8 * Lo.FY,
+                                     nullptr, Lo.FY, n - 5, weps, st));
+  }
   if (!force_hlle) {
     HostPlanes C{fx, Lo.FX, n - 6}, E{fx + 4 * Lo.FX, Lo.FX, n - 6}, P{fx + 8 * Lo.FX, Lo.FX, n - 6};
     WENO_TIMED(HC_BLEND, Lx::blend(C, E, P, m - 5, n - 6, jp_lo, jp_hi, nullptr, st));
   }
-  // y sweep
-  PL.ld = n - 5;
-  PR.ld = n - 5;
-  WENO_TIMED(HC_PASS1_Y, Lx::pass1(u, m, n - 5, gamma, true, !cons, PL, PR, weps, st));
-  WENO_TIMED(HC_PASS2_Y, Lx::pass2(PL, PR, m - 6, n - 5, gamma, true, kind, fy, fy + 4 * Lo.FY, fy + 8 * Lo.FY,
-                                   nullptr, Lo.FY, n - 5, weps, st));
   if (!force_hlle) {
     HostPlanes C{fy, Lo.FY, n - 5}, E{fy + 4 * Lo.FY, Lo.FY, n - 5}, P{fy + 8 * Lo.FY, Lo.FY, n - 5};
     WENO_TIMED(HC_BLEND, Lx::blend(C, E, P, m - 6, n - 5, jp_lo, jp_hi, nullptr, st));
@@ -212,6 +223,19 @@ int weno_reconstruct(const double* u, int64_t m, int64_t n, int64_t c, int64_t s
   HostPlanes PL{ws, P1, c1}, PR{at(ws, align_up(4 * P1 * sizeof(double), 256)), P1, c1};
   HostView v{u, s0, s1, s2};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (quad_faces(m, n)) {
+    const HostPlanes P[4] = {PL, PR, PL, PR};
+    const FaceDst D{q_l, f_l, q_r, f_r, 0, 0};
+    const int dirs = ydir ? 2 : 1;
+    if (mode == WENO_FAST) {
+      WENO_CK((Launch<double, true>::pass1_quads(v, m, n, dirs, gamma, cons == 0, P, 1e-12, st)));
+      WENO_CK((Launch<double, true>::pass2_quads(P, m, n, dirs, gamma, 0, D, D, 1e-12, st)));
+    } else {
+      WENO_CK((Launch<double, false>::pass1_quads(v, m, n, dirs, gamma, cons == 0, P, 1e-12, st)));
+      WENO_CK((Launch<double, false>::pass2_quads(P, m, n, dirs, gamma, 0, D, D, 1e-12, st)));
+    }
+    return WENO_OK;
+  }
   if (mode == WENO_FAST) {
     WENO_CK((Launch<double, true>::pass1(v, r1, c1, gamma, ydir != 0, cons == 0, PL, PR, 1e-12, st)));
     WENO_CK((Launch<double, true>::pass2(PL, PR, r2, c2, gamma, ydir != 0, 0, q_l, f_l, q_r, f_r, 0, 0, 1e-12, st)));
@@ -266,7 +290,7 @@ int weno_riemann(const double* q_l, const double* f_l, const double* q_r, const 
 
 size_t weno_l_local_workspace(int64_t m, int64_t n, int force_hlle) {
   if (m < 6 || n < 6) return 0;
-  return ResidualLayout(m, n, force_hlle != 0, sizeof(double)).total;
+  return ResidualLayout(m, n, force_hlle != 0, sizeof(double), true).total;
 }
 
 int weno_l_local(const double* u, int64_t m, int64_t n, int64_t c, int64_t s0, int64_t s1, int64_t s2, double dx,
@@ -280,7 +304,9 @@ int weno_l_local(const double* u, int64_t m, int64_t n, int64_t c, int64_t s0, i
   if (!force_hlle && (m < 8 || n < 8))
     return fail(WENO_ERR_SHAPE, "l_local: the HLLC/HLLE blend's shock sensor needs at least 8 x 8 cells, got "
                 "(%lld, %lld)", (long long)m, (long long)n);
-  ResidualLayout Lo(m, n, force_hlle != 0, sizeof(double));
+  ResidualLayout Lo(m, n, force_hlle != 0, sizeof(double), true);
+  if (ws_bytes < Lo.total)  // a workspace without room for both sweeps at once runs them in turn
+    Lo = ResidualLayout(m, n, force_hlle != 0, sizeof(double), false);
   if (!ws || ws_bytes < Lo.total) return fail(WENO_ERR_WORKSPACE, "l_local: workspace of %zu bytes needed", Lo.total);
   HostView v{u, s0, s1, s2};
   WENO_CK(residual_dispatch(mode, v, m, n, Lo, ws, gamma, dx, force_hlle != 0, jp_lo, jp_hi, cons != 0, out,
@@ -342,7 +368,7 @@ extern "C" int weno_l_local_host(const double* u, int64_t m, int64_t n, int64_t 
   }
   const size_t in_bytes = (size_t)(m * n * c) * sizeof(double);
   const size_t out_bytes = (size_t)((m - 6) * (n - 6) * 4) * sizeof(double);
-  ResidualLayout Lo(m, n, force_hlle != 0, sizeof(double));
+  ResidualLayout Lo(m, n, force_hlle != 0, sizeof(double), true);
   WENO_CK(grow(&hc.d_in, &hc.in_bytes, in_bytes));
   WENO_CK(grow(&hc.d_out, &hc.out_bytes, out_bytes));
   WENO_CK(grow(&hc.ws, &hc.ws_bytes, Lo.total));
@@ -392,7 +418,10 @@ namespace {
 
 // pass 1 and 2 of both sweeps and the residual; two sensor blends; df64: the marked
 // faces of the two pass 1
-int launches_per_residual(const weno_solver* s) { return 5 + (s->force_hlle ? 0 : 2) + (s->prec == 48 ? 2 : 0); }
+// faces of the two pass 1; small FP64 grids: both sweeps in one launch per pass
+int launches_per_residual(const weno_solver* s) {
+  return 5 + (s->force_hlle ? 0 : 2) + (s->prec == 48 ? 2 : 0) - (s->layout->quads ? 2 : 0);
+}
 
 HostPlanes state_planes(weno_solver* s, void* base) { return HostPlanes{base, s->PS, s->N}; }
 
@@ -544,7 +573,7 @@ int weno_solver_create(weno_solver** out, int64_t nx, int64_t ny, double dx, dou
   if ((e = cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, s->device)))
     return bail(e, "cudaDeviceGetAttribute");
   const size_t state_bytes = (size_t)(4 * s->PS) * s->es;
-  s->layout = new ResidualLayout(s->M, s->N, s->force_hlle, s->es);
+  s->layout = new ResidualLayout(s->M, s->N, s->force_hlle, s->es, precision == 64);
   if ((e = cudaMalloc(&s->q, state_bytes))) return bail(e, "cudaMalloc(state)");
   if ((e = cudaMalloc(&s->q1, state_bytes))) return bail(e, "cudaMalloc(stage 1)");
   if ((e = cudaMalloc(&s->q2, state_bytes))) return bail(e, "cudaMalloc(stage 2)");

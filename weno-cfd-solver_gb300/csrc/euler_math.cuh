@@ -336,17 +336,18 @@ __device__ __forceinline__ T weno_combine(T e0, T e1, T e2, T d0, T d1, T d2, T 
 // candidates: w0 p0 + w1 p1 + w2 p2.  The three divisions of each kind share
 // one piece of code (a loop): FP64 is the bound, not the latency of one warp,
 // and integer divisions unrolled at every use would not fit the instruction cache.
-template <class T>
+// U = 3 unrolls them, for the kernels that one warp's latency bounds.
+template <class T, int U = 1>
 __device__ __forceinline__ T weno_combine_exact(T e0, T e1, T e2, T d0, T d1, T d2, T p0, T p1, T p2) {
   T a0 = e0 * e0, a1 = e1 * e1, a2 = e2 * e2;
-#pragma unroll 1
+#pragma unroll(U)
   for (int k = 0; k < 3; ++k) {  // rotates (d, a) so that every k divides the front pair
     const T q = d0 / a0;
     a0 = a1, a1 = a2, a2 = q;
     d0 = d1, d1 = d2;
   }
   const T sum = a0 + a1 + a2;
-#pragma unroll 1
+#pragma unroll(U)
   for (int k = 0; k < 3; ++k) {
     const T w = a0 / sum;
     a0 = a1, a1 = a2, a2 = w;
@@ -397,12 +398,12 @@ __device__ __forceinline__ void div_pair(f64 a, f64 b, f64 c, f64 d, f64& x, f64
 // weno.rs:214-257, exact: the left-biased value at the right face of u2 and the
 // right-biased one at the left face of u3, the reference's operations.  The
 // right stencils are the left ones shifted by a cell, so one loop body serves both.
-template <class T>
+template <class T, int U = 1>
 __device__ __forceinline__ void weno5_lr_exact(const T u[6], T weps, T& left, T& right) {
   // candidate polynomials (x6): two are shared by the two sides
   const T f1 = -u[4] + T(5.0) * u[3] + mul_pow2<1>(u[2]);
   const T f2 = -u[1] + T(5.0) * u[2] + mul_pow2<1>(u[3]);
-#pragma unroll 1
+#pragma unroll(U == 1 ? 1 : 2)
   for (int side = 0; side < 2; ++side) {
     const T v0 = side ? u[1] : u[0], v1 = side ? u[2] : u[1], v2 = side ? u[3] : u[2], v3 = side ? u[4] : u[3],
             v4 = side ? u[5] : u[4];
@@ -410,7 +411,7 @@ __device__ __forceinline__ void weno5_lr_exact(const T u[6], T weps, T& left, T&
     js_betas(v0, v1, v2, v3, v4, b0, b1, b2);
     // 2 u0 - 7 u1 + 11 u2 (left, third candidate), 2 u5 - 7 u4 + 11 u3 (right, first)
     const T g = mul_pow2<1>(side ? u[5] : u[0]) - T(7.0) * (side ? u[4] : u[1]) + T(11.0) * v2;
-    const T r = weno_combine_exact<T>(weps + b0, weps + b1, weps + b2, side ? T(0.1) : T(0.3), T(0.6),
+    const T r = weno_combine_exact<T, U>(weps + b0, weps + b1, weps + b2, side ? T(0.1) : T(0.3), T(0.6),
                                       side ? T(0.3) : T(0.1), side ? g : f1, side ? f1 : f2, side ? f2 : g) /
                 T(6.0);
     left = side ? left : r;
@@ -666,7 +667,7 @@ __device__ __forceinline__ void weno5_gq_two(T q0, T q1, T q2, T q3, T q4, T q5,
   gq_weights<T>(q3, hB0, hB1, hB2, hB0 * hB0 + C4, hB1 * hB1 + C3, hB2 * hB2 + C2, raB, rbB);
 }
 
-template <class T, bool FAST>
+template <class T, bool FAST, int U = 1>
 __device__ __forceinline__ void weno5_gq_pair(T q0, T q1, T q2, T q3, T q4, T& ra, T& rb, T weps) {
   const T S = T(kSqrt3_12);
   if constexpr (FAST) {
@@ -705,9 +706,9 @@ __device__ __forceinline__ void weno5_gq_pair(T q0, T q1, T q2, T q3, T q4, T& r
     // point a: q2 + g0, q2 - (q3 - q1) S, q2 - g2; point b: the mirror (negation
     // is exact: -q1 + q3 and q1 - q3 are opposite)
     const T g1 = (-q1 + q3) * S;
-#pragma unroll 1
+#pragma unroll(U == 1 ? 1 : 2)
     for (int pt = 0; pt < 2; ++pt) {
-      const T r = weno_combine_exact<T>(e0, e1, e2, pt ? T(kGqA2) : T(kGqA0), T(kGqA1), pt ? T(kGqA0) : T(kGqA2),
+      const T r = weno_combine_exact<T, U>(e0, e1, e2, pt ? T(kGqA2) : T(kGqA0), T(kGqA1), pt ? T(kGqA0) : T(kGqA2),
                                         q2 + (pt ? -g0 : g0), q2 - (pt ? -g1 : g1), q2 - (pt ? -g2 : g2));
       ra = pt ? ra : r;
       rb = r;
@@ -1082,7 +1083,7 @@ __device__ __forceinline__ void pass1_face_quad(const T c[6][4], int f, T gamma,
 #pragma unroll
     for (int s = 0; s < 6; ++s) w[s] = pick4(c[s], f);
     if constexpr (FAST) weno5_lr_fast<T>(w[0], w[1], w[2], w[3], w[4], w[5], weps, ql_f, qr_f);
-    else weno5_lr_exact<T>(w, weps, ql_f, qr_f);
+    else weno5_lr_exact<T, 3>(w, weps, ql_f, qr_f);
   } else {
     T rho_a, u_a, v_a, h_a, c_a, ic_a = T(0.0), irho_a = T(0.0);
     roe_avg<T, FAST>(c[2], c[3], gamma, rho_a, u_a, v_a, h_a, c_a, ic_a, irho_a);
@@ -1106,7 +1107,7 @@ __device__ __forceinline__ void pass1_face_quad(const T c[6][4], int f, T gamma,
       pick_row(M, f, row);
 #pragma unroll
       for (int s = 0; s < 6; ++s) w[s] = row_vec4<T>(row, c[s]);
-      weno5_lr_exact<T>(w, weps, l, r);
+      weno5_lr_exact<T, 3>(w, weps, l, r);
       quad_gather(l, chl);
       quad_gather(r, chr);
       right_eig<T, Y>(rho_a, u_a, v_a, h_a, c_a, M);

@@ -349,15 +349,16 @@ __global__ void __launch_bounds__(128) k_pass2_two(Planes<T> PL, Planes<T> PR, i
 // Small FP64 grids: four lanes per face.  With fewer than about six warps per SM
 // the one-thread-per-face kernels wait for their own chain of dependent
 // operations (an FP64 one takes 64 cycles: a 64 x 64 residual spent 50 us in each
-// pass); a quad shares the fields of a face among its lanes, which costs a third
+// of four passes); a quad shares the fields of a face among its lanes, which costs a third
 // more FP64 instructions (the averages, repeated on four lanes) and leaves a
 // chain about a sixth as long.  The faces' values are those of k_pass1 / k_pass2 /
 // k_pass2_two operation by operation.
 // ---------------------------------------------------------------------------
 // The face (row, col) and component of this lane; lanes past the end work on the
 // last face and store nothing.
-__device__ __forceinline__ bool locate_quad(int64_t rows, int64_t cols, int64_t& row, int64_t& col, int& k) {
-  int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+__device__ __forceinline__ bool locate_quad(unsigned block, int64_t rows, int64_t cols, int64_t& row, int64_t& col,
+                                            int& k) {
+  int64_t e = ((int64_t)block * blockDim.x + threadIdx.x) >> 2;
   k = threadIdx.x & 3;
   const bool in = e < rows * cols;
   if (!in) e = rows * cols - 1;
@@ -367,11 +368,11 @@ __device__ __forceinline__ bool locate_quad(int64_t rows, int64_t cols, int64_t&
 }
 
 template <bool FAST, bool Y, bool CHAR>
-__global__ void __launch_bounds__(32) k_pass1_quad(CView<f64> u, int64_t rows, int64_t cols, f64 gamma,
-                                                    Planes<f64> PL, Planes<f64> PR, f64 weps) {
+__device__ __forceinline__ void pass1_quad(unsigned block, const CView<f64>& u, int64_t rows, int64_t cols, f64 gamma,
+                                           const Planes<f64>& PL, const Planes<f64>& PR, f64 weps) {
   int64_t row, col;
   int k;
-  const bool in = locate_quad(rows, cols, row, col, k);
+  const bool in = locate_quad(block, rows, cols, row, col, k);
   f64 c[6][4], l, r;
 #pragma unroll
   for (int s = 0; s < 6; ++s)
@@ -383,22 +384,32 @@ __global__ void __launch_bounds__(32) k_pass1_quad(CView<f64> u, int64_t rows, i
   PR.at(k, row, col) = r;
 }
 
+// Pass 1 of an (m, n) array: the first nbx blocks the x faces, the others the y
+// faces (either may be none), so that one launch covers both sweeps.
+template <bool FAST, bool CHAR>
+__global__ void __launch_bounds__(32) k_pass1_quad(CView<f64> u, int64_t m, int64_t n, unsigned nbx, f64 gamma,
+                                                    Planes<f64> PLx, Planes<f64> PRx, Planes<f64> PLy,
+                                                    Planes<f64> PRy, f64 weps) {
+  if (blockIdx.x < nbx) pass1_quad<FAST, false, CHAR>(blockIdx.x, u, m - 5, n, gamma, PLx, PRx, weps);
+  else pass1_quad<FAST, true, CHAR>(blockIdx.x - nbx, u, m, n - 5, gamma, PLy, PRy, weps);
+}
+
 template <bool FAST, bool Y, int OUT>
-__global__ void __launch_bounds__(32) k_pass2_quad(Planes<f64> PL, Planes<f64> PR, int64_t rows, int64_t cols,
-                                                    f64 gamma, Pass2Dst dst, f64 weps) {
+__device__ __forceinline__ void pass2_quad(unsigned block, const Planes<f64>& PL, const Planes<f64>& PR, int64_t rows,
+                                           int64_t cols, f64 gamma, const Pass2Dst& dst, f64 weps) {
   int64_t row, col;
   int k;
-  const bool in = locate_quad(rows, cols, row, col, k);
+  const bool in = locate_quad(block, rows, cols, row, col, k);
   constexpr bool SUM = FAST && OUT == P2_HLLE;
   constexpr int S = SUM ? 2 : 1;
   f64 ql[4], fl[4], qr[4], fr[4];
-#pragma unroll 1
+#pragma unroll
   for (int side = 0; side < 2; ++side) {
     const Planes<f64> P{side ? PR.p : PL.p, PL.ps, PL.ld};
     f64 s[5], a, b, a1[4], a2[4];
 #pragma unroll
     for (int t = 0; t < 5; ++t) s[t] = Y ? P.at(k, row + 1 + t, col) : P.at(k, row, col + 1 + t);
-    weno5_gq_pair<f64, FAST>(s[0], s[1], s[2], s[3], s[4], a, b, weps);
+    weno5_gq_pair<f64, FAST, 3>(s[0], s[1], s[2], s[3], s[4], a, b, weps);
     quad_gather(a, a1);
     quad_gather(b, a2);
     f64 f[4];
@@ -443,6 +454,15 @@ __global__ void __launch_bounds__(32) k_pass2_quad(Planes<f64> PL, Planes<f64> P
       if (k == 0) static_cast<f64*>(dst.c)[e] = f64(0.5) * (r.p_l + r.p_r);
     }
   }
+}
+
+// Pass 2 of the same: (m-5) x (n-6) x faces, then (m-6) x (n-5) y faces.
+template <bool FAST, int OUT>
+__global__ void __launch_bounds__(32) k_pass2_quad(Planes<f64> PLx, Planes<f64> PRx, Planes<f64> PLy, Planes<f64> PRy,
+                                                    int64_t m, int64_t n, unsigned nbx, f64 gamma, Pass2Dst dx,
+                                                    Pass2Dst dy, f64 weps) {
+  if (blockIdx.x < nbx) pass2_quad<FAST, false, OUT>(blockIdx.x, PLx, PRx, m - 5, n - 6, gamma, dx, weps);
+  else pass2_quad<FAST, true, OUT>(blockIdx.x - nbx, PLy, PRy, m - 6, n - 5, gamma, dy, weps);
 }
 
 // Riemann solver on caller-provided dense (rows, cols, 4) face arrays

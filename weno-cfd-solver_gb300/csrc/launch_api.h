@@ -23,6 +23,22 @@ struct HostPlanes {
   int64_t ps, ld;
 };
 
+// Where pass 2 puts its faces (see Launch::pass2).
+struct FaceDst {
+  void *a, *b, *c, *d;
+  int64_t ps, ld;
+};
+
+// FP64 grids of at most this many faces per sweep take four lanes per face and one
+// launch for both sweeps (Launch::pass1_quads, pass2_quads): six warps per SM of
+// the one-thread form.  Below, that form is a chain of dependent operations (64 x 64
+// residual: 4 x 50 us in its passes); above, the FP64 pipe is busy and the quads'
+// repeated averages cost a third more of it.
+constexpr int64_t kQuadFaces = (int64_t)152 * 6 * 32;
+inline bool quad_faces(int64_t m, int64_t n) {
+  return m > 5 && n > 5 && (m - 5) * n <= kQuadFaces && m * (n - 5) <= kQuadFaces;
+}
+
 struct StepCtl;
 namespace dfm {
 struct df64;
@@ -39,6 +55,12 @@ struct Launch {
   static cudaError_t pass2(HostPlanes PL, HostPlanes PR, int64_t rows, int64_t cols, double gamma, bool ydir,
                            int kind, void* a, void* b, void* c, void* d, int64_t ps, int64_t ld, double weps,
                            cudaStream_t st);
+  // Both passes of an (m, n) array with four lanes per face (double only): dirs 1 the
+  // x sweep, 2 the y sweep, 3 both in one launch; P holds q_l, q_r of x, then of y.
+  static cudaError_t pass1_quads(HostView u, int64_t m, int64_t n, int dirs, double gamma, bool chr,
+                                 const HostPlanes P[4], double weps, cudaStream_t st);
+  static cudaError_t pass2_quads(const HostPlanes P[4], int64_t m, int64_t n, int dirs, double gamma, int kind,
+                                 const FaceDst& x, const FaceDst& y, double weps, cudaStream_t st);
   // Riemann solver on dense (rows, cols, 4) face arrays.  kind 0 HLLC / 1 HLLE
   // -> dense out; kind 2 -> planes Fc (a), Fe (b), pbar (c).
   static cudaError_t riemann(const void* ql, const void* fl, const void* qr, const void* fr, int64_t rows,

@@ -48,15 +48,9 @@ inline Shape shape(int64_t rows, int64_t cols) {
   return Shape{dim3((unsigned)((rows * cols + block - 1) / block), 1, 1), dim3(block, 1, 1)};
 }
 
-// Four lanes per face (k_pass1_quad, k_pass2_quad) up to six warps per SM of the
-// one-thread form: below, that form is a chain of dependent operations (64 x 64
-// residual: 50 us in each pass against 9 with quads); above, the FP64 pipe is busy
-// and the quads' repeated averages cost a third more of it.
-template <class T>
-inline bool use_quads(int64_t rows, int64_t cols) {
-  return is_native_f64<T> && rows * cols <= (int64_t)152 * 6 * 32;
+inline unsigned quad_blocks(int64_t rows, int64_t cols) {
+  return rows > 0 && cols > 0 ? (unsigned)((rows * cols * 4 + 31) / 32) : 0u;
 }
-inline unsigned quad_grid(int64_t rows, int64_t cols) { return (unsigned)((rows * cols * 4 + 31) / 32); }
 
 }  // namespace detail
 }  // inline namespace WENO_TU_NS
@@ -70,17 +64,6 @@ cudaError_t Launch<H, FAST>::pass1(HostView u, int64_t rows, int64_t cols, doubl
   const Shape g = shape<T>(rows, cols);
   auto U = cview<T>(u);
   auto L = planes<T>(PL), R = planes<T>(PR);
-  if constexpr (is_native_f64<T>) {
-    if (use_quads<T>(rows, cols)) {
-      const unsigned n = quad_grid(rows, cols);
-      const T gm = (T)gamma, we = (T)weps;
-      if (!ydir && chr) k_pass1_quad<FAST, false, true><<<n, 32, 0, st>>>(U, rows, cols, gm, L, R, we);
-      else if (!ydir) k_pass1_quad<FAST, false, false><<<n, 32, 0, st>>>(U, rows, cols, gm, L, R, we);
-      else if (chr) k_pass1_quad<FAST, true, true><<<n, 32, 0, st>>>(U, rows, cols, gm, L, R, we);
-      else k_pass1_quad<FAST, true, false><<<n, 32, 0, st>>>(U, rows, cols, gm, L, R, we);
-      return cudaGetLastError();
-    }
-  }
   if constexpr (FAST && is_native_f64<T>) {
     if (!chr) {  // component-wise: two faces per thread along the sweep
       const Shape g2 = ydir ? shape<T>(rows, (cols + 1) / 2) : shape<T>((rows + 1) / 2, cols);
@@ -114,23 +97,6 @@ cudaError_t Launch<H, FAST>::pass2(HostPlanes PL, HostPlanes PR, int64_t rows, i
   auto L = planes<T>(PL), R = planes<T>(PR);
   Pass2Dst dst{a, b, c, d, ps, ld};
   const T gm = (T)gamma;
-  if constexpr (is_native_f64<T>) {
-    if (use_quads<T>(rows, cols)) {
-      const unsigned n = quad_grid(rows, cols);
-#define WENO_P2Q(Y, K) k_pass2_quad<FAST, Y, K><<<n, 32, 0, st>>>(L, R, rows, cols, gm, dst, (T)weps)
-      if (!ydir) {
-        if (kind == 0) WENO_P2Q(false, P2_STATES);
-        else if (kind == 1) WENO_P2Q(false, P2_HLLE);
-        else WENO_P2Q(false, P2_BLEND);
-      } else {
-        if (kind == 0) WENO_P2Q(true, P2_STATES);
-        else if (kind == 1) WENO_P2Q(true, P2_HLLE);
-        else WENO_P2Q(true, P2_BLEND);
-      }
-#undef WENO_P2Q
-      return cudaGetLastError();
-    }
-  }
   if constexpr (FAST && !std::is_same<T, df64>::value) {
     // two faces per thread along the transverse direction (df64 keeps one:
     // its larger per-face register footprint outweighs the shared differences)
@@ -160,6 +126,45 @@ cudaError_t Launch<H, FAST>::pass2(HostPlanes PL, HostPlanes PR, int64_t rows, i
 #undef WENO_P2
   }
   return cudaGetLastError();
+}
+
+template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::pass1_quads(HostView u, int64_t m, int64_t n, int dirs, double gamma, bool chr,
+                                         const HostPlanes P[4], double weps, cudaStream_t st) {
+  using T = dev_t<H>;
+  using namespace detail;
+  if constexpr (is_native_f64<T>) {
+    const unsigned bx = (dirs & 1) ? quad_blocks(m - 5, n) : 0, by = (dirs & 2) ? quad_blocks(m, n - 5) : 0;
+    if (bx + by == 0) return cudaSuccess;
+    const auto U = cview<T>(u);
+    const T gm = (T)gamma, we = (T)weps;
+    const auto A = planes<T>(P[0]), B = planes<T>(P[1]), C = planes<T>(P[2]), D = planes<T>(P[3]);
+    if (chr) k_pass1_quad<FAST, true><<<bx + by, 32, 0, st>>>(U, m, n, bx, gm, A, B, C, D, we);
+    else k_pass1_quad<FAST, false><<<bx + by, 32, 0, st>>>(U, m, n, bx, gm, A, B, C, D, we);
+    return cudaGetLastError();
+  } else {
+    return cudaErrorNotSupported;
+  }
+}
+
+template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::pass2_quads(const HostPlanes P[4], int64_t m, int64_t n, int dirs, double gamma, int kind,
+                                         const FaceDst& x, const FaceDst& y, double weps, cudaStream_t st) {
+  using T = dev_t<H>;
+  using namespace detail;
+  if constexpr (is_native_f64<T>) {
+    const unsigned bx = (dirs & 1) ? quad_blocks(m - 5, n - 6) : 0, by = (dirs & 2) ? quad_blocks(m - 6, n - 5) : 0;
+    if (bx + by == 0) return cudaSuccess;
+    const T gm = (T)gamma, we = (T)weps;
+    const auto A = planes<T>(P[0]), B = planes<T>(P[1]), C = planes<T>(P[2]), D = planes<T>(P[3]);
+    const Pass2Dst dx{x.a, x.b, x.c, x.d, x.ps, x.ld}, dy{y.a, y.b, y.c, y.d, y.ps, y.ld};
+    if (kind == 0) k_pass2_quad<FAST, P2_STATES><<<bx + by, 32, 0, st>>>(A, B, C, D, m, n, bx, gm, dx, dy, we);
+    else if (kind == 1) k_pass2_quad<FAST, P2_HLLE><<<bx + by, 32, 0, st>>>(A, B, C, D, m, n, bx, gm, dx, dy, we);
+    else k_pass2_quad<FAST, P2_BLEND><<<bx + by, 32, 0, st>>>(A, B, C, D, m, n, bx, gm, dx, dy, we);
+    return cudaGetLastError();
+  } else {
+    return cudaErrorNotSupported;
+  }
 }
 
 template <class H, bool FAST>
