@@ -180,6 +180,33 @@ __device__ __forceinline__ void tile_gq_side(const T* p, int ks, int ts, T weps,
   }
 }
 
+// Component-wise pass 1 of one cell (five cells along the sweep, all components):
+// its states at its right face (l, q_l there) and at its left face (r, q_r there).
+template <class T, bool FAST>
+__device__ __forceinline__ void cell_states(const T c[5][4], T weps, T l[4], T r[4]) {
+  if constexpr (is_f32<T>) {
+#pragma unroll
+    for (int k = 0; k < 4; k += 2) {
+      f32x2 v[5], a, b;
+#pragma unroll
+      for (int s = 0; s < 5; ++s) v[s] = f32x2(c[s][k], c[s][k + 1]);
+      weno5_cell_fast<f32x2>(v, f32x2(weps), b, a);
+      l[k] = a.v.x, l[k + 1] = a.v.y, r[k] = b.v.x, r[k + 1] = b.v.y;
+    }
+  } else {
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+      T v[5], a, b;
+#pragma unroll
+      for (int s = 0; s < 5; ++s) v[s] = pick4(c[s], k);
+      if constexpr (FAST) weno5_cell_fast<T>(v, weps, b, a);
+      else weno5_cell_exact<T>(v, weps, b, a);
+      put4(l, k, a);
+      put4(r, k, b);
+    }
+  }
+}
+
 // Riemann solver of one tile face and its store into the face buffer F
 // (HLLE flux planes, or HLLC + HLLE + mean pressure for the sensor blend).
 // S = 2 (HLLE only): states and fluxes are twice the face averages.
@@ -296,22 +323,43 @@ __global__ void __launch_bounds__(NT) k_stage_tiles(const SolveDesc* __restrict_
     __syncthreads();
 
     // ---- x sweep: pass 1 on faces fi = i0-HF+fr (global face rows 0..nx) ----
-    for (int e = tid; e < G::P1XR * G::P1XC; e += NT) {
-      const int fr = e / G::P1XC, c = e % G::P1XC;
-      const int fi = i0 - HF + fr;
-      if (fi < 0 || fi > nx) continue;
-      // pass-1 column J = j0+1-HF+c <-> tile column c+1
-      T cells[6][4];
+    if constexpr (!CHAR) {
+      // one cell per thread (the left one of face fr, the right one of face fr - 1)
+      for (int e = tid; e < (G::P1XR + 1) * G::P1XC; e += NT) {
+        const int fr = e / G::P1XC, c = e % G::P1XC;
+        const int fi = i0 - HF + fr;
+        const bool has_l = fr < G::P1XR && fi >= 0 && fi <= nx, has_r = fr > 0 && fi > 0 && fi <= nx + 1;
+        if (!has_l && !has_r) continue;
+        T cells[5][4], l[4], r[4];
 #pragma unroll
-      for (int s = 0; s < 6; ++s)
+        for (int s = 0; s < 5; ++s)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) cells[s][k] = U[k * G::UR * G::UC + (fr + s) * G::UC + c + 1 + G::CO];
-      T ql[4], qr[4];
-      pass1_face<T, FAST, false, CHAR>(cells, gamma, ql, qr, weps);
+          for (int k = 0; k < 4; ++k) cells[s][k] = U[k * G::UR * G::UC + (fr + s) * G::UC + c + 1 + G::CO];
+        cell_states<T, FAST>(cells, weps, l, r);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        P1[k * G::P1 + e] = ql[k];
-        P1[(4 + k) * G::P1 + e] = qr[k];
+        for (int k = 0; k < 4; ++k) {
+          if (has_l) P1[k * G::P1 + e] = l[k];
+          if (has_r) P1[(4 + k) * G::P1 + e - G::P1XC] = r[k];
+        }
+      }
+    } else {
+      for (int e = tid; e < G::P1XR * G::P1XC; e += NT) {
+        const int fr = e / G::P1XC, c = e % G::P1XC;
+        const int fi = i0 - HF + fr;
+        if (fi < 0 || fi > nx) continue;
+        // pass-1 column J = j0+1-HF+c <-> tile column c+1
+        T cells[6][4];
+#pragma unroll
+        for (int s = 0; s < 6; ++s)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) cells[s][k] = U[k * G::UR * G::UC + (fr + s) * G::UC + c + 1 + G::CO];
+        T ql[4], qr[4];
+        pass1_face<T, FAST, false, CHAR>(cells, gamma, ql, qr, weps);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          P1[k * G::P1 + e] = ql[k];
+          P1[(4 + k) * G::P1 + e] = qr[k];
+        }
       }
     }
     __syncthreads();
@@ -370,21 +418,42 @@ __global__ void __launch_bounds__(NT) k_stage_tiles(const SolveDesc* __restrict_
     __syncthreads();
 
     // ---- y sweep: pass 1 on rows I = i0+1-HF+r, faces fj = j0-HF+fc ----
-    for (int e = tid; e < G::P1YR * G::P1YC; e += NT) {
-      const int r = e / G::P1YC, fc = e % G::P1YC;
-      const int I = i0 + 1 - HF + r, fj = j0 - HF + fc;
-      if (I < 0 || I >= nx + 6 || fj < 0 || fj > ny) continue;
-      T cells[6][4];
+    if constexpr (!CHAR) {
+      for (int e = tid; e < G::P1YR * (G::P1YC + 1); e += NT) {
+        const int r = e / (G::P1YC + 1), fc = e % (G::P1YC + 1);
+        const int I = i0 + 1 - HF + r, fj = j0 - HF + fc;
+        if (I < 0 || I >= nx + 6) continue;
+        const bool has_l = fc < G::P1YC && fj >= 0 && fj <= ny, has_r = fc > 0 && fj > 0 && fj <= ny + 1;
+        if (!has_l && !has_r) continue;
+        T cells[5][4], lv[4], rv[4];
 #pragma unroll
-      for (int s = 0; s < 6; ++s)
+        for (int s = 0; s < 5; ++s)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) cells[s][k] = U[k * G::UR * G::UC + (r + 1) * G::UC + fc + s + G::CO];
-      T ql[4], qr[4];
-      pass1_face<T, FAST, true, CHAR>(cells, gamma, ql, qr, weps);
+          for (int k = 0; k < 4; ++k) cells[s][k] = U[k * G::UR * G::UC + (r + 1) * G::UC + fc + s + G::CO];
+        cell_states<T, FAST>(cells, weps, lv, rv);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        P1[k * G::P1 + e] = ql[k];
-        P1[(4 + k) * G::P1 + e] = qr[k];
+        for (int k = 0; k < 4; ++k) {
+          if (has_l) P1[k * G::P1 + r * G::P1YC + fc] = lv[k];
+          if (has_r) P1[(4 + k) * G::P1 + r * G::P1YC + fc - 1] = rv[k];
+        }
+      }
+    } else {
+      for (int e = tid; e < G::P1YR * G::P1YC; e += NT) {
+        const int r = e / G::P1YC, fc = e % G::P1YC;
+        const int I = i0 + 1 - HF + r, fj = j0 - HF + fc;
+        if (I < 0 || I >= nx + 6 || fj < 0 || fj > ny) continue;
+        T cells[6][4];
+#pragma unroll
+        for (int s = 0; s < 6; ++s)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) cells[s][k] = U[k * G::UR * G::UC + (r + 1) * G::UC + fc + s + G::CO];
+        T ql[4], qr[4];
+        pass1_face<T, FAST, true, CHAR>(cells, gamma, ql, qr, weps);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          P1[k * G::P1 + e] = ql[k];
+          P1[(4 + k) * G::P1 + e] = qr[k];
+        }
       }
     }
     __syncthreads();
@@ -562,6 +631,40 @@ __global__ void __launch_bounds__(NT) k_staged_pass1(const SolveDesc* __restrict
     const int nxc = xc1 - xc0, nxf = (xr1 - xr0) * nxc;
     const int nyc = yc1 - yc0, nyf = (yr1 - yr0) * nyc;
     const T* q = Qin + d.off;
+    if constexpr (!CHAR) {
+      // one cell per thread: rows xr0 .. xr1 (columns yc0 .. yc1), one more than the faces
+      const int nxn = nxf + nxc, nyc1 = nyc + 1, nyn = (yr1 - yr0) * nyc1;
+      for (int e = threadIdx.x; e < nxn + nyn; e += NT) {
+        T cells[5][4], l[4], r[4];
+        if (e < nxn) {
+          const int fi = xr0 + e / nxc, J = xc0 + e % nxc;  // padded row fi + 2
+#pragma unroll
+          for (int s = 0; s < 5; ++s) staged_cell(d, q, fi + s, J + 3, cells[s]);
+          cell_states<T, FAST>(cells, weps, l, r);
+          T* w = W + d.w_p1x + (long long)fi * d.l_p1x + (J + 2);
+          const bool has_l = fi < xr1, has_r = fi > xr0;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (has_l) w[k * d.s_p1x] = l[k];
+            if (has_r) w[(4 + k) * d.s_p1x - d.l_p1x] = r[k];
+          }
+        } else {
+          const int e2 = e - nxn;
+          const int I = yr0 + e2 / nyc1, fj = yc0 + e2 % nyc1;  // padded column fj + 2
+#pragma unroll
+          for (int s = 0; s < 5; ++s) staged_cell(d, q, I + 3, fj + s, cells[s]);
+          cell_states<T, FAST>(cells, weps, l, r);
+          T* w = W + d.w_p1y + (long long)(I + 2) * d.l_p1y + fj;
+          const bool has_l = fj < yc1, has_r = fj > yc0;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (has_l) w[k * d.s_p1y] = l[k];
+            if (has_r) w[(4 + k) * d.s_p1y - 1] = r[k];
+          }
+        }
+      }
+      continue;
+    }
     for (int e = threadIdx.x; e < nxf + nyf; e += NT) {
       T cells[6][4], ql[4], qr[4];
       if (e < nxf) {

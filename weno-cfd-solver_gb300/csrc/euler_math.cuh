@@ -333,13 +333,12 @@ __device__ __forceinline__ T weno_combine(T e0, T e1, T e2, T d0, T d1, T d2, T 
 }
 
 // The exact weights, a_k = d_k/(eps+b_k)^2 and w_k = a_k/sum, applied to the
-// candidates: w0 p0 + w1 p1 + w2 p2.  The three divisions of each kind share
+// candidates: w0 p0 + w1 p1 + w2 p2, from the squares (passed in a_k).  The three divisions of each kind share
 // one piece of code (a loop): FP64 is the bound, not the latency of one warp,
 // and integer divisions unrolled at every use would not fit the instruction cache.
 // U = 3 unrolls them, for the kernels that one warp's latency bounds.
 template <class T, int U = 1>
-__device__ __forceinline__ T weno_combine_exact(T e0, T e1, T e2, T d0, T d1, T d2, T p0, T p1, T p2) {
-  T a0 = e0 * e0, a1 = e1 * e1, a2 = e2 * e2;
+__device__ __forceinline__ T weno_combine_exact(T a0, T a1, T a2, T d0, T d1, T d2, T p0, T p1, T p2) {
 #pragma unroll(U)
   for (int k = 0; k < 3; ++k) {  // rotates (d, a) so that every k divides the front pair
     const T q = d0 / a0;
@@ -411,8 +410,9 @@ __device__ __forceinline__ void weno5_lr_exact(const T u[6], T weps, T& left, T&
     js_betas(v0, v1, v2, v3, v4, b0, b1, b2);
     // 2 u0 - 7 u1 + 11 u2 (left, third candidate), 2 u5 - 7 u4 + 11 u3 (right, first)
     const T g = mul_pow2<1>(side ? u[5] : u[0]) - T(7.0) * (side ? u[4] : u[1]) + T(11.0) * v2;
-    const T r = weno_combine_exact<T, U>(weps + b0, weps + b1, weps + b2, side ? T(0.1) : T(0.3), T(0.6),
-                                      side ? T(0.3) : T(0.1), side ? g : f1, side ? f1 : f2, side ? f2 : g) /
+    const T e0 = weps + b0, e1 = weps + b1, e2 = weps + b2;
+    const T r = weno_combine_exact<T, U>(e0 * e0, e1 * e1, e2 * e2, side ? T(0.1) : T(0.3), T(0.6),
+                                         side ? T(0.3) : T(0.1), side ? g : f1, side ? f1 : f2, side ? f2 : g) /
                 T(6.0);
     left = side ? left : r;
     right = r;
@@ -527,44 +527,72 @@ __device__ __forceinline__ void weno5_lr_fast(T u0, T u1, T u2, T u3, T u4, T u5
   }
 }
 
-// weno5_lr_fast of two neighbouring faces of one field (A between u2 and u3,
-// B between u3 and u4; FAST native double), sharing what the two faces have in
-// common: the differences, and -- since A's right state and B's left state are
-// both reconstructions about cell u3 from the stencils 1-3, 2-4, 3-5 -- their
-// indicators and weight products.  Every shared value is computed with the
-// operations weno5_lr_fast performs for each face on its own, so A and B get
-// the bits of two separate calls (the component-wise pass 1 of the FAST
-// double solver).
-__device__ __forceinline__ void weno5_lr_fast_two(f64 u0, f64 u1, f64 u2, f64 u3, f64 u4, f64 u5, f64 u6, f64 weps,
-                                                  f64& lA, f64& rA, f64& lB, f64& rB) {
-  const f64 d0 = u1 - u0, d1 = u2 - u1, d2 = u3 - u2, d3 = u4 - u3, d4 = u5 - u4, d5 = u6 - u5;
-  const f64 D1 = d1 - d0, D2 = d2 - d1, D3 = d3 - d2, D4 = d4 - d3, D5 = d5 - d4;
-  const f64 w4 = 4.0 * weps;
-  const f64 C1 = kC43 * D1 * D1 + w4, C2 = kC43 * D2 * D2 + w4, C3 = kC43 * D3 * D3 + w4,
-               C4 = kC43 * D4 * D4 + w4, C5 = kC43 * D5 * D5 + w4;
-  // face A: as weno5_lr_fast(u0..u5)
-  const f64 sl0 = d3 - 3.0 * d2, sl1 = d1 + d2, sl2 = 3.0 * d1 - d0;
-  const f64 sr0 = d4 - 3.0 * d3, sr1 = d2 + d3, sr2 = 3.0 * d2 - d1;
-  const f64 el0 = sl0 * sl0 + C3, el1 = sl1 * sl1 + C2, el2 = sl2 * sl2 + C1;
-  const f64 er0 = sr0 * sr0 + C4, er1 = sr1 * sr1 + C3, er2 = sr2 * sr2 + C2;
-  const f64 gl0 = d2 - sl0, gl1 = sl1 + d2, gl2 = 2.0 * sl2 - d1;
-  const f64 gr2 = -d2 - sr2, gr1 = -d2 - sr1, gr0 = 2.0 * sr0 + d3;
-  // face B: as weno5_lr_fast(u1..u6); its left stencils and indicators are A's right ones
-  const f64 tr0 = d5 - 3.0 * d4, tr1 = d3 + d4, tr2 = 3.0 * d3 - d2;
-  const f64 fr0 = tr0 * tr0 + C5, fr1 = tr1 * tr1 + C4, fr2 = tr2 * tr2 + C3;
-  const f64 hl0 = d3 - sr0, hl1 = sr1 + d3, hl2 = 2.0 * sr2 - d2;
-  const f64 hr2 = -d3 - tr2, hr1 = -d3 - tr1, hr0 = 2.0 * tr0 + d4;
-  f64 P0, P1, P2, nl, dl, nr, dr;
-  weno_nd_products(el0, el1, el2, P0, P1, P2);
-  weno_nd_combine(P0, P1, P2, gl0, gl1, gl2, nl, dl);
-  weno_nd_products(er2, er1, er0, P0, P1, P2);
-  weno_nd_combine(P0, P1, P2, gr2, gr1, gr0, nr, dr);
-  div_pair(nl, dl, nr, dr, lA, rA, 6.0, u2, u3);
-  // B's left from the same products in the other order (products commute)
-  weno_nd_combine(P2, P1, P0, hl0, hl1, hl2, nl, dl);
-  weno_nd_products(fr2, fr1, fr0, P0, P1, P2);
-  weno_nd_combine(P0, P1, P2, hr2, hr1, hr0, nr, dr);
-  div_pair(nl, dl, nr, dr, lB, rB, 6.0, u3, u4);
+// Both face states of one cell u[2] of a field from its five cells, component-wise
+// pass 1: `lf` at its left face, `rf` at its right face.  The operations are those
+// of weno5_lr_fast seen from the cell (indicators and weight products once for
+// both states), odd under the mirror image of the stencil.
+template <class T>
+__device__ __forceinline__ void weno5_cell_fast(const T u[5], T weps, T& lf, T& rf) {
+  const T d0 = u[1] - u[0], d1 = u[2] - u[1], d2 = u[3] - u[2], d3 = u[4] - u[3];
+  if constexpr (is_native_f64<T>) {
+    if (ffw::covers(max(max_magnitude(d0, d1), max_magnitude(d2, d3)), weps.v)) {
+      const ffw::ff w = ffw::eps75(weps.v);
+      const ffw::ff f0 = ffw::from_double(d0.v), f1 = ffw::from_double(d1.v), f2 = ffw::from_double(d2.v),
+                    f3 = ffw::from_double(d3.v);
+      const ffw::ff qr = ffw::side(f2, f3, w), qm = ffw::centre(f1, f2, w), ql = ffw::side(f1, f0, w);
+      double cn, cm, cf;
+      ffw::face_weights(qr, qm, ql, cn, cm, cf);
+      rf = u[2] + face_slope(d2, d3, d1, d0, cn, cm, cf);
+      ffw::face_weights(ql, qm, qr, cn, cm, cf);
+      lf = u[2] - face_slope(d1, d0, d2, d3, cn, cm, cf);
+      return;
+    }
+  }
+  const T D1 = d1 - d0, D2 = d2 - d1, D3 = d3 - d2;
+  const T w4 = T(4.0) * weps;
+  const T sr = d3 - T(3.0) * d2, sm = d1 + d2, sl = T(3.0) * d1 - d0;
+  const T er = sr * sr + (T(kC43) * D3 * D3 + w4), em = sm * sm + (T(kC43) * D2 * D2 + w4),
+          el = sl * sl + (T(kC43) * D1 * D1 + w4);
+  // slopes (x6) of the stencils reaching over the face, central and behind the cell
+  const T rn = d2 - sr, rm = sm + d2, rr = T(2.0) * sl - d1;
+  const T ln = d1 + sl, lm = sm + d1, ll = -d2 - T(2.0) * sr;
+  if constexpr (is_native_f64<T>) {
+    T Pr, Pm, Pl, nr, dr, nl, dl;
+    weno_nd_products(er, em, el, Pr, Pm, Pl);
+    weno_nd_combine(Pr, Pm, Pl, rn, rm, rr, nr, dr);
+    weno_nd_combine(Pl, Pm, Pr, ln, lm, ll, nl, dl);
+    div_pair(nr, dr, -nl, dl, rf, lf, 6.0, u[2], u[2]);
+  } else {
+    const T ar = qrcp<T, true>(er * er), am = qrcp<T, true>(em * em), al = qrcp<T, true>(el * el);
+    const T r0 = T(0.3) * ar, m0 = T(0.6) * am, l0 = T(0.1) * al, l1 = T(0.3) * al, r1 = T(0.1) * ar;
+    rf = u[2] + qdiv<T, true>(r0 * rn + m0 * rm + l0 * rr, (r0 + m0 + l0) * T(6.0));
+    lf = u[2] - qdiv<T, true>(l1 * ln + m0 * lm + r1 * ll, (l1 + m0 + r1) * T(6.0));
+  }
+}
+
+// The same in the reference's operations (weno.rs:214-257): the left-biased state
+// at the right face and the right-biased one at the left face share the indicators.
+template <class T>
+__device__ __forceinline__ void weno5_cell_exact(const T u[5], T weps, T& lf, T& rf) {
+  T b0, b1, b2;
+  js_betas(u[0], u[1], u[2], u[3], u[4], b0, b1, b2);
+  const T e0 = weps + b0, e1 = weps + b1, e2 = weps + b2;
+  const T s0 = e0 * e0, s1 = e1 * e1, s2 = e2 * e2;
+  const T fu = T(5.0) * u[2], el = T(11.0) * u[2], two = mul_pow2<1>(u[2]);
+#pragma unroll 1
+  for (int side = 0; side < 2; ++side) {  // left face (right-biased), then right face
+    // -u4 + 5 u3 + 2 u2, -u1 + 5 u2 + 2 u3, 2 u0 - 7 u1 + 11 u2 at the right face;
+    // 2 u4 - 7 u3 + 11 u2, -u3 + 5 u2 + 2 u1, -u0 + 5 u1 + 2 u2 at the left one
+    const T a = side ? u[4] : u[0], b = side ? u[3] : u[1], c = side ? u[1] : u[3], d = side ? u[0] : u[4];
+    const T near = -a + T(5.0) * b + two;
+    const T mid = -c + fu + mul_pow2<1>(b);
+    const T far = mul_pow2<1>(d) - T(7.0) * c + el;
+    const T r = weno_combine_exact<T>(s0, s1, s2, side ? T(0.3) : T(0.1), T(0.6), side ? T(0.1) : T(0.3),
+                                      side ? near : far, mid, side ? far : near) /
+                T(6.0);
+    lf = side ? lf : r;
+    rf = r;
+  }
 }
 
 // FAST float: the four fields' left/right reconstructions as two packed pairs
@@ -701,6 +729,7 @@ __device__ __forceinline__ void weno5_gq_pair(T q0, T q1, T q2, T q3, T q4, T& r
     T b0, b1, b2;
     js_betas(q0, q1, q2, q3, q4, b0, b1, b2);
     const T e0 = weps + b0, e1 = weps + b1, e2 = weps + b2;
+    const T s0 = e0 * e0, s1 = e1 * e1, s2 = e2 * e2;
     const T g0 = (T(3.0) * q2 - mul_pow2<2>(q3) + q4) * S;
     const T g2 = (T(3.0) * q2 - mul_pow2<2>(q1) + q0) * S;
     // point a: q2 + g0, q2 - (q3 - q1) S, q2 - g2; point b: the mirror (negation
@@ -708,7 +737,7 @@ __device__ __forceinline__ void weno5_gq_pair(T q0, T q1, T q2, T q3, T q4, T& r
     const T g1 = (-q1 + q3) * S;
 #pragma unroll(U == 1 ? 1 : 2)
     for (int pt = 0; pt < 2; ++pt) {
-      const T r = weno_combine_exact<T, U>(e0, e1, e2, pt ? T(kGqA2) : T(kGqA0), T(kGqA1), pt ? T(kGqA0) : T(kGqA2),
+      const T r = weno_combine_exact<T, U>(s0, s1, s2, pt ? T(kGqA2) : T(kGqA0), T(kGqA1), pt ? T(kGqA0) : T(kGqA2),
                                         q2 + (pt ? -g0 : g0), q2 - (pt ? -g1 : g1), q2 - (pt ? -g2 : g2));
       ra = pt ? ra : r;
       rb = r;

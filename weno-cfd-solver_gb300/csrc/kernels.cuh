@@ -126,33 +126,43 @@ __global__ void __launch_bounds__(128) k_pass1_marked(CView<df64> u, int64_t row
   }
 }
 
-// Component-wise pass 1, FAST double: two neighbouring faces per thread along
-// the sweep (rows for x, columns for y), whose seven cells and shared
-// reconstructions about the middle cell serve both (weno5_lr_fast_two; the
-// same bits as one face per thread).
-template <bool Y>
-__global__ void __launch_bounds__(128) k_pass1_cons2(CView<f64> u, int64_t rows, int64_t cols, Planes<f64> PL,
-                                                      Planes<f64> PR, f64 weps) {
+// Component-wise pass 1, one cell per thread: the cell's indicators serve the
+// state at its right face (q_l there) and at its left face (q_r there), so every
+// stencil's are formed once instead of on two faces.  Thread t of a sweep owns
+// the cell t + 2, the left one of face t and the right one of face t - 1.
+template <class T, bool FAST, bool Y>
+__global__ void __launch_bounds__(128) k_pass1_cells(CView<T> u, int64_t rows, int64_t cols, Planes<T> PL,
+                                                      Planes<T> PR, T weps) {
   int64_t row, col;
-  if (!locate(Y ? rows : (rows + 1) / 2, Y ? (cols + 1) / 2 : cols, row, col)) return;
-  if constexpr (Y) col *= 2;
-  else row *= 2;
-  const bool two = Y ? (col + 1 < cols) : (row + 1 < rows);
-  const int64_t rowB = Y ? row : row + 1, colB = Y ? col + 1 : col;
+  if (!locate(Y ? rows : rows + 1, Y ? cols + 1 : cols, row, col)) return;
+  const bool has_l = Y ? col < cols : row < rows, has_r = Y ? col > 0 : row > 0;
+  const int64_t rr = Y ? row : row - 1, rc = Y ? col - 1 : col;
+  constexpr int STEP = is_f32<T> ? 2 : 1;
+#pragma unroll(is_f32<T> ? 2 : 1)
+  for (int k = 0; k < 4; k += STEP) {
+    if constexpr (is_f32<T>) {
+      f32x2 v[5], l, r;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    f64 v[7];
+      for (int s = 0; s < 5; ++s)
+        v[s] = Y ? f32x2(u.at(row, col + s, k), u.at(row, col + s, k + 1))
+                 : f32x2(u.at(row + s, col, k), u.at(row + s, col, k + 1));
+      weno5_cell_fast<f32x2>(v, f32x2(weps), r, l);
+      if (has_l) {
+        PL.at(k, row, col) = l.v.x;
+        PL.at(k + 1, row, col) = l.v.y;
+      }
+      if (has_r) {
+        PR.at(k, rr, rc) = r.v.x;
+        PR.at(k + 1, rr, rc) = r.v.y;
+      }
+    } else {
+      T v[5], l, r;
 #pragma unroll
-    for (int s = 0; s < 6; ++s) v[s] = Y ? u.at(row, col + s, k) : u.at(row + s, col, k);
-    // the seventh cell exists only when face B does
-    v[6] = two ? (Y ? u.at(row, col + 6, k) : u.at(row + 6, col, k)) : v[5];
-    f64 lA, rA, lB, rB;
-    weno5_lr_fast_two(v[0], v[1], v[2], v[3], v[4], v[5], v[6], weps, lA, rA, lB, rB);
-    PL.at(k, row, col) = lA;
-    PR.at(k, row, col) = rA;
-    if (two) {
-      PL.at(k, rowB, colB) = lB;
-      PR.at(k, rowB, colB) = rB;
+      for (int s = 0; s < 5; ++s) v[s] = Y ? u.at(row, col + s, k) : u.at(row + s, col, k);
+      if constexpr (FAST) weno5_cell_fast<T>(v, weps, r, l);
+      else weno5_cell_exact<T>(v, weps, r, l);
+      if (has_l) PL.at(k, row, col) = l;
+      if (has_r) PR.at(k, rr, rc) = r;
     }
   }
 }
