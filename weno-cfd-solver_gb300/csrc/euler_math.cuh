@@ -127,11 +127,22 @@ __device__ __forceinline__ T qdiv(T a, T b) {
   if constexpr (FAST && is_f32<T>) return __fdividef(a, b);
   else return a / b;
 }
+// 1 / b.  FAST float: the hardware reciprocal itself, for arguments that are never
+// subnormal (clamped densities, guarded denominators, spacings): __fdividef(1, b)
+// gives the same bits there but carries four instructions for subnormal b.
 template <class T, bool FAST>
 __device__ __forceinline__ T qrcp(T b) {
-  if constexpr (FAST && is_f32<T>) return __fdividef(1.0f, b);
+  if constexpr (FAST && is_f32<T>) return rcp_seed(b);
   else return T(1.0) / b;
 }
+// 1 / e^2 of the float weights; 2^-126 keeps the square normal for a vanishing
+// epsilon and is below half a unit of any other.
+__device__ __forceinline__ float inv_square(float e) { return rcp_seed(__fmaf_rn(e, e, 0x1p-126f)); }
+__device__ __forceinline__ f32x2 inv_square(f32x2 e) {
+  const float2 s = __ffma2_rn(e.v, e.v, make_float2(0x1p-126f, 0x1p-126f));
+  return f32x2(rcp_seed(s.x), rcp_seed(s.y));
+}
+__device__ __forceinline__ df64 inv_square(df64 e) { return df64(1.0) / (e * e); }
 // sqrt(x), 1/sqrt(x) and 1/x of the FAST forms (x > 0).  An f64 takes the integer
 // root and reciprocal and one product; float (CUDA's rsqrtf, within 2 ulp) and
 // df64 one reciprocal square root r, x r and r r.
@@ -325,9 +336,9 @@ __device__ __forceinline__ void weno_range(f64& e0, f64& e1, f64& e2) {
 template <class T>
 __device__ __forceinline__ T weno_combine(T e0, T e1, T e2, T d0, T d1, T d2, T p0, T p1, T p2, T scale) {
   static_assert(!is_native_f64<T>, "FAST double takes the common-denominator form (weno_nd)");
-  const T a0 = d0 * qrcp<T, true>(e0 * e0);
-  const T a1 = d1 * qrcp<T, true>(e1 * e1);
-  const T a2 = d2 * qrcp<T, true>(e2 * e2);
+  const T a0 = d0 * inv_square(e0);
+  const T a1 = d1 * inv_square(e1);
+  const T a2 = d2 * inv_square(e2);
   const T num = a0 * p0 + a1 * p1 + a2 * p2;
   return qdiv<T, true>(num, (a0 + a1 + a2) * scale);
 }
@@ -563,7 +574,7 @@ __device__ __forceinline__ void weno5_cell_fast(const T u[5], T weps, T& lf, T& 
     weno_nd_combine(Pl, Pm, Pr, ln, lm, ll, nl, dl);
     div_pair(nr, dr, -nl, dl, rf, lf, 6.0, u[2], u[2]);
   } else {
-    const T ar = qrcp<T, true>(er * er), am = qrcp<T, true>(em * em), al = qrcp<T, true>(el * el);
+    const T ar = inv_square(er), am = inv_square(em), al = inv_square(el);
     const T r0 = T(0.3) * ar, m0 = T(0.6) * am, l0 = T(0.1) * al, l1 = T(0.3) * al, r1 = T(0.1) * ar;
     rf = u[2] + qdiv<T, true>(r0 * rn + m0 * rm + l0 * rr, (r0 + m0 + l0) * T(6.0));
     lf = u[2] - qdiv<T, true>(l1 * ln + m0 * lm + r1 * ll, (l1 + m0 + r1) * T(6.0));
@@ -635,7 +646,7 @@ __device__ __forceinline__ void gq_weights(T q2, T h0, T h1, T h2, T f0, T f1, T
     ra = fma(r0, u0, fma(-r2, u2, -u1)) * (sb * t) + q2;
     rb = fma(r0, u2, fma(-r2, u0, u1)) * (sa * t) + q2;
   } else {
-    const T r0 = qrcp<T, true>(f0 * f0), r1 = qrcp<T, true>(f1 * f1), r2 = qrcp<T, true>(f2 * f2);
+    const T r0 = inv_square(f0), r1 = inv_square(f1), r2 = inv_square(f2);
     const T ca0 = T(kGqA0 / kGqA1) * r0, ca1 = r1, ca2 = T(kGqA2 / kGqA1) * r2;
     const T cb0 = T(kGqA2 / kGqA1) * r0, cb2 = T(kGqA0 / kGqA1) * r2;
     ra = qdiv<T, true>((ca0 * h0 - ca1 * h1 - ca2 * h2) * S, ca0 + ca1 + ca2) + q2;

@@ -260,9 +260,9 @@ cudaError_t Launch<H, FAST>::bc_transmissive(HostView q, int nc, int64_t M, int6
                                              cudaStream_t st) {
   using T = dev_t<H>;
   using namespace detail;
-  const dim3 g = grid2d(M, N, kBlk);
-  if (nc == 8) k_bc_transmissive<T, 8><<<g, kBlk, 0, st>>>(s3<T>(q), M, N, ctl);
-  else k_bc_transmissive<T, 4><<<g, kBlk, 0, st>>>(s3<T>(q), M, N, ctl);
+  const unsigned g = (unsigned)((ghost_count(M, N) + 127) / 128);
+  if (nc == 8) k_bc_transmissive<T, 8><<<g, 128, 0, st>>>(s3<T>(q), M, N, ctl);
+  else k_bc_transmissive<T, 4><<<g, 128, 0, st>>>(s3<T>(q), M, N, ctl);
   return cudaGetLastError();
 }
 
@@ -271,11 +271,11 @@ cudaError_t Launch<H, FAST>::bc_dmr(HostView q, int nc, int64_t nx, int64_t ny, 
                                     const StepCtl* ctl, cudaStream_t st) {
   using T = dev_t<H>;
   using namespace detail;
-  const dim3 g = grid2d(nx + 6, ny + 6, kBlk);
+  const unsigned g = (unsigned)((ghost_count(nx + 6, ny + 6) + 127) / 128);
   Post8<T> post;
   for (int k = 0; k < 8; ++k) post.v[k] = T(post8[k]);
-  if (nc == 8) k_bc_dmr<T, 8><<<g, kBlk, 0, st>>>(s3<T>(q), nx, ny, bound, post, ctl);
-  else k_bc_dmr<T, 4><<<g, kBlk, 0, st>>>(s3<T>(q), nx, ny, bound, post, ctl);
+  if (nc == 8) k_bc_dmr<T, 8><<<g, 128, 0, st>>>(s3<T>(q), nx, ny, bound, post, ctl);
+  else k_bc_dmr<T, 4><<<g, 128, 0, st>>>(s3<T>(q), nx, ny, bound, post, ctl);
   return cudaGetLastError();
 }
 
