@@ -121,6 +121,11 @@ cudaError_t residual_pipeline(HostView u, int64_t m, int64_t n, const ResidualLa
     WENO_TIMED(HC_PASS2_Y, Lx::pass2(PL, PR, m - 6, n - 5, gamma, true, kind, fy, fy + 4 * Lo.FY, fy + 8 * Lo.FY,
                                      nullptr, Lo.FY, n - 5, weps, st));
   }
+  HostPlanes Fx{fx, Lo.FX, n - 6}, Fy{fy, Lo.FY, n - 5};
+  if (std::is_same<T, float>::value && !force_hlle) {
+    WENO_TIMED(HC_RESIDUAL, Lx::residual_blend(Fx, Fy, m - 6, n - 6, dx, jp_lo, jp_hi, stage, Qn, Qs, Qo, ctl, st));
+    return cudaSuccess;
+  }
   if (!force_hlle) {
     HostPlanes C{fx, Lo.FX, n - 6}, E{fx + 4 * Lo.FX, Lo.FX, n - 6}, P{fx + 8 * Lo.FX, Lo.FX, n - 6};
     WENO_TIMED(HC_BLEND, Lx::blend(C, E, P, m - 5, n - 6, jp_lo, jp_hi, nullptr, st));
@@ -129,7 +134,6 @@ cudaError_t residual_pipeline(HostView u, int64_t m, int64_t n, const ResidualLa
     HostPlanes C{fy, Lo.FY, n - 5}, E{fy + 4 * Lo.FY, Lo.FY, n - 5}, P{fy + 8 * Lo.FY, Lo.FY, n - 5};
     WENO_TIMED(HC_BLEND, Lx::blend(C, E, P, m - 6, n - 5, jp_lo, jp_hi, nullptr, st));
   }
-  HostPlanes Fx{fx, Lo.FX, n - 6}, Fy{fy, Lo.FY, n - 5};
   WENO_TIMED(HC_RESIDUAL, Lx::residual(Fx, Fy, m - 6, n - 6, dx, stage, out, Qn, Qs, Qo, ctl, st));
 #undef WENO_TIMED
   return cudaSuccess;
@@ -416,11 +420,12 @@ struct weno_solver {
 
 namespace {
 
-// pass 1 and 2 of both sweeps and the residual; two sensor blends; df64: the marked
+// pass 1 and 2 of both sweeps and the residual; two sensor blends (FP32: inside the
+// residual); df64: the marked
 // faces of the two pass 1
 // faces of the two pass 1; small FP64 grids: both sweeps in one launch per pass
 int launches_per_residual(const weno_solver* s) {
-  return 5 + (s->force_hlle ? 0 : 2) + (s->prec == 48 ? 2 : 0) - (s->layout->quads ? 2 : 0);
+  return 5 + (s->force_hlle || s->prec == 32 ? 0 : 2) + (s->prec == 48 ? 2 : 0) - (s->layout->quads ? 2 : 0);
 }
 
 HostPlanes state_planes(weno_solver* s, void* base) { return HostPlanes{base, s->PS, s->N}; }

@@ -68,8 +68,14 @@ __device__ __forceinline__ bool locate(int64_t rows, int64_t cols, int64_t& row,
 // to reconstruct: a NaN no arithmetic produces.
 constexpr uint32_t kDf64Marker = 0x7fc0df64u;
 
+// Resident blocks per SM that pass 1 is compiled for (4 warps each).  FP64: 4, at
+// 128 registers (at 156 and three blocks the 2048^2 step took 2.6 % longer); FP32: 8,
+// at 64 (6: 2.7 % longer, 7: 1 %, 9 spills: 1.6 %); df64: 4 (3: 2 % longer).
+template <class T>
+constexpr int kPass1Blocks = is_native_f64<T> ? 4 : (is_f32<T> ? 8 : 4);
+
 template <class T, bool FAST, bool Y, bool CHAR>
-__global__ void __launch_bounds__(128) k_pass1(CView<T> u, int64_t rows, int64_t cols, T gamma, Planes<T> PL,
+__global__ void __launch_bounds__(128, kPass1Blocks<T>) k_pass1(CView<T> u, int64_t rows, int64_t cols, T gamma, Planes<T> PL,
                                                 Planes<T> PR, T weps) {
   int64_t row, col;
   if (!locate(rows, cols, row, col)) return;
@@ -520,11 +526,9 @@ __global__ void __launch_bounds__(128) k_riemann(const T* QL, const T* FL, const
 // differences (still divided by 2*dx) on its edges.  rows, cols >= 2.
 // Output: planes (DENSE = false) or a dense (rows, cols, 4) array.
 // ---------------------------------------------------------------------------
-template <class T, bool FAST, bool DENSE>
-__global__ void __launch_bounds__(128) k_blend(Planes<T> Fc, Planes<T> Fe, Planes<T> Pbar, int64_t rows,
-                                                int64_t cols, T jp_lo, T jp_hi, T* out, Planes<T> Fout) {
-  int64_t row, col;
-  if (!locate(rows, cols, row, col)) return;
+template <class T, bool FAST>
+__device__ __forceinline__ T blend_weight(const Planes<T>& Pbar, int64_t rows, int64_t cols, int64_t row, int64_t col,
+                                          T jp_lo, T jp_hi) {
   const int64_t min_dim = rows < cols ? rows : cols;
   const T dx = T(1.0) / T((double)min_dim);
   const T two_dx = T(2.0) * dx;
@@ -535,7 +539,15 @@ __global__ void __launch_bounds__(128) k_blend(Planes<T> Fc, Planes<T> Fe, Plane
   const T p = Pbar.at(0, row, col);
   const T dpdx = qdiv<T, FAST>(Pbar.at(0, rb, col) - Pbar.at(0, ra, col), two_dx);
   const T dpdy = qdiv<T, FAST>(Pbar.at(0, row, cb) - Pbar.at(0, row, ca), two_dx);
-  const T w = sensor_weight<T, FAST>(dpdx, dpdy, p, jp_lo, jp_hi);
+  return sensor_weight<T, FAST>(dpdx, dpdy, p, jp_lo, jp_hi);
+}
+
+template <class T, bool FAST, bool DENSE>
+__global__ void __launch_bounds__(128) k_blend(Planes<T> Fc, Planes<T> Fe, Planes<T> Pbar, int64_t rows,
+                                                int64_t cols, T jp_lo, T jp_hi, T* out, Planes<T> Fout) {
+  int64_t row, col;
+  if (!locate(rows, cols, row, col)) return;
+  const T w = blend_weight<T, FAST>(Pbar, rows, cols, row, col, jp_lo, jp_hi);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const T f = w * Fc.at(k, row, col) + (T(1.0) - w) * Fe.at(k, row, col);
@@ -553,6 +565,33 @@ __global__ void __launch_bounds__(128) k_blend(Planes<T> Fc, Planes<T> Fe, Plane
 //   STAGE 3: qn = ((1/3)*q + (2/3)*q2) + ((2/3)*dt)*L
 // Fx planes are (m-5) x (n-6) faces, Fy planes (m-6) x (n-5).
 // ---------------------------------------------------------------------------
+
+// What a stage does with the residual L of cell (row, col).
+template <class T, int STAGE>
+__device__ __forceinline__ void residual_store(const T L[4], int64_t row, int64_t col, int64_t cols, T* out,
+                                               const Planes<T>& Qn, const Planes<T>& Qs, const Planes<T>& Qo,
+                                               const StepCtl* ctl) {
+  if constexpr (STAGE == 0) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) out[(row * cols + col) * 4 + k] = L[k];
+  } else {
+    const double dt = ctl->dt;
+    const int64_t r = row + 3, c = col + 3;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const T qn = Qn.at(k, r, c);
+      T v;
+      if constexpr (STAGE == 1) {
+        v = qn + T(dt) * L[k];
+      } else if constexpr (STAGE == 2) {
+        v = T(0.75) * qn + T(0.25) * Qs.at(k, r, c) + T(0.25 * dt) * L[k];
+      } else {
+        v = T(1.0 / 3.0) * qn + T(2.0 / 3.0) * Qs.at(k, r, c) + T((2.0 / 3.0) * dt) * L[k];
+      }
+      Qo.at(k, r, c) = v;
+    }
+  }
+}
 
 template <class T, bool FAST, int STAGE>
 __global__ void __launch_bounds__(128) k_residual(Planes<T> Fx, Planes<T> Fy, int64_t rows, int64_t cols, T dx,
@@ -579,26 +618,37 @@ __global__ void __launch_bounds__(128) k_residual(Planes<T> Fx, Planes<T> Fy, in
       L[k] = -(dfdx + dgdy);
     }
   }
-  if constexpr (STAGE == 0) {
+  residual_store<T, STAGE>(L, row, col, cols, out, Qn, Qs, Qo, ctl);
+}
+
+// The same with the sensor blend of the four faces of the cell in place of k_blend
+// (planes 0..3 HLLC, 4..7 HLLE, 8 the mean pressure).  FP32 only: each weight is
+// formed on two cells, which costs less than the 13 planes that k_blend reads and
+// writes per direction (17 us per launch at 2049 x 512, a quarter of the stage);
+// in FP64 the second weight would cost more than the planes.
+template <int STAGE>
+__global__ void __launch_bounds__(128) k_residual_blend(Planes<float> Fx, Planes<float> Fy, int64_t rows, int64_t cols,
+                                                         float dx, float jp_lo, float jp_hi, Planes<float> Qn,
+                                                         Planes<float> Qs, Planes<float> Qo, const StepCtl* ctl) {
+  int64_t row, col;
+  if (!locate(rows, cols, row, col)) return;
+  if (!ctl->active) return;
+  const Planes<float> Px{Fx.p + 8 * Fx.ps, Fx.ps, Fx.ld}, Py{Fy.p + 8 * Fy.ps, Fy.ps, Fy.ld};
+  const float xa = blend_weight<float, true>(Px, rows + 1, cols, row, col, jp_lo, jp_hi);
+  const float xb = blend_weight<float, true>(Px, rows + 1, cols, row + 1, col, jp_lo, jp_hi);
+  const float ya = blend_weight<float, true>(Py, rows, cols + 1, row, col, jp_lo, jp_hi);
+  const float yb = blend_weight<float, true>(Py, rows, cols + 1, row, col + 1, jp_lo, jp_hi);
+  const float idx = qrcp<float, true>(dx);
+  float L[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) out[(row * cols + col) * 4 + k] = L[k];
-  } else {
-    const double dt = ctl->dt;
-    const int64_t r = row + 3, c = col + 3;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const T qn = Qn.at(k, r, c);
-      T v;
-      if constexpr (STAGE == 1) {
-        v = qn + T(dt) * L[k];
-      } else if constexpr (STAGE == 2) {
-        v = T(0.75) * qn + T(0.25) * Qs.at(k, r, c) + T(0.25 * dt) * L[k];
-      } else {
-        v = T(1.0 / 3.0) * qn + T(2.0 / 3.0) * Qs.at(k, r, c) + T((2.0 / 3.0) * dt) * L[k];
-      }
-      Qo.at(k, r, c) = v;
-    }
+  for (int k = 0; k < 4; ++k) {
+    const float fa = xa * Fx.at(k, row, col) + (1.0f - xa) * Fx.at(4 + k, row, col);
+    const float fb = xb * Fx.at(k, row + 1, col) + (1.0f - xb) * Fx.at(4 + k, row + 1, col);
+    const float ga = ya * Fy.at(k, row, col) + (1.0f - ya) * Fy.at(4 + k, row, col);
+    const float gb = yb * Fy.at(k, row, col + 1) + (1.0f - yb) * Fy.at(4 + k, row, col + 1);
+    L[k] = -((fb - fa) + (gb - ga)) * idx;
   }
+  residual_store<float, STAGE>(L, row, col, cols, nullptr, Qn, Qs, Qo, ctl);
 }
 
 // ---------------------------------------------------------------------------

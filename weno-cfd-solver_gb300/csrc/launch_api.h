@@ -74,6 +74,11 @@ struct Launch {
   static cudaError_t residual(HostPlanes Fx, HostPlanes Fy, int64_t rows, int64_t cols, double dx, int stage,
                               void* out, HostPlanes Qn, HostPlanes Qs, HostPlanes Qo, const StepCtl* ctl,
                               cudaStream_t st);
+  // The same with the sensor blend of the faces (planes as pass 2 kind 2 leaves them)
+  // inside, stages 1..3, float only.
+  static cudaError_t residual_blend(HostPlanes Fx, HostPlanes Fy, int64_t rows, int64_t cols, double dx, double jp_lo,
+                                    double jp_hi, int stage, HostPlanes Qn, HostPlanes Qs, HostPlanes Qo,
+                                    const StepCtl* ctl, cudaStream_t st);
   static cudaError_t flux(HostView q, int64_t rows, int64_t cols, double gamma, bool ydir, void* out, cudaStream_t st);
   static cudaError_t con2primi(HostView q, int64_t rows, int64_t cols, double gamma, void* p, void* a, void* rho,
                                void* u, void* v, void* h, cudaStream_t st);

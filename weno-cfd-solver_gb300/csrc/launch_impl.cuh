@@ -231,6 +231,26 @@ cudaError_t Launch<H, FAST>::residual(HostPlanes Fx, HostPlanes Fy, int64_t rows
 }
 
 template <class H, bool FAST>
+cudaError_t Launch<H, FAST>::residual_blend(HostPlanes Fx, HostPlanes Fy, int64_t rows, int64_t cols, double dx,
+                                            double jp_lo, double jp_hi, int stage, HostPlanes Qn, HostPlanes Qs,
+                                            HostPlanes Qo, const StepCtl* ctl, cudaStream_t st) {
+  using namespace detail;
+  if (rows <= 0 || cols <= 0) return cudaSuccess;
+  if constexpr (is_f32<H>) {
+    const Shape g = shape<float>(rows, cols);
+    const auto X = planes<float>(Fx), Yp = planes<float>(Fy), N = planes<float>(Qn), S = planes<float>(Qs),
+               O = planes<float>(Qo);
+    const float d = (float)dx, lo = (float)jp_lo, hi = (float)jp_hi;
+    if (stage == 1) k_residual_blend<1><<<g.grid, g.block, 0, st>>>(X, Yp, rows, cols, d, lo, hi, N, S, O, ctl);
+    else if (stage == 2) k_residual_blend<2><<<g.grid, g.block, 0, st>>>(X, Yp, rows, cols, d, lo, hi, N, S, O, ctl);
+    else k_residual_blend<3><<<g.grid, g.block, 0, st>>>(X, Yp, rows, cols, d, lo, hi, N, S, O, ctl);
+    return cudaGetLastError();
+  } else {
+    return cudaErrorNotSupported;
+  }
+}
+
+template <class H, bool FAST>
 cudaError_t Launch<H, FAST>::flux(HostView q, int64_t rows, int64_t cols, double gamma, bool ydir, void* out,
                                   cudaStream_t st) {
   using T = dev_t<H>;
