@@ -19,6 +19,17 @@ constexpr int kStagedConfig = 4;
 constexpr int kTileTX[kNumTileConfigs] = {8, 16, 16, 8, 16};
 constexpr int kTileTY[kNumTileConfigs] = {32, 32, 16, 64, 32};
 
+// The fused stage kernel of one tile shape (batch_tile.cuh; each shape of each FP64
+// arithmetic is a translation unit of its own, so that they compile in parallel).
+template <class T, bool FAST, int TX, int TY>
+struct StageTile {
+  static int ctas_per_sm(bool chr, bool blend);
+  static cudaError_t launch(bool chr, bool blend, const SolveDesc* solves, SolveCtl* ctl, const void* tiles, int ntiles,
+                            int grid, const void* tmaps, const void* qn, void* qo, int stage, double gamma,
+                            double jp_lo, double jp_hi, double weps, int skip_tile, unsigned long long wait_ns,
+                            cudaStream_t st);
+};
+
 template <class T, bool FAST>
 struct BatchLaunch {
   // TMA box of one tile: columns (innermost, also the shared-memory row pitch) and rows.

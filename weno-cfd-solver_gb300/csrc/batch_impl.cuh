@@ -16,39 +16,6 @@ constexpr size_t tile_smem() {
   return sizeof(T) * (size_t)TileGeom<TX, TY, BLEND>::TOTAL;
 }
 
-template <class T, bool FAST, bool CHAR, bool BLEND, int TX, int TY>
-cudaError_t launch_stage(const SolveDesc* solves, SolveCtl* ctl, const int4* tiles, int ntiles, int grid,
-                         const CUtensorMap* tmaps, const T* qn, T* qo, int stage, T gamma, T jp_lo, T jp_hi, T weps,
-                         int skip_tile, unsigned long long wait_ns, cudaStream_t st) {
-  constexpr size_t sm = tile_smem<T, TX, TY, BLEND>();
-  if constexpr (sm > 227 * 1024) {
-    return cudaErrorInvalidConfiguration;
-  } else {
-    auto k = k_stage_tiles<T, FAST, CHAR, BLEND, TX, TY, kNT>;
-    // The attribute is per device and cheap to set: set it on every launch (also
-    // keeps host threads from racing on a cached flag).
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    k<<<grid, kNT, sm, st>>>(solves, ctl, tiles, ntiles, tmaps, qn, qo, stage, gamma, jp_lo, jp_hi, weps, skip_tile,
-                             wait_ns);
-    return cudaGetLastError();
-  }
-}
-
-template <class T, bool FAST, bool CHAR, bool BLEND, int TX, int TY>
-int occupancy() {
-  constexpr size_t sm = tile_smem<T, TX, TY, BLEND>();
-  if constexpr (sm > 227 * 1024) {
-    return 0;
-  } else {
-    auto k = k_stage_tiles<T, FAST, CHAR, BLEND, TX, TY, kNT>;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) return 0;
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kNT, sm) != cudaSuccess) return 0;
-    return n;
-  }
-}
-
 }  // namespace bdetail
 }  // inline namespace WENO_TU_NS
 
@@ -83,13 +50,8 @@ size_t BatchLaunch<H, FAST>::smem_bytes(int cfg, bool blend) {
 
 template <class H, bool FAST>
 int BatchLaunch<H, FAST>::ctas_per_sm(int cfg, bool chr, bool blend) {
-  using T = dev_t<H>;
   int r = 0;
-#define WENO_OCC(TX, TY)                                                                   \
-  if (chr && blend) r = bdetail::occupancy<T, FAST, true, true, TX, TY>();                 \
-  else if (chr) r = bdetail::occupancy<T, FAST, true, false, TX, TY>();                    \
-  else if (blend) r = bdetail::occupancy<T, FAST, false, true, TX, TY>();                  \
-  else r = bdetail::occupancy<T, FAST, false, false, TX, TY>();
+#define WENO_OCC(TX, TY) r = StageTile<H, FAST, TX, TY>::ctas_per_sm(chr, blend)
   WENO_TILE_SWITCH(cfg, WENO_OCC)
 #undef WENO_OCC
   return r;
@@ -100,26 +62,11 @@ cudaError_t BatchLaunch<H, FAST>::stage(int cfg, bool chr, bool blend, const Sol
                                         const void* tiles, int ntiles, int grid, const void* tmaps, const void* qn,
                                         void* qo, int stage, double gamma, double jp_lo, double jp_hi,
                                         double weps, int skip_tile, unsigned long long wait_ns, cudaStream_t st) {
-  using T = dev_t<H>;
   if (ntiles <= 0 || grid <= 0) return cudaSuccess;
-  const int4* tl = static_cast<const int4*>(tiles);
-  const CUtensorMap* a = static_cast<const CUtensorMap*>(tmaps);
-  const T* b = static_cast<const T*>(qn);
-  T* o = static_cast<T*>(qo);
   cudaError_t e = cudaSuccess;
-#define WENO_ST(TX, TY)                                                                                           \
-  if (chr && blend)                                                                                               \
-    e = bdetail::launch_stage<T, FAST, true, true, TX, TY>(solves, ctl, tl, ntiles, grid, a, b, o, stage, (T)gamma, \
-                                                           (T)jp_lo, (T)jp_hi, (T)weps, skip_tile, wait_ns, st);                               \
-  else if (chr)                                                                                                   \
-    e = bdetail::launch_stage<T, FAST, true, false, TX, TY>(solves, ctl, tl, ntiles, grid, a, b, o, stage,         \
-                                                            (T)gamma, (T)jp_lo, (T)jp_hi, (T)weps, skip_tile, wait_ns, st);                    \
-  else if (blend)                                                                                                 \
-    e = bdetail::launch_stage<T, FAST, false, true, TX, TY>(solves, ctl, tl, ntiles, grid, a, b, o, stage,         \
-                                                            (T)gamma, (T)jp_lo, (T)jp_hi, (T)weps, skip_tile, wait_ns, st);                    \
-  else                                                                                                            \
-    e = bdetail::launch_stage<T, FAST, false, false, TX, TY>(solves, ctl, tl, ntiles, grid, a, b, o, stage,        \
-                                                             (T)gamma, (T)jp_lo, (T)jp_hi, (T)weps, skip_tile, wait_ns, st);
+#define WENO_ST(TX, TY)                                                                                              \
+  e = StageTile<H, FAST, TX, TY>::launch(chr, blend, solves, ctl, tiles, ntiles, grid, tmaps, qn, qo, stage, gamma, \
+                                         jp_lo, jp_hi, weps, skip_tile, wait_ns, st)
   WENO_TILE_SWITCH(cfg, WENO_ST)
 #undef WENO_ST
   return e;

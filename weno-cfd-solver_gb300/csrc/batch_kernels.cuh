@@ -180,6 +180,32 @@ __device__ __forceinline__ void tile_gq_side(const T* p, int ks, int ts, T weps,
   }
 }
 
+// The averages (S = 2, FAST HLLE: the sums) of the two Gauss states of a side and of
+// their fluxes, into the left or the right pair: a loop over the sides keeps one
+// copy of the FP64 code (instruction cache, compile time).
+template <class T, bool FAST, bool Y, int S>
+__device__ __forceinline__ void put_side(int side, const T a1[4], const T a2[4], T gamma, T ql[4], T fl[4], T qr[4],
+                                         T fr[4]) {
+  T f[4];
+  if constexpr (FAST) {
+    euler_flux_sum<T, Y>(a1, a2, gamma, f);
+  } else {
+    T f1[4], f2[4];
+    euler_flux_pair<T, FAST, Y>(a1, a2, gamma, f1, f2);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) f[k] = f1[k] + f2[k];
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const T q = S == 1 ? half(T(a1[k] + a2[k])) : T(a1[k] + a2[k]);
+    const T g = S == 1 ? half(f[k]) : f[k];
+    ql[k] = side ? ql[k] : q;
+    fl[k] = side ? fl[k] : g;
+    qr[k] = q;
+    fr[k] = g;
+  }
+}
+
 // Component-wise pass 1 of one cell (five cells along the sweep, all components):
 // its states at its right face (l, q_l there) and at its left face (r, q_r there).
 template <class T, bool FAST>
@@ -369,22 +395,11 @@ __global__ void __launch_bounds__(NT) k_stage_tiles(const SolveDesc* __restrict_
       const int fi = i0 - HF + fr, jj = j0 - HF + fc;
       if (fi < 0 || fi > nx || jj < 0 || jj >= ny) continue;
       T ql[4], qr[4], fl[4], fr_[4];
-      {
-        T a1[4], a2[4], f1[4], f2[4];
-        tile_gq_side<T, FAST>(P1 + fr * G::P1XC + fc, G::P1, 1, weps, a1, a2);
-        euler_flux_pair<T, FAST, false>(a1, a2, gamma, f1, f2);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          fl[k] = S == 1 ? T(0.5) * (f1[k] + f2[k]) : f1[k] + f2[k];
-          ql[k] = S == 1 ? T(0.5) * (a1[k] + a2[k]) : a1[k] + a2[k];
-        }
-        tile_gq_side<T, FAST>(P1 + 4 * G::P1 + fr * G::P1XC + fc, G::P1, 1, weps, a1, a2);
-        euler_flux_pair<T, FAST, false>(a1, a2, gamma, f1, f2);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          fr_[k] = S == 1 ? T(0.5) * (f2[k] + f1[k]) : f2[k] + f1[k];
-          qr[k] = S == 1 ? T(0.5) * (a1[k] + a2[k]) : a1[k] + a2[k];
-        }
+#pragma unroll(is_f32<T> ? 2 : 1)
+      for (int side = 0; side < 2; ++side) {
+        T a1[4], a2[4];
+        tile_gq_side<T, FAST>(P1 + fr * G::P1XC + fc + (side ? 4 * G::P1 : 0), G::P1, 1, weps, a1, a2);
+        put_side<T, FAST, false, S>(side, a1, a2, gamma, ql, fl, qr, fr_);
       }
       tile_face_flux<T, FAST, false, BLEND, S>(ql, fl, qr, fr_, gamma, FX, G::FXR * G::FXC, e);
     }
@@ -463,22 +478,11 @@ __global__ void __launch_bounds__(NT) k_stage_tiles(const SolveDesc* __restrict_
       const int ii = i0 - HF + fr, fj = j0 - HF + fc;
       if (ii < 0 || ii >= nx || fj < 0 || fj > ny) continue;
       T ql[4], qr[4], fl[4], fr_[4];
-      {
-        T a1[4], a2[4], f1[4], f2[4];
-        tile_gq_side<T, FAST>(P1 + fr * G::P1YC + fc, G::P1, G::P1YC, weps, a1, a2);
-        euler_flux_pair<T, FAST, true>(a1, a2, gamma, f1, f2);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          fl[k] = S == 1 ? T(0.5) * (f1[k] + f2[k]) : f1[k] + f2[k];
-          ql[k] = S == 1 ? T(0.5) * (a1[k] + a2[k]) : a1[k] + a2[k];
-        }
-        tile_gq_side<T, FAST>(P1 + 4 * G::P1 + fr * G::P1YC + fc, G::P1, G::P1YC, weps, a1, a2);
-        euler_flux_pair<T, FAST, true>(a1, a2, gamma, f1, f2);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          fr_[k] = S == 1 ? T(0.5) * (f2[k] + f1[k]) : f2[k] + f1[k];
-          qr[k] = S == 1 ? T(0.5) * (a1[k] + a2[k]) : a1[k] + a2[k];
-        }
+#pragma unroll(is_f32<T> ? 2 : 1)
+      for (int side = 0; side < 2; ++side) {
+        T a1[4], a2[4];
+        tile_gq_side<T, FAST>(P1 + fr * G::P1YC + fc + (side ? 4 * G::P1 : 0), G::P1, G::P1YC, weps, a1, a2);
+        put_side<T, FAST, true, S>(side, a1, a2, gamma, ql, fl, qr, fr_);
       }
       tile_face_flux<T, FAST, true, BLEND, S>(ql, fl, qr, fr_, gamma, FY, G::FYR * G::FYC, e);
     }
@@ -614,10 +618,9 @@ __device__ __forceinline__ void staged_cell(const SolveDesc& d, const T* q, int 
 // Pass 1 of both directions for every tile: q_l, q_r of each face into P1x / P1y.
 // Qin is the pool of the stage input.
 template <class T, bool FAST, bool CHAR, int TX, int TY, int NT>
-__global__ void __launch_bounds__(NT) k_staged_pass1(const SolveDesc* __restrict__ solves,
-                                                      const SolveCtl* __restrict__ ctl,
-                                                      const int4* __restrict__ tiles, int ntiles, const T* Qin, T* W,
-                                                      T gamma, T weps) {
+__global__ void __launch_bounds__(NT)
+    k_staged_pass1(const SolveDesc* __restrict__ solves, const SolveCtl* __restrict__ ctl,
+                   const int4* __restrict__ tiles, int ntiles, const T* Qin, T* W, T gamma, T weps) {
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int4 tl = tiles[t];
     if (!ctl[tl.x].active) continue;
@@ -739,10 +742,9 @@ __device__ __forceinline__ void staged_gq_two(const f64* p, long long ks, long l
 // and the Riemann solver of every face a tile owns, into Fx / Fy.  FAST double
 // takes two transverse neighbours per thread (as the single-grid k_pass2_two).
 template <class T, bool FAST, bool BLEND, int TX, int TY, int NT>
-__global__ void __launch_bounds__(NT) k_staged_pass2(const SolveDesc* __restrict__ solves,
-                                                      const SolveCtl* __restrict__ ctl,
-                                                      const int4* __restrict__ tiles, int ntiles, T* W, T gamma,
-                                                      T weps) {
+__global__ void __launch_bounds__(NT)
+    k_staged_pass2(const SolveDesc* __restrict__ solves, const SolveCtl* __restrict__ ctl,
+                   const int4* __restrict__ tiles, int ntiles, T* W, T gamma, T weps) {
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int4 tl = tiles[t];
     if (!ctl[tl.x].active) continue;
@@ -760,76 +762,57 @@ __global__ void __launch_bounds__(NT) k_staged_pass2(const SolveDesc* __restrict
       const int nyi = ((yr1 - i0 + 1) / 2) * nyc;              // y-face pairs (ii, ii+1)
       for (int e = threadIdx.x; e < nxi + nyi; e += NT) {
         T qlA[4], flA[4], qlB[4], flB[4], qrA[4], frA[4], qrB[4], frB[4];
-        if (e < nxi) {
-          const int fi = i0 + e / nxp, jj = j0 + 2 * (e % nxp);
-          const bool two = jj + 1 < xc1;
-          const T* p = W + d.w_p1x + (long long)fi * d.l_p1x + jj;
-          staged_gq_two<false, SUM>(p, d.s_p1x, 1, two, gamma, weps, qlA, flA, qlB, flB);
-          staged_gq_two<false, SUM>(p + 4 * d.s_p1x, d.s_p1x, 1, two, gamma, weps, qrA, frA, qrB, frB);
-          tile_face_flux<T, FAST, false, BLEND, S>(qlA, flA, qrA, frA, gamma, W + d.w_fx, (int)d.s_fx,
-                                                   fi * d.ld + jj);
-          if (two)
-            tile_face_flux<T, FAST, false, BLEND, S>(qlB, flB, qrB, frB, gamma, W + d.w_fx, (int)d.s_fx,
-                                                     fi * d.ld + jj + 1);
-        } else {
-          const int e2 = e - nxi;
-          const int ii = i0 + 2 * (e2 / nyc), fj = j0 + e2 % nyc;
-          const bool two = ii + 1 < yr1;
-          const T* p = W + d.w_p1y + (long long)ii * d.l_p1y + fj;
-          staged_gq_two<true, SUM>(p, d.s_p1y, d.l_p1y, two, gamma, weps, qlA, flA, qlB, flB);
-          staged_gq_two<true, SUM>(p + 4 * d.s_p1y, d.s_p1y, d.l_p1y, two, gamma, weps, qrA, frA, qrB, frB);
-          tile_face_flux<T, FAST, true, BLEND, S>(qlA, flA, qrA, frA, gamma, W + d.w_fy, (int)d.s_fy,
-                                                  ii * d.l_p1y + fj);
-          if (two)
-            tile_face_flux<T, FAST, true, BLEND, S>(qlB, flB, qrB, frB, gamma, W + d.w_fy, (int)d.s_fy,
-                                                    (ii + 1) * d.l_p1y + fj);
+        const bool x = e < nxi;
+        const int e2 = e - nxi;
+        const int fi = i0 + (x ? e / nxp : 2 * (e2 / nyc)), fj = j0 + (x ? 2 * (e % nxp) : e2 % nyc);
+        const bool two = x ? fj + 1 < xc1 : fi + 1 < yr1;
+        const T* p = x ? W + d.w_p1x + (long long)fi * d.l_p1x + fj : W + d.w_p1y + (long long)fi * d.l_p1y + fj;
+        const long long ks = x ? d.s_p1x : d.s_p1y, ts = x ? 1 : d.l_p1y;
+#pragma unroll 1
+        for (int side = 0; side < 2; ++side) {  // one copy of the code, left then right
+          if (x) staged_gq_two<false, SUM>(p + side * 4 * ks, ks, ts, two, gamma, weps, qrA, frA, qrB, frB);
+          else staged_gq_two<true, SUM>(p + side * 4 * ks, ks, ts, two, gamma, weps, qrA, frA, qrB, frB);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            qlA[k] = side ? qlA[k] : qrA[k];
+            flA[k] = side ? flA[k] : frA[k];
+            qlB[k] = side ? qlB[k] : qrB[k];
+            flB[k] = side ? flB[k] : frB[k];
+          }
+        }
+        T* F = W + (x ? d.w_fx : d.w_fy);
+        const int fs = (int)(x ? d.s_fx : d.s_fy);
+        int o = x ? fi * d.ld + fj : fi * d.l_p1y + fj;
+#pragma unroll 1
+        for (int face = 0; face < (two ? 2 : 1); ++face) {
+          if (x) tile_face_flux<T, FAST, false, BLEND, S>(qlA, flA, qrA, frA, gamma, F, fs, o);
+          else tile_face_flux<T, FAST, true, BLEND, S>(qlA, flA, qrA, frA, gamma, F, fs, o);
+          o += x ? 1 : d.l_p1y;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) qlA[k] = qlB[k], flA[k] = flB[k], qrA[k] = qrB[k], frA[k] = frB[k];
         }
       }
     } else {
       // FAST HLLE takes the Gauss-point sums (twice the face averages)
       constexpr int S = FAST && !BLEND ? 2 : 1;
       for (int e = threadIdx.x; e < nxf + nyf; e += NT) {
-        T ql[4], qr[4], fl[4], fr_[4], a1[4], a2[4], f1[4], f2[4];
-        if (e < nxf) {
-          const int fi = i0 + e / nxc, jj = j0 + e % nxc;
-          // the five transverse pass-1 states J = jj-2 .. jj+2 (columns jj .. jj+4)
-          const T* p = W + d.w_p1x + (long long)fi * d.l_p1x + jj;
-          tile_gq_side<T, FAST>(p, (int)d.s_p1x, 1, weps, a1, a2);
-          euler_flux_pair<T, FAST, false>(a1, a2, gamma, f1, f2);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            fl[k] = S == 1 ? T(0.5) * (f1[k] + f2[k]) : f1[k] + f2[k];
-            ql[k] = S == 1 ? T(0.5) * (a1[k] + a2[k]) : a1[k] + a2[k];
-          }
-          tile_gq_side<T, FAST>(p + 4 * d.s_p1x, (int)d.s_p1x, 1, weps, a1, a2);
-          euler_flux_pair<T, FAST, false>(a1, a2, gamma, f1, f2);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            fr_[k] = S == 1 ? T(0.5) * (f2[k] + f1[k]) : f2[k] + f1[k];
-            qr[k] = S == 1 ? T(0.5) * (a1[k] + a2[k]) : a1[k] + a2[k];
-          }
-          tile_face_flux<T, FAST, false, BLEND, S>(ql, fl, qr, fr_, gamma, W + d.w_fx, (int)d.s_fx, fi * d.ld + jj);
-        } else {
-          const int e2 = e - nxf;
-          const int ii = i0 + e2 / nyc, fj = j0 + e2 % nyc;
-          // the five transverse pass-1 states I = ii-2 .. ii+2 (rows ii .. ii+4)
-          const T* p = W + d.w_p1y + (long long)ii * d.l_p1y + fj;
-          tile_gq_side<T, FAST>(p, (int)d.s_p1y, d.l_p1y, weps, a1, a2);
-          euler_flux_pair<T, FAST, true>(a1, a2, gamma, f1, f2);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            fl[k] = S == 1 ? T(0.5) * (f1[k] + f2[k]) : f1[k] + f2[k];
-            ql[k] = S == 1 ? T(0.5) * (a1[k] + a2[k]) : a1[k] + a2[k];
-          }
-          tile_gq_side<T, FAST>(p + 4 * d.s_p1y, (int)d.s_p1y, d.l_p1y, weps, a1, a2);
-          euler_flux_pair<T, FAST, true>(a1, a2, gamma, f1, f2);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            fr_[k] = S == 1 ? T(0.5) * (f2[k] + f1[k]) : f2[k] + f1[k];
-            qr[k] = S == 1 ? T(0.5) * (a1[k] + a2[k]) : a1[k] + a2[k];
-          }
-          tile_face_flux<T, FAST, true, BLEND, S>(ql, fl, qr, fr_, gamma, W + d.w_fy, (int)d.s_fy, ii * d.l_p1y + fj);
+        T ql[4], qr[4], fl[4], fr_[4];
+        const bool x = e < nxf;
+        const int e2 = e - nxf;
+        const int fi = i0 + (x ? e / nxc : e2 / nyc), fj = j0 + (x ? e % nxc : e2 % nyc);
+        // the five transverse pass-1 states: columns fj .. fj+4 of an x face, rows fi .. fi+4 of a y face
+        const T* p = x ? W + d.w_p1x + (long long)fi * d.l_p1x + fj : W + d.w_p1y + (long long)fi * d.l_p1y + fj;
+        const long long ks = x ? d.s_p1x : d.s_p1y;
+        const int ts = x ? 1 : d.l_p1y;
+#pragma unroll(is_f32<T> ? 2 : 1)
+        for (int side = 0; side < 2; ++side) {
+          T a1[4], a2[4];
+          tile_gq_side<T, FAST>(p + side * 4 * ks, (int)ks, ts, weps, a1, a2);
+          if (x) put_side<T, FAST, false, S>(side, a1, a2, gamma, ql, fl, qr, fr_);
+          else put_side<T, FAST, true, S>(side, a1, a2, gamma, ql, fl, qr, fr_);
         }
+        if (x) tile_face_flux<T, FAST, false, BLEND, S>(ql, fl, qr, fr_, gamma, W + d.w_fx, (int)d.s_fx, fi * d.ld + fj);
+        else tile_face_flux<T, FAST, true, BLEND, S>(ql, fl, qr, fr_, gamma, W + d.w_fy, (int)d.s_fy, fi * d.l_p1y + fj);
       }
     }
   }

@@ -1,7 +1,7 @@
 """Build libweno_gb300.so (sm_103a) in place, next to this file.
 
-Three translation units are compiled in parallel with nvcc and linked into one
-shared library with a C ABI (include/weno_gb300.h):
+The translation units (UNITS) are compiled in parallel with nvcc and linked into one
+shared library with a C ABI (include/weno_gb300.h), among them:
 
 * csrc/tu_exact.cu -- kernels with --fmad=false (reference-identical doubles)
 * csrc/tu_fast.cu  -- kernels with FMA contraction and the FAST forms
@@ -40,6 +40,13 @@ UNITS = {
     "batch_f64.cu": ["--fmad=true"],
     "batch_f32.cu": ["--fmad=true"],
 }
+# The fused FP64 tile kernels, one unit per tile shape and arithmetic (batch_tile.cu):
+# most of the compile time, so they run in parallel.
+for _x, _y in ((8, 32), (16, 32), (16, 16), (8, 64)):
+    _d = [f"-DWENO_TILE_X={_x}", f"-DWENO_TILE_Y={_y}"]
+    UNITS[f"batch_tile.cu:exact_{_x}x{_y}"] = ["--fmad=false", f"-DWENO_TILE_NS=tile_exact_{_x}x{_y}", *_d]
+    UNITS[f"batch_tile.cu:fast_{_x}x{_y}"] = ["--fmad=true", "-DWENO_TILE_FAST", f"-DWENO_TILE_NS=tile_fast_{_x}x{_y}",
+                                              *_d]
 
 
 def _nvcc() -> str:
@@ -69,8 +76,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(objdir, exist_ok=True)
 
     def compile_unit(name):
-        obj = os.path.join(objdir, name.replace(".cu", ".o"))
-        cmd = [nvcc, *COMMON, *UNITS[name], "-c", os.path.join(CSRC, name), "-o", obj]
+        obj = os.path.join(objdir, name.replace(".cu", "").replace(":", "_") + ".o")
+        cmd = [nvcc, *COMMON, *UNITS[name], "-c", os.path.join(CSRC, name.split(":")[0]), "-o", obj]
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
         r = subprocess.run(cmd, capture_output=True, text=True)
@@ -80,8 +87,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(r.stderr)
         return obj
 
-    with cf.ThreadPoolExecutor(max_workers=len(UNITS)) as ex:
-        objs = list(ex.map(compile_unit, UNITS))
+    # the longest first
+    units = sorted(UNITS, key=lambda u: not u.startswith("batch_tile"))
+    with cf.ThreadPoolExecutor(max_workers=max(4, os.cpu_count() or 4)) as ex:
+        objs = list(ex.map(compile_unit, units))
     tmp = LIB_PATH + ".tmp"
     r = subprocess.run([nvcc, "-shared", *ARCH, "-o", tmp, *objs], capture_output=True, text=True)
     if r.returncode != 0:
