@@ -80,20 +80,21 @@ cudaError_t BatchLaunch<H, FAST>::staged(bool chr, bool blend, const SolveDesc* 
   using T = dev_t<H>;
   if (ntiles <= 0 || grid <= 0) return cudaSuccess;
   constexpr int TX = kTileTX[kStagedConfig], TY = kTileTY[kStagedConfig], NT = bdetail::kNT;
+  constexpr int NP = kStagedThreads<T, FAST>;
   const int4* tl = static_cast<const int4*>(tiles);
   T* W = static_cast<T*>(ws);
   const T* Qs = static_cast<const T*>(qs);
   if (chr)
-    k_staged_pass1<T, FAST, true, TX, TY, NT><<<grid, NT, 0, st>>>(solves, ctl, tl, ntiles, Qs, W, (T)gamma, (T)weps);
+    k_staged_pass1<T, FAST, true, TX, TY, NP><<<grid, NP, 0, st>>>(solves, ctl, tl, ntiles, Qs, W, (T)gamma, (T)weps);
   else
-    k_staged_pass1<T, FAST, false, TX, TY, NT><<<grid, NT, 0, st>>>(solves, ctl, tl, ntiles, Qs, W, (T)gamma,
+    k_staged_pass1<T, FAST, false, TX, TY, NP><<<grid, NP, 0, st>>>(solves, ctl, tl, ntiles, Qs, W, (T)gamma,
                                                                      (T)weps);
   cudaError_t e = cudaGetLastError();
   if (e) return e;
   if (blend)
-    k_staged_pass2<T, FAST, true, TX, TY, NT><<<grid, NT, 0, st>>>(solves, ctl, tl, ntiles, W, (T)gamma, (T)weps);
+    k_staged_pass2<T, FAST, true, TX, TY, NP><<<grid, NP, 0, st>>>(solves, ctl, tl, ntiles, W, (T)gamma, (T)weps);
   else
-    k_staged_pass2<T, FAST, false, TX, TY, NT><<<grid, NT, 0, st>>>(solves, ctl, tl, ntiles, W, (T)gamma, (T)weps);
+    k_staged_pass2<T, FAST, false, TX, TY, NP><<<grid, NP, 0, st>>>(solves, ctl, tl, ntiles, W, (T)gamma, (T)weps);
   if ((e = cudaGetLastError())) return e;
   const T* Qn = static_cast<const T*>(qn);
   T* Qo = static_cast<T*>(qo);

@@ -615,10 +615,21 @@ __device__ __forceinline__ void staged_cell(const SolveDesc& d, const T* q, int 
   if (flip) v[2] = -v[2];
 }
 
+// Threads and resident blocks of the staged passes.  FAST FP64: blocks of 128, three
+// per SM (168 registers); blocks of 256 at the 196-214 registers that pass 2 takes
+// unbounded leave 8 warps per SM, too few for the FP64 pipe.  Six boards of 128-1024
+// cells a side, two steps: 14.0 to 13.3 ms component-wise with the blend, 15.6 to
+// 14.7 ms characteristic HLLE.  Exact FP64 keeps 256 unbounded: at 168 registers the
+// component-wise steps take 9.2 ms for 8.5 and the characteristic ones 17.3 for 13.2.
+template <class T, bool FAST>
+constexpr int kStagedThreads = is_native_f64<T> && FAST ? 128 : 256;
+template <class T, bool FAST>
+constexpr int kStagedBlocks = is_native_f64<T> && FAST ? 3 : 0;
+
 // Pass 1 of both directions for every tile: q_l, q_r of each face into P1x / P1y.
 // Qin is the pool of the stage input.
 template <class T, bool FAST, bool CHAR, int TX, int TY, int NT>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, kStagedBlocks<T, FAST>)
     k_staged_pass1(const SolveDesc* __restrict__ solves, const SolveCtl* __restrict__ ctl,
                    const int4* __restrict__ tiles, int ntiles, const T* Qin, T* W, T gamma, T weps) {
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -742,7 +753,7 @@ __device__ __forceinline__ void staged_gq_two(const f64* p, long long ks, long l
 // and the Riemann solver of every face a tile owns, into Fx / Fy.  FAST double
 // takes two transverse neighbours per thread (as the single-grid k_pass2_two).
 template <class T, bool FAST, bool BLEND, int TX, int TY, int NT>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, kStagedBlocks<T, FAST>)
     k_staged_pass2(const SolveDesc* __restrict__ solves, const SolveCtl* __restrict__ ctl,
                    const int4* __restrict__ tiles, int ntiles, T* W, T gamma, T weps) {
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
