@@ -2,18 +2,19 @@
 //
 // Every function follows the reference's Rust core (weno_ext/src/utils.rs,
 // weno.rs, riemann.rs) and is templated on
-//   T    -- double or float, the arithmetic type;
+//   T    -- f64 (a double whose operations are spelled for the FP64 pipe,
+//           f64.cuh), float or df64, the arithmetic type;
 //   FAST -- false: the reference's operation order, so that a translation unit
 //           compiled with --fmad=false reproduces the Rust IEEE-754 doubles bit
-//           for bit; true: the same mathematics with fewer FP64 divisions
-//           (shared reciprocals, a common-denominator form of the WENO weights)
-//           and FMA contraction, checked against the oracle by tolerance.
+//           for bit; true: the same mathematics with fewer FP64 operations and
+//           FMA contraction, checked against the oracle by tolerance.
 //
-// GB300 executes FP64 at 1/64 of the FP32 rate and a correctly rounded FP64
-// divide costs about ten FMA slots, so the FAST forms are written to remove
-// divides and square roots rather than memory traffic; the FP64 reciprocals
-// and square roots that remain take the seeded Newton forms of fp64_fast.cuh
-// (three and five FP64 operations, within 1-2 ulp).
+// GB300 executes FP64 at 1/64 of the FP32 rate and every FP64 kernel here is bound
+// by that pipe, so both arithmetics are written to need few of its slots rather
+// than little memory traffic: additions and products issue as FMAs (16 cycles a
+// warp and SM where DADD and DMUL take 19), comparisons, divisions and square
+// roots run on the integer pipe (rn64.cuh), and the FAST WENO weights run on the
+// FP32 pipe as float pairs (ffw.cuh).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -68,17 +69,13 @@ __device__ __forceinline__ T mul_add(T a, T b, T c) {
   else return a * b + c;
 }
 
-// Clamps and tests against a non-negative bound.  FAST native double reads the
-// operands' bits as signed 64-bit integers: for non-negative doubles that order
-// is the numeric order, and every value with the sign bit set (negatives, -0)
-// reads below any non-negative bound, so the result is max(x, c) / x < c for
-// every non-NaN x, on the integer pipe instead of an FP64 slot (GB300 issues
-// FP64 compares and min/max at the FP64 rate).  A NaN x with the sign bit clear
-// passes through where fmax would return the bound; NaN propagates through
-// the neighbouring arithmetic either way.  Used by the fluxes and the Riemann
-// solvers (pass 2); the pass-1 Roe average and limiter keep the FP64 forms:
-// there the integer forms measured 1.6 % slower, at 5 resident CTAs per SM
-// and equally when held to the FP64 build's 4.
+// max(x, c) against a non-negative bound.  FAST native double reads the operands'
+// bits as signed 64-bit integers: for non-negative doubles that order is the numeric
+// order, and every value with the sign bit set (negatives, -0) reads below any
+// non-negative bound, so the result is max(x, c) for every non-NaN x, in one integer
+// compare (an f64's general compare orders the bits of both signs and looks for
+// NaN).  A NaN x with the sign bit clear passes through where fmax would return the
+// bound; NaN propagates through the neighbouring arithmetic either way.
 template <class T, bool FAST>
 __device__ __forceinline__ T cmax(T x, T c) {
   if constexpr (FAST && is_native_f64<T>) return f64_bits(x) > f64_bits(c) ? x : c;

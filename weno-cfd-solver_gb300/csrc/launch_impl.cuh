@@ -1,5 +1,5 @@
-// Launcher definitions (see launch_api.h).  Included only by tu_exact.cu and
-// tu_fast.cu.
+// Launcher definitions (see launch_api.h).  Included only by tu_exact.cu, tu_fast.cu
+// and tu_df64.cu.
 #pragma once
 
 #include "kernels.cuh"
