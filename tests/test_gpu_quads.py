@@ -49,3 +49,28 @@ def test_reconstruct(wx, orc, mn, ydir):
         got = (wx.weno_y_py if ydir else wx.weno_x_py)(q, G, cons=cons)
         for a, b in zip(got, ref):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("mn", [(8, 8), (9, 41), (150, 160)], ids=lambda s: f"{s[0]}x{s[1]}")
+@pytest.mark.parametrize("hlle", [True, False], ids=["hlle", "blend"])
+def test_workspace_for_one_sweep(wx, mn, hlle):
+    """A workspace without the second sweep's pass-1 planes runs the sweeps in turn, to the same
+    bits; a smaller one is refused."""
+    import torch
+    from weno_ext import _lib
+    L = _lib.load()
+    m, n = mn
+    q = torch.from_numpy(quadrant(np.random.default_rng(m), m - 6, n - 6)).cuda()
+    full = L.weno_l_local_workspace(m, n, int(hlle))
+    p1 = -(-max((m - 5) * n, m * (n - 5)) // 64) * 64  # planes are padded to 64 values
+    one = full - 2 * 4 * 8 * p1
+    outs = []
+    for wsb in (full, one, one - 256):
+        out = torch.zeros((m - 6, n - 6, 4), dtype=torch.float64, device="cuda")
+        ws = torch.zeros(full, dtype=torch.uint8, device="cuda")
+        rc = L.weno_l_local(q.data_ptr(), m, n, q.shape[2], *q.stride(), 0.01, G, int(hlle), 0.2, 1.0, 0, _lib.EXACT,
+                            out.data_ptr(), ws.data_ptr(), wsb, torch.cuda.current_stream().cuda_stream)
+        outs.append((rc, out.cpu().numpy()))
+    assert outs[0][0] == 0 and outs[1][0] == 0 and outs[2][0] != 0
+    assert np.abs(outs[0][1]).max() > 0
+    assert np.array_equal(outs[0][1], outs[1][1])
