@@ -420,10 +420,9 @@ struct weno_solver {
 
 namespace {
 
-// pass 1 and 2 of both sweeps and the residual; two sensor blends (FP32: inside the
-// residual); df64: the marked
-// faces of the two pass 1
-// faces of the two pass 1; small FP64 grids: both sweeps in one launch per pass
+// Pass 1 and 2 of both sweeps and the residual; two sensor blends (FP32: inside the
+// residual); df64: the marked faces of the two pass 1; small FP64 grids: both sweeps
+// in one launch per pass.
 int launches_per_residual(const weno_solver* s) {
   return 5 + (s->force_hlle || s->prec == 32 ? 0 : 2) + (s->prec == 48 ? 2 : 0) - (s->layout->quads ? 2 : 0);
 }
