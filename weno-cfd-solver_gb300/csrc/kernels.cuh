@@ -69,8 +69,9 @@ __device__ __forceinline__ bool locate(int64_t rows, int64_t cols, int64_t& row,
 constexpr uint32_t kDf64Marker = 0x7fc0df64u;
 
 // Resident blocks per SM that pass 1 is compiled for (4 warps each).  FP64: 4, at
-// 128 registers (at 156 and three blocks the 2048^2 step took 2.6 % longer); FP32: 8,
-// at 64 (6: 2.7 % longer, 7: 1 %, 9 spills: 1.6 %); df64: 4 (3: 2 % longer).
+// 128 registers (at three blocks the FAST 2048^2 step took 2.6 % longer, exact ones
+// of 300 x 310 2.6 % and of 2000 x 1500 0.3 %); FP32: 8, at 64 (6: 2.7 % longer, 7:
+// 1 %, 9 spills: 1.6 %); df64: 4 (3: 2 % longer).
 template <class T>
 constexpr int kPass1Blocks = is_native_f64<T> ? 4 : (is_f32<T> ? 8 : 4);
 
@@ -320,6 +321,15 @@ __device__ __forceinline__ void gq_side_two(const Planes<T>& P, int64_t row, int
   }
 }
 
+// Resident blocks per SM that k_pass2_two is compiled for.  The FP64 blend takes 136
+// registers in the x sweep unbounded, three blocks; at four (128) two component-wise
+// blend steps of 1024 x 1030 take 9.42-9.56 ms for 9.73-9.82, characteristic ones of
+// 2000 x 700 16.68 for 17.04.  The others fit four (FP64) or seven to eight (FP32) as
+// they are, and slow down with a bound: FP64 HLLE by 0.5 % at 4, FP32 by 0.1-0.8 % at 8
+// and 3 % at 9.
+template <class T, int OUT>
+constexpr int kPass2Blocks = is_native_f64<T> && OUT == P2_BLEND ? 4 : 0;
+
 // FAST pass 2 with two faces per thread along the transverse direction
 // (columns for the x sweep, rows for the y sweep): the six transverse values
 // of each component serve both faces, whose Gauss-point reconstructions share
@@ -327,7 +337,7 @@ __device__ __forceinline__ void gq_side_two(const Planes<T>& P, int64_t row, int
 // with the weights on the FP32 pipe (453 with FP64 weights), a 2048^2 HLLE sweep
 // 1.72 ms for 3.74, the pipe 84-86 % busy.
 template <class T, bool Y, int OUT>
-__global__ void __launch_bounds__(128) k_pass2_two(Planes<T> PL, Planes<T> PR, int64_t rows, int64_t cols, T gamma,
+__global__ void __launch_bounds__(128, kPass2Blocks<T, OUT>) k_pass2_two(Planes<T> PL, Planes<T> PR, int64_t rows, int64_t cols, T gamma,
                                                     Pass2Dst dst, T weps) {
   int64_t row, col;
   if (!locate(Y ? (rows + 1) / 2 : rows, Y ? cols : (cols + 1) / 2, row, col)) return;
