@@ -225,25 +225,6 @@ void fl_free(std::map<long long, long long>& fl, long long off, long long len) {
 long long pool_alloc(weno_batch* b, long long len) { return fl_alloc(b->free_list, len); }
 void pool_free(weno_batch* b, long long off, long long len) { fl_free(b->free_list, off, len); }
 
-// Face workspace of one solve in the staged configuration (element counts; see
-// k_staged_pass1): fills the layout fields of `d` with offsets relative to the
-// solve's block and returns the block's length.
-long long staged_layout(SolveDesc& d, int lq, int nf) {
-  auto up = [lq](long long x) { return (x + lq - 1) / lq * lq; };
-  const long long nx = d.nx, ny = d.ny;
-  d.l_p1x = (int)up(ny + 4);
-  d.l_p1y = (int)up(ny + 1);
-  d.s_p1x = align64((nx + 1) * d.l_p1x);
-  d.s_p1y = align64((nx + 4) * d.l_p1y);
-  d.s_fx = align64((nx + 1) * d.ld);
-  d.s_fy = align64(nx * d.l_p1y);
-  d.w_p1x = 0;
-  d.w_p1y = 8 * d.s_p1x;
-  d.w_fx = d.w_p1y + 8 * d.s_p1y;
-  d.w_fy = d.w_fx + nf * d.s_fx;
-  return d.w_fy + nf * d.s_fy;
-}
-
 // Workspace elements reserved per pool cell in the staged configuration: the
 // face arrays of a solve take about 16 + 2 NF values per cell, more for small
 // grids (halo rows and columns, 64-element plane alignment).

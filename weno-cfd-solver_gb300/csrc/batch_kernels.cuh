@@ -21,26 +21,11 @@
 #pragma once
 
 #include "euler_math.cuh"
+#include "solve_desc.h"
 #include "step_ctl.h"
 #include "tma.cuh"
 
 namespace weno {
-
-struct SolveDesc {
-  long long off;  // element offset of plane 0 in each pool
-  long long ps;   // plane stride (elements)
-  int nx, ny;
-  int ld;         // row pitch (elements): ny rounded up to a multiple of 16 bytes
-  int bc;         // 0 transmissive (mirror), 1 oblique-shock / DMR segments
-  int bound;      // DMR: last row of the inflow segment on the lower boundary
-  double dx;      // cell size (dx = dy)
-  double post[8]; // DMR inflow state: conserved channels 0..3, primitive channels 4..7
-  // Staged tile configuration only: this solve's face workspace, element offsets
-  // in the workspace pool (see k_staged_pass1).
-  long long w_p1x, w_p1y, w_fx, w_fy;  // plane 0 of each array
-  long long s_p1x, s_p1y, s_fx, s_fy;  // plane strides
-  int l_p1x, l_p1y;                    // row pitches of P1x and of P1y / Fy (Fx uses ld)
-};
 
 struct SolveCtl {
   double t, t_end, dt, cfl_dx;
@@ -132,12 +117,12 @@ struct TileGeom {
   static constexpr int TOTAL = U_ELEMS + P1_ELEMS + F_ELEMS + DX_ELEMS;
 };
 
-// Sensor weight at face (fr, fc) of a local face array of R x C entries whose
-// global origin is (gr0, gc0) in a global face array of GR x GC entries
-// (riemann.rs:352-410: central differences, one-sided on the global edges).
-template <class T, bool FAST>
-__device__ __forceinline__ T tile_sensor(const T* pbar, int R, int C, int fr, int fc, int gr, int gc, int GR, int GC,
-                                         T jp_lo, T jp_hi) {
+// Sensor weight at element e, row pitch C, of a local face array: face (gr, gc) of a
+// global face array of GR x GC entries (riemann.rs:352-410: central differences,
+// one-sided on the global edges).
+template <class T, bool FAST, class I>
+__device__ __forceinline__ T tile_sensor(const T* pbar, int C, I e, int gr, int gc, int GR, int GC, T jp_lo,
+                                         T jp_hi) {
   const int min_dim = GR < GC ? GR : GC;
   const T dx = T(1.0) / T((double)min_dim);
   const T two_dx = T(2.0) * dx;
@@ -145,10 +130,9 @@ __device__ __forceinline__ T tile_sensor(const T* pbar, int R, int C, int fr, in
   const int rb = gr == 0 ? 1 : (gr == GR - 1 ? 0 : 1);
   const int ca = gc == 0 ? 0 : (gc == GC - 1 ? -1 : -1);
   const int cb = gc == 0 ? 1 : (gc == GC - 1 ? 0 : 1);
-  (void)R;
-  const T p = pbar[fr * C + fc];
-  const T dpdx = qdiv<T, FAST>(pbar[(fr + rb) * C + fc] - pbar[(fr + ra) * C + fc], two_dx);
-  const T dpdy = qdiv<T, FAST>(pbar[fr * C + fc + cb] - pbar[fr * C + fc + ca], two_dx);
+  const T p = pbar[e];
+  const T dpdx = qdiv<T, FAST>(pbar[e + rb * C] - pbar[e + ra * C], two_dx);
+  const T dpdy = qdiv<T, FAST>(pbar[e + cb] - pbar[e + ca], two_dx);
   return sensor_weight<T, FAST>(dpdx, dpdy, p, jp_lo, jp_hi);
 }
 
@@ -156,8 +140,8 @@ __device__ __forceinline__ T tile_sensor(const T* pbar, int R, int C, int fr, in
 // points at the first of five transverse values of component 0, `ks` is the
 // component stride and `ts` the transverse stride.  FAST float runs the
 // components as two packed pairs on the FP32x2 instructions.
-template <class T, bool FAST>
-__device__ __forceinline__ void tile_gq_side(const T* p, int ks, int ts, T weps, T a1[4], T a2[4]) {
+template <class T, bool FAST, class I>
+__device__ __forceinline__ void tile_gq_side(const T* p, I ks, int ts, T weps, T a1[4], T a2[4]) {
   if constexpr (FAST && is_f32<T>) {
 #pragma unroll
     for (int k = 0; k < 4; k += 2) {
@@ -236,9 +220,9 @@ __device__ __forceinline__ void cell_states(const T c[5][4], T weps, T l[4], T r
 // Riemann solver of one tile face and its store into the face buffer F
 // (HLLE flux planes, or HLLC + HLLE + mean pressure for the sensor blend).
 // S = 2 (HLLE only): states and fluxes are twice the face averages.
-template <class T, bool FAST, bool Y, bool BLEND, int S = 1>
+template <class T, bool FAST, bool Y, bool BLEND, int S, class I>
 __device__ __forceinline__ void tile_face_flux(const T ql[4], const T fl[4], const T qr[4], const T fr[4], T gamma,
-                                               T* F, int FN, int e) {
+                                               T* F, I FN, I e) {
   static_assert(S == 1 || !BLEND, "doubled states feed the HLLE flux only");
   const RiemannPre<T, FAST, Y> rp = riemann_pre<T, FAST, Y, S>(ql, qr, gamma);
   T H[4];
@@ -248,13 +232,13 @@ __device__ __forceinline__ void tile_face_flux(const T ql[4], const T fl[4], con
     hllc_flux<T, FAST, Y>(rp, ql, fl, qr, fr, Gc);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      F[k * FN + e] = Gc[k];
-      F[(4 + k) * FN + e] = H[k];
+      plane_value(F, k, FN, e) = Gc[k];
+      plane_value(F, 4 + k, FN, e) = H[k];
     }
-    F[8 * FN + e] = T(0.5) * (rp.p_l + rp.p_r);
+    plane_value(F, 8, FN, e) = T(0.5) * (rp.p_l + rp.p_r);
   } else {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) F[k * FN + e] = H[k];
+    for (int k = 0; k < 4; ++k) plane_value(F, k, FN, e) = H[k];
   }
 }
 
@@ -413,8 +397,8 @@ __global__ void __launch_bounds__(NT) k_stage_tiles(const SolveDesc* __restrict_
       const int FN = G::FXR * G::FXC;
       T wa = T(1.0), wb = T(1.0);
       if constexpr (BLEND) {
-        wa = tile_sensor<T, FAST>(FX + 8 * FN, G::FXR, G::FXC, fxr, fxc, i, j, nx + 1, ny, jp_lo, jp_hi);
-        wb = tile_sensor<T, FAST>(FX + 8 * FN, G::FXR, G::FXC, fxr + 1, fxc, i + 1, j, nx + 1, ny, jp_lo, jp_hi);
+        wa = tile_sensor<T, FAST>(FX + 8 * FN, G::FXC, fxr * G::FXC + fxc, i, j, nx + 1, ny, jp_lo, jp_hi);
+        wb = tile_sensor<T, FAST>(FX + 8 * FN, G::FXC, (fxr + 1) * G::FXC + fxc, i + 1, j, nx + 1, ny, jp_lo, jp_hi);
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -502,8 +486,8 @@ __global__ void __launch_bounds__(NT) k_stage_tiles(const SolveDesc* __restrict_
       const int FM = G::FYR * G::FYC;
       T va = T(1.0), vb = T(1.0);
       if constexpr (BLEND) {
-        va = tile_sensor<T, FAST>(FY + 8 * FM, G::FYR, G::FYC, fyr, fyc, i, j, nx, ny + 1, jp_lo, jp_hi);
-        vb = tile_sensor<T, FAST>(FY + 8 * FM, G::FYR, G::FYC, fyr, fyc + 1, i, j + 1, nx, ny + 1, jp_lo, jp_hi);
+        va = tile_sensor<T, FAST>(FY + 8 * FM, G::FYC, fyr * G::FYC + fyc, i, j, nx, ny + 1, jp_lo, jp_hi);
+        vb = tile_sensor<T, FAST>(FY + 8 * FM, G::FYC, fyr * G::FYC + fyc + 1, i, j + 1, nx, ny + 1, jp_lo, jp_hi);
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -655,7 +639,7 @@ __global__ void __launch_bounds__(NT, kStagedBlocks<T, FAST>)
 #pragma unroll
           for (int s = 0; s < 5; ++s) staged_cell(d, q, fi + s, J + 3, cells[s]);
           cell_states<T, FAST>(cells, weps, l, r);
-          T* w = W + d.w_p1x + (long long)fi * d.l_p1x + (J + 2);
+          T* w = W + p1x_elem(d, fi, J + 2);
           const bool has_l = fi < xr1, has_r = fi > xr0;
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
@@ -668,7 +652,7 @@ __global__ void __launch_bounds__(NT, kStagedBlocks<T, FAST>)
 #pragma unroll
           for (int s = 0; s < 5; ++s) staged_cell(d, q, I + 3, fj + s, cells[s]);
           cell_states<T, FAST>(cells, weps, l, r);
-          T* w = W + d.w_p1y + (long long)(I + 2) * d.l_p1y + fj;
+          T* w = W + p1y_elem(d, I + 2, fj);
           const bool has_l = fj < yc1, has_r = fj > yc0;
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
@@ -686,7 +670,7 @@ __global__ void __launch_bounds__(NT, kStagedBlocks<T, FAST>)
 #pragma unroll
         for (int s = 0; s < 6; ++s) staged_cell(d, q, fi + s, J + 3, cells[s]);
         pass1_face<T, FAST, false, CHAR>(cells, gamma, ql, qr, weps);
-        T* w = W + d.w_p1x + (long long)fi * d.l_p1x + (J + 2);
+        T* w = W + p1x_elem(d, fi, J + 2);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           w[k * d.s_p1x] = ql[k];
@@ -698,7 +682,7 @@ __global__ void __launch_bounds__(NT, kStagedBlocks<T, FAST>)
 #pragma unroll
         for (int s = 0; s < 6; ++s) staged_cell(d, q, I + 3, fj + s, cells[s]);
         pass1_face<T, FAST, true, CHAR>(cells, gamma, ql, qr, weps);
-        T* w = W + d.w_p1y + (long long)(I + 2) * d.l_p1y + fj;
+        T* w = W + p1y_elem(d, I + 2, fj);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           w[k * d.s_p1y] = ql[k];
@@ -777,7 +761,7 @@ __global__ void __launch_bounds__(NT, kStagedBlocks<T, FAST>)
         const int e2 = e - nxi;
         const int fi = i0 + (x ? e / nxp : 2 * (e2 / nyc)), fj = j0 + (x ? 2 * (e % nxp) : e2 % nyc);
         const bool two = x ? fj + 1 < xc1 : fi + 1 < yr1;
-        const T* p = x ? W + d.w_p1x + (long long)fi * d.l_p1x + fj : W + d.w_p1y + (long long)fi * d.l_p1y + fj;
+        const T* p = W + (x ? p1x_elem(d, fi, fj) : p1y_elem(d, fi, fj));
         const long long ks = x ? d.s_p1x : d.s_p1y, ts = x ? 1 : d.l_p1y;
 #pragma unroll 1
         for (int side = 0; side < 2; ++side) {  // one copy of the code, left then right
@@ -791,13 +775,12 @@ __global__ void __launch_bounds__(NT, kStagedBlocks<T, FAST>)
             flB[k] = side ? flB[k] : frB[k];
           }
         }
-        T* F = W + (x ? d.w_fx : d.w_fy);
-        const int fs = (int)(x ? d.s_fx : d.s_fy);
-        int o = x ? fi * d.ld + fj : fi * d.l_p1y + fj;
+        const long long fs = x ? d.s_fx : d.s_fy;
+        long long o = x ? fx_elem(d, fi, fj) : fy_elem(d, fi, fj);
 #pragma unroll 1
         for (int face = 0; face < (two ? 2 : 1); ++face) {
-          if (x) tile_face_flux<T, FAST, false, BLEND, S>(qlA, flA, qrA, frA, gamma, F, fs, o);
-          else tile_face_flux<T, FAST, true, BLEND, S>(qlA, flA, qrA, frA, gamma, F, fs, o);
+          if (x) tile_face_flux<T, FAST, false, BLEND, S>(qlA, flA, qrA, frA, gamma, W, fs, o);
+          else tile_face_flux<T, FAST, true, BLEND, S>(qlA, flA, qrA, frA, gamma, W, fs, o);
           o += x ? 1 : d.l_p1y;
 #pragma unroll
           for (int k = 0; k < 4; ++k) qlA[k] = qlB[k], flA[k] = flB[k], qrA[k] = qrB[k], frA[k] = frB[k];
@@ -812,18 +795,18 @@ __global__ void __launch_bounds__(NT, kStagedBlocks<T, FAST>)
         const int e2 = e - nxf;
         const int fi = i0 + (x ? e / nxc : e2 / nyc), fj = j0 + (x ? e % nxc : e2 % nyc);
         // the five transverse pass-1 states: columns fj .. fj+4 of an x face, rows fi .. fi+4 of a y face
-        const T* p = x ? W + d.w_p1x + (long long)fi * d.l_p1x + fj : W + d.w_p1y + (long long)fi * d.l_p1y + fj;
+        const T* p = W + (x ? p1x_elem(d, fi, fj) : p1y_elem(d, fi, fj));
         const long long ks = x ? d.s_p1x : d.s_p1y;
         const int ts = x ? 1 : d.l_p1y;
 #pragma unroll(is_f32<T> ? 2 : 1)
         for (int side = 0; side < 2; ++side) {
           T a1[4], a2[4];
-          tile_gq_side<T, FAST>(p + side * 4 * ks, (int)ks, ts, weps, a1, a2);
+          tile_gq_side<T, FAST>(p + side * 4 * ks, ks, ts, weps, a1, a2);
           if (x) put_side<T, FAST, false, S>(side, a1, a2, gamma, ql, fl, qr, fr_);
           else put_side<T, FAST, true, S>(side, a1, a2, gamma, ql, fl, qr, fr_);
         }
-        if (x) tile_face_flux<T, FAST, false, BLEND, S>(ql, fl, qr, fr_, gamma, W + d.w_fx, (int)d.s_fx, fi * d.ld + fj);
-        else tile_face_flux<T, FAST, true, BLEND, S>(ql, fl, qr, fr_, gamma, W + d.w_fy, (int)d.s_fy, fi * d.l_p1y + fj);
+        if (x) tile_face_flux<T, FAST, false, BLEND, S>(ql, fl, qr, fr_, gamma, W, d.s_fx, fx_elem(d, fi, fj));
+        else tile_face_flux<T, FAST, true, BLEND, S>(ql, fl, qr, fr_, gamma, W, d.s_fy, fy_elem(d, fi, fj));
       }
     }
   }
@@ -854,15 +837,15 @@ __global__ void __launch_bounds__(NT) k_staged_residual(const SolveDesc* __restr
     for (int e = tid; e < TX * TY; e += NT) {
       const int i = i0 + e / TY, j = j0 + e % TY;
       if (i >= nx || j >= ny) continue;
+      const long long xa = plane_elem(i, lx, j), xb = xa + lx;
+      const long long ya = plane_elem(i, ly, j), yb = ya + 1;
       T wa = T(1.0), wb = T(1.0), va = T(1.0), vb = T(1.0);
       if constexpr (BLEND) {
-        wa = tile_sensor<T, FAST>(Fx + 8 * fxs, 0, lx, i, j, i, j, nx + 1, ny, jp_lo, jp_hi);
-        wb = tile_sensor<T, FAST>(Fx + 8 * fxs, 0, lx, i + 1, j, i + 1, j, nx + 1, ny, jp_lo, jp_hi);
-        va = tile_sensor<T, FAST>(Fy + 8 * fys, 0, ly, i, j, i, j, nx, ny + 1, jp_lo, jp_hi);
-        vb = tile_sensor<T, FAST>(Fy + 8 * fys, 0, ly, i, j + 1, i, j + 1, nx, ny + 1, jp_lo, jp_hi);
+        wa = tile_sensor<T, FAST>(Fx + 8 * fxs, lx, xa, i, j, nx + 1, ny, jp_lo, jp_hi);
+        wb = tile_sensor<T, FAST>(Fx + 8 * fxs, lx, xb, i + 1, j, nx + 1, ny, jp_lo, jp_hi);
+        va = tile_sensor<T, FAST>(Fy + 8 * fys, ly, ya, i, j, nx, ny + 1, jp_lo, jp_hi);
+        vb = tile_sensor<T, FAST>(Fy + 8 * fys, ly, yb, i, j + 1, nx, ny + 1, jp_lo, jp_hi);
       }
-      const long long xa = (long long)i * lx + j, xb = xa + lx;
-      const long long ya = (long long)i * ly + j, yb = ya + 1;
       T L[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
