@@ -327,12 +327,32 @@ __device__ __forceinline__ void weno_range(f64& e0, f64& e1, f64& e2) {
   e2 = e2 * sc;
 }
 
+// The same for the reciprocal weights of df64, which has the float exponent range: the
+// smallest (eps + beta_k), at least 2^-126, is brought into [1, 2) and the others are
+// held at 2^30, where a weight is below 2^-58 of the largest one's and drops out of
+// the 48 bits.  Without it 1/(eps + beta)^2 overflowed for an epsilon below 2^-63 in
+// a uniform flow (the shear field's is eps rho^2: rho below 2.5e-6) and vanished in
+// all three for differences above 2^31, and the face state was NaN.
+__device__ __forceinline__ df64 weno_scaled(df64 e, float scale) {
+  const float h = e.hi * scale;
+  if (h < 1.0f) return df64(1.0f, 0.0f);
+  return h > 0x1p30f ? df64(0x1p30f, 0.0f) : df64(h, e.lo * scale);
+}
+__device__ __forceinline__ void weno_range(df64& e0, df64& e1, df64& e2) {
+  const float low = fminf(fmaxf(fminf(fminf(e0.hi, e1.hi), e2.hi), 0x1p-126f), 0x1p126f);
+  const float scale = __uint_as_float((254u << 23) - (__float_as_uint(low) & 0x7f800000u));  // 2^-(exponent of low)
+  e0 = weno_scaled(e0, scale);
+  e1 = weno_scaled(e1, scale);
+  e2 = weno_scaled(e2, scale);
+}
+
 // Non-linear weighting of three candidate values with linear weights d in FAST
 // float and df64 (whose float exponent range rules out products of fourth
 // powers): reciprocals.  FAST native double uses weno_nd instead.
 template <class T>
 __device__ __forceinline__ T weno_combine(T e0, T e1, T e2, T d0, T d1, T d2, T p0, T p1, T p2, T scale) {
   static_assert(!is_native_f64<T>, "FAST double takes the common-denominator form (weno_nd)");
+  if constexpr (std::is_same<T, df64>::value) weno_range(e0, e1, e2);
   const T a0 = d0 * inv_square(e0);
   const T a1 = d1 * inv_square(e1);
   const T a2 = d2 * inv_square(e2);
@@ -643,6 +663,7 @@ __device__ __forceinline__ void gq_weights(T q2, T h0, T h1, T h2, T f0, T f1, T
     ra = fma(r0, u0, fma(-r2, u2, -u1)) * (sb * t) + q2;
     rb = fma(r0, u2, fma(-r2, u0, u1)) * (sa * t) + q2;
   } else {
+    if constexpr (std::is_same<T, df64>::value) weno_range(f0, f1, f2);
     const T r0 = inv_square(f0), r1 = inv_square(f1), r2 = inv_square(f2);
     const T ca0 = T(kGqA0 / kGqA1) * r0, ca1 = r1, ca2 = T(kGqA2 / kGqA1) * r2;
     const T cb0 = T(kGqA2 / kGqA1) * r0, cb2 = T(kGqA0 / kGqA1) * r2;
