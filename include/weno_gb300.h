@@ -137,6 +137,8 @@ typedef struct weno_solver weno_solver;
 
 /* weno_eps: the WENO5 smoothness epsilon (<= 0: the reference's 1e-12,
  * weno.rs:223 / utils.rs:3); the density and pressure floors stay 1e-12.
+ * FP32: where epsilon plus indicators are below about 1e-19 their squares leave
+ * the float range and the weights become the linear ones.
  * Debugging aid: with the environment variable WENO_DEBUG_NAN_FILL=1 the
  * solver's (and weno_batch_create's) internal buffers start as NaN bit
  * patterns instead of zeros, so reads of data a step did not write show up. */

@@ -58,3 +58,14 @@ def test_large_differences_df64(wx, cons, scale):
     assert np.isfinite(got).all()
     for c in range(4):
         assert rel_l1(got[..., c], ref[..., c]) <= TOL["df64"], c
+
+
+@pytest.mark.parametrize("cons", [False, True], ids=["char", "cons"])
+def test_fp32_below_its_range_takes_linear_weights(wx, cons):
+    """Indicators whose squares vanish in FP32 (states of order 1e-9 with an epsilon to match): the weights
+    are the linear ones, those of native FP64 with an epsilon far above every indicator."""
+    q = flow(1e-9)
+    ref = run(wx, q, 64, 1.0, cons, "exact")
+    got = run(wx, q, 32, 1e-30, cons)
+    for c in range(4):
+        assert rel_l1(got[..., c], ref[..., c]) <= TOL[32], c

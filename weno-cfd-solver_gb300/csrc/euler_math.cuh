@@ -132,11 +132,15 @@ __device__ __forceinline__ T qrcp(T b) {
   if constexpr (FAST && is_f32<T>) return rcp_seed(b);
   else return T(1.0) / b;
 }
-// 1 / e^2 of the float weights; 2^-126 keeps the square normal for a vanishing
-// epsilon and is below half a unit of any other.
-__device__ __forceinline__ float inv_square(float e) { return rcp_seed(__fmaf_rn(e, e, 0x1p-126f)); }
+// 1 / e^2 of the float weights.  For a vanishing e, 2^-123 keeps six times the sum of
+// three of them, a denominator, below 2^126, from which on the fast division gives
+// zero (the slope was lost, and the scheme first order, where e was below 1e-19); the
+// weights become the linear ones there.  It is below half a unit of the square of any
+// e above 1e-15.
+constexpr float kSquareFloor = 0x1p-123f;
+__device__ __forceinline__ float inv_square(float e) { return rcp_seed(__fmaf_rn(e, e, kSquareFloor)); }
 __device__ __forceinline__ f32x2 inv_square(f32x2 e) {
-  const float2 s = __ffma2_rn(e.v, e.v, make_float2(0x1p-126f, 0x1p-126f));
+  const float2 s = __ffma2_rn(e.v, e.v, make_float2(kSquareFloor, kSquareFloor));
   return f32x2(rcp_seed(s.x), rcp_seed(s.y));
 }
 __device__ __forceinline__ df64 inv_square(df64 e) { return df64(1.0) / (e * e); }
