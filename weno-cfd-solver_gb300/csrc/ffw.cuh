@@ -26,8 +26,10 @@
 // mirror-image states, as the reference's do.
 //
 // Range: differences below 2^22 (smaller than 2^-70 count as zero) and an epsilon in
-// [2^-58, 2^40] keep every float, the low parts of the inverse squares included,
-// normal; callers take the FP64 weights otherwise.
+// [2^-48, 2^40); callers take the FP64 weights otherwise.  The lower end keeps the low
+// part of the reciprocal of the weights' sum, eps^2 / 2^24, a normal float: at 2^-58 it
+// has three bits left and the weights of a smooth stencil are off by 2^-27 of their sum
+// (2^-43 at 2^-50, 2^-45 from 2^-48 on).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -107,12 +109,12 @@ __device__ __forceinline__ double to_double(ff a) {
 __device__ __forceinline__ uint32_t magnitude(double d) { return (uint32_t)__double2hiint(d) & 0x7fffffffu; }
 __device__ __forceinline__ bool covers(uint32_t dmax, double eps) {
   return dmax < ((1023u + 22u) << 20) &&
-         (uint32_t)__double2hiint(eps) - ((1023u - 58u) << 20) < ((58u + 40u) << 20);
+         (uint32_t)__double2hiint(eps) - ((1023u - 48u) << 20) < ((48u + 40u) << 20);
 }
 
 // The same for float pairs.
 __device__ __forceinline__ bool covers_pair(float dmax, float eps) {
-  return dmax < 0x1p22f && eps >= 0x1p-58f && eps <= 0x1p40f;
+  return dmax < 0x1p22f && eps >= 0x1p-48f && eps < 0x1p40f;
 }
 
 // 0.75 eps.
