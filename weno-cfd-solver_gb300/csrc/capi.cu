@@ -53,25 +53,25 @@ int cuda_fail(cudaError_t e, const char* where) {
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 inline int64_t align_elems(int64_t x) { return (x + 63) / 64 * 64; }  // 256 B for f32, 512 B for f64
 
-// Workspace of the residual pipeline for an (m, n) array: pass-1 planes
-// (reused by both directions, except by small FP64 grids, which run both at once)
-// and the face planes of x and y.
+// Workspace of the residual pipeline for an (m, n) array: pass-1 planes (reused by
+// both directions; with `room` those of the y sweep have their own, as the quads, which
+// run both at once, need) and the face planes of x and y.
 struct ResidualLayout {
   int64_t m, n, P1, FX, FY;
   int nf;
   size_t es;
   bool quads;
   size_t off_pl, off_pr, off_ply, off_pry, off_fx, off_fy, total;
-  ResidualLayout(int64_t m_, int64_t n_, bool force_hlle, size_t es_, bool native_f64)
-      : m(m_), n(n_), es(es_), quads(native_f64 && quad_faces(m_, n_)) {
+  ResidualLayout(int64_t m_, int64_t n_, bool force_hlle, size_t es_, bool room, bool quads_)
+      : m(m_), n(n_), es(es_), quads(room && quads_) {
     P1 = align_elems(std::max((m - 5) * n, m * (n - 5)));
     FX = align_elems(std::max<int64_t>((m - 5) * (n - 6), 0));
     FY = align_elems(std::max<int64_t>((m - 6) * (n - 5), 0));
     nf = force_hlle ? 4 : 9;
     off_pl = 0;
     off_pr = off_pl + align_up(4 * P1 * es, 256);
-    off_ply = quads ? off_pr + align_up(4 * P1 * es, 256) : off_pl;
-    off_pry = quads ? off_ply + align_up(4 * P1 * es, 256) : off_pr;
+    off_ply = room ? off_pr + align_up(4 * P1 * es, 256) : off_pl;
+    off_pry = room ? off_ply + align_up(4 * P1 * es, 256) : off_pr;
     off_fx = off_pry + align_up(4 * P1 * es, 256);
     off_fy = off_fx + align_up(nf * FX * es, 256);
     total = off_fy + align_up(nf * FY * es, 256);
@@ -227,7 +227,7 @@ int weno_reconstruct(const double* u, int64_t m, int64_t n, int64_t c, int64_t s
   HostPlanes PL{ws, P1, c1}, PR{at(ws, align_up(4 * P1 * sizeof(double), 256)), P1, c1};
   HostView v{u, s0, s1, s2};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (quad_faces(m, n)) {
+  if (quad_faces(m, n, mode == WENO_FAST, cons != 0, false)) {
     const HostPlanes P[4] = {PL, PR, PL, PR};
     const FaceDst D{q_l, f_l, q_r, f_r, 0, 0};
     const int dirs = ydir ? 2 : 1;
@@ -294,7 +294,7 @@ int weno_riemann(const double* q_l, const double* f_l, const double* q_r, const 
 
 size_t weno_l_local_workspace(int64_t m, int64_t n, int force_hlle) {
   if (m < 6 || n < 6) return 0;
-  return ResidualLayout(m, n, force_hlle != 0, sizeof(double), true).total;
+  return ResidualLayout(m, n, force_hlle != 0, sizeof(double), quad_room(m, n), false).total;
 }
 
 int weno_l_local(const double* u, int64_t m, int64_t n, int64_t c, int64_t s0, int64_t s1, int64_t s2, double dx,
@@ -308,9 +308,10 @@ int weno_l_local(const double* u, int64_t m, int64_t n, int64_t c, int64_t s0, i
   if (!force_hlle && (m < 8 || n < 8))
     return fail(WENO_ERR_SHAPE, "l_local: the HLLC/HLLE blend's shock sensor needs at least 8 x 8 cells, got "
                 "(%lld, %lld)", (long long)m, (long long)n);
-  ResidualLayout Lo(m, n, force_hlle != 0, sizeof(double), true);
+  const bool quads = quad_faces(m, n, mode == WENO_FAST, cons != 0, force_hlle == 0);
+  ResidualLayout Lo(m, n, force_hlle != 0, sizeof(double), quad_room(m, n), quads);
   if (ws_bytes < Lo.total)  // a workspace without room for both sweeps at once runs them in turn
-    Lo = ResidualLayout(m, n, force_hlle != 0, sizeof(double), false);
+    Lo = ResidualLayout(m, n, force_hlle != 0, sizeof(double), false, false);
   if (!ws || ws_bytes < Lo.total) return fail(WENO_ERR_WORKSPACE, "l_local: workspace of %zu bytes needed", Lo.total);
   HostView v{u, s0, s1, s2};
   WENO_CK(residual_dispatch(mode, v, m, n, Lo, ws, gamma, dx, force_hlle != 0, jp_lo, jp_hi, cons != 0, out,
@@ -372,7 +373,8 @@ extern "C" int weno_l_local_host(const double* u, int64_t m, int64_t n, int64_t 
   }
   const size_t in_bytes = (size_t)(m * n * c) * sizeof(double);
   const size_t out_bytes = (size_t)((m - 6) * (n - 6) * 4) * sizeof(double);
-  ResidualLayout Lo(m, n, force_hlle != 0, sizeof(double), true);
+  const bool quads = quad_faces(m, n, mode == WENO_FAST, cons != 0, force_hlle == 0);
+  ResidualLayout Lo(m, n, force_hlle != 0, sizeof(double), quads, quads);
   WENO_CK(grow(&hc.d_in, &hc.in_bytes, in_bytes));
   WENO_CK(grow(&hc.d_out, &hc.out_bytes, out_bytes));
   WENO_CK(grow(&hc.ws, &hc.ws_bytes, Lo.total));
@@ -577,7 +579,8 @@ int weno_solver_create(weno_solver** out, int64_t nx, int64_t ny, double dx, dou
   if ((e = cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, s->device)))
     return bail(e, "cudaDeviceGetAttribute");
   const size_t state_bytes = (size_t)(4 * s->PS) * s->es;
-  s->layout = new ResidualLayout(s->M, s->N, s->force_hlle, s->es, precision == 64);
+  const bool quads = precision == 64 && quad_faces(s->M, s->N, s->mode == WENO_FAST, s->cons, !s->force_hlle);
+  s->layout = new ResidualLayout(s->M, s->N, s->force_hlle, s->es, quads, quads);
   if ((e = cudaMalloc(&s->q, state_bytes))) return bail(e, "cudaMalloc(state)");
   if ((e = cudaMalloc(&s->q1, state_bytes))) return bail(e, "cudaMalloc(stage 1)");
   if ((e = cudaMalloc(&s->q2, state_bytes))) return bail(e, "cudaMalloc(stage 2)");

@@ -380,10 +380,10 @@ __global__ void __launch_bounds__(128, kPass2Blocks<T, OUT>) k_pass2_two(Planes<
 }
 
 // ---------------------------------------------------------------------------
-// Small FP64 grids: four lanes per face.  With fewer than about six warps per SM
-// the one-thread-per-face kernels wait for their own chain of dependent
-// operations (an FP64 one takes 64 cycles: a 64 x 64 residual spent 50 us in each
-// of four passes); a quad shares the fields of a face among its lanes, which costs a third
+// Small FP64 grids: four lanes per face.  With fewer than about four warps per SM
+// (the line is in launch_api.h) the one-thread-per-face kernels wait for their own
+// chain of dependent operations (an FP64 one takes 64 cycles: a 64 x 64 residual spent
+// 50 us in each of four passes); a quad shares the fields of a face among its lanes, which costs a third
 // more FP64 instructions (the averages, repeated on four lanes) and leaves a
 // chain about a sixth as long.  The faces' values are those of k_pass1 / k_pass2 /
 // k_pass2_two operation by operation.

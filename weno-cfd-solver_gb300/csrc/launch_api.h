@@ -29,15 +29,35 @@ struct FaceDst {
   int64_t ps, ld;
 };
 
-// FP64 grids of at most this many faces per sweep take four lanes per face and one
-// launch for both sweeps (Launch::pass1_quads, pass2_quads): six warps per SM of
-// the one-thread form.  Below, that form is a chain of dependent operations (64 x 64
-// residual: 4 x 50 us in its passes); above, the FP64 pipe is busy and the quads'
-// repeated averages cost a third more of it.
-constexpr int64_t kQuadFaces = (int64_t)152 * 6 * 32;
-inline bool quad_faces(int64_t m, int64_t n) {
-  return m > 5 && n > 5 && (m - 5) * n <= kQuadFaces && m * (n - 5) <= kQuadFaces;
+// FP64 grids of few faces take four lanes per face and one launch for both sweeps
+// (Launch::pass1_quads, pass2_quads): there the one-thread form is a chain of
+// dependent operations (64 x 64 residual: 4 x 50 us in its passes), and the quads'
+// repeated averages, a third more of the FP64 pipe, cost less.  The line lies where the
+// quads' one-warp blocks of eight faces no longer fill whole waves: an SM holds 16 of
+// them at the registers of the exact characteristic pass 1 (126), 14 at those of the
+// exact blend's pass 2 (138), and a sweep is one such wave, both sweeps are two.  FAST
+// component-wise kernels are ahead up to 24.  Residual in us, quads against one thread
+// per face, below and above the line:
+//   exact, HLLE     142^2 198 : 226 (char), 152 : 181 (cons)   145^2 263 : 233, 150^2 192 : 189
+//   exact, blend    130^2 234 : 240 (char), 177 : 195 (cons)   138^2 256 : 242, 208 : 197
+//   FAST, char      142^2  96 : 110 (HLLE), 124 : 139 (blend)  150^2 111 : 106, 147 : 135
+//   FAST, cons      172^2  84 :  91 (HLLE), 118 : 122 (blend)
+// and one sweep's reconstruction: exact char 140^2 78 : 103, 155^2 133 : 109; FAST char
+// 140^2 41 : 43, 155^2 53 : 45; FAST cons 172^2 34 : 37.
+constexpr int kQuadBlocksMost = 24;
+constexpr int quad_blocks_per_sm(bool fast, bool cons, bool blend) {
+  return fast ? (cons ? kQuadBlocksMost : 16) : (blend ? 14 : 16);
 }
+inline bool within_quads(int64_t m, int64_t n, int blocks_per_sm) {
+  const int64_t most = (int64_t)152 * 8 * blocks_per_sm;  // faces of a sweep
+  return m > 5 && n > 5 && (m - 5) * n <= most && m * (n - 5) <= most;
+}
+inline bool quad_faces(int64_t m, int64_t n, bool fast, bool cons, bool blend) {
+  return within_quads(m, n, quad_blocks_per_sm(fast, cons, blend));
+}
+// Grids whose workspace has room for both sweeps at once (reported without the mode
+// and the reconstruction, so for the largest of the above).
+inline bool quad_room(int64_t m, int64_t n) { return within_quads(m, n, kQuadBlocksMost); }
 
 struct StepCtl;
 namespace dfm {
