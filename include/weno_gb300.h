@@ -167,8 +167,11 @@ int weno_solver_totals(weno_solver* s, double* out4);
 /* CUDA-event timing of kernel groups, recorded on the solver's stream during
  * runs with use_graph=0.  Classes: 0 CFL reduction + dt, 1 boundary fills,
  * 2 x pass 1, 3 x pass 2, 4 sensor blends, 5 y pass 1, 6 y pass 2,
- * 7 residual + stage combination.  Enabling resets the record; the report
- * synchronises and returns the summed milliseconds and launch-group counts. */
+ * 7 residual + stage combination.  FP32 has the sensor blend inside class 7 and
+ * reports 0 for class 4; small FP64 grids, whose sweeps share their launches,
+ * launch them one after the other while timing is on.  Enabling resets the
+ * record; the report synchronises and returns the summed milliseconds and
+ * launch-group counts. */
 int weno_solver_enable_timing(weno_solver* s, int on);
 int weno_solver_timing_report(weno_solver* s, double* ms, int64_t* launches, int nclasses);
 /* Number of kernel launches one step enqueues (for launch accounting). */

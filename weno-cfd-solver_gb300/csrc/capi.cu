@@ -109,8 +109,11 @@ cudaError_t residual_pipeline(HostView u, int64_t m, int64_t n, const ResidualLa
     const HostPlanes P[4] = {PL, PR, {at(ws, Lo.off_ply), Lo.P1, n - 5}, {at(ws, Lo.off_pry), Lo.P1, n - 5}};
     const FaceDst X{fx, fx + 4 * Lo.FX, fx + 8 * Lo.FX, nullptr, Lo.FX, n - 6};
     const FaceDst Y{fy, fy + 4 * Lo.FY, fy + 8 * Lo.FY, nullptr, Lo.FY, n - 5};
-    WENO_TIMED(HC_PASS1_X, Lx::pass1_quads(u, m, n, 3, gamma, !cons, P, weps, st));
-    WENO_TIMED(HC_PASS2_X, Lx::pass2_quads(P, m, n, 3, gamma, kind, X, Y, weps, st));
+    // both sweeps in one launch; with timing on one after the other, each in its class
+    for (int dirs = tm.mark ? 1 : 3; dirs <= (tm.mark ? 2 : 3); ++dirs) {
+      WENO_TIMED(dirs == 2 ? HC_PASS1_Y : HC_PASS1_X, Lx::pass1_quads(u, m, n, dirs, gamma, !cons, P, weps, st));
+      WENO_TIMED(dirs == 2 ? HC_PASS2_Y : HC_PASS2_X, Lx::pass2_quads(P, m, n, dirs, gamma, kind, X, Y, weps, st));
+    }
   } else {
     WENO_TIMED(HC_PASS1_X, Lx::pass1(u, m - 5, n, gamma, false, !cons, PL, PR, weps, st));
     WENO_TIMED(HC_PASS2_X, Lx::pass2(PL, PR, m - 5, n - 6, gamma, false, kind, fx, fx + 4 * Lo.FX, fx + 8 * Lo.FX,
@@ -123,6 +126,7 @@ cudaError_t residual_pipeline(HostView u, int64_t m, int64_t n, const ResidualLa
   }
   HostPlanes Fx{fx, Lo.FX, n - 6}, Fy{fy, Lo.FY, n - 5};
   if (std::is_same<T, float>::value && !force_hlle) {
+    // (timing: the blend is part of the residual's class)
     WENO_TIMED(HC_RESIDUAL, Lx::residual_blend(Fx, Fy, m - 6, n - 6, dx, jp_lo, jp_hi, stage, Qn, Qs, Qo, ctl, st));
     return cudaSuccess;
   }
