@@ -6,19 +6,6 @@
 
 namespace weno {
 
-inline namespace WENO_TU_NS {
-namespace bdetail {
-
-constexpr int kNT = 256;
-
-template <class T, int TX, int TY, bool BLEND>
-constexpr size_t tile_smem() {
-  return sizeof(T) * (size_t)TileGeom<TX, TY, BLEND>::TOTAL;
-}
-
-}  // namespace bdetail
-}  // inline namespace WENO_TU_NS
-
 // Fused configurations only (0-3); the staged configuration has its own launcher.
 #define WENO_TILE_SWITCH(cfg, MACRO) \
   switch (cfg) {                     \
@@ -42,7 +29,7 @@ size_t BatchLaunch<H, FAST>::smem_bytes(int cfg, bool blend) {
   using T = dev_t<H>;
   size_t r = 0;
 #define WENO_SM(TX, TY) \
-  r = blend ? bdetail::tile_smem<T, TX, TY, true>() : bdetail::tile_smem<T, TX, TY, false>()
+  r = blend ? tile_smem<T, TX, TY, true>() : tile_smem<T, TX, TY, false>()
   WENO_TILE_SWITCH(cfg, WENO_SM)
 #undef WENO_SM
   return r > 227 * 1024 ? 0 : r;
@@ -79,7 +66,7 @@ cudaError_t BatchLaunch<H, FAST>::staged(bool chr, bool blend, const SolveDesc* 
                                          double weps, cudaStream_t st) {
   using T = dev_t<H>;
   if (ntiles <= 0 || grid <= 0) return cudaSuccess;
-  constexpr int TX = kTileTX[kStagedConfig], TY = kTileTY[kStagedConfig], NT = bdetail::kNT;
+  constexpr int TX = kTileTX[kStagedConfig], TY = kTileTY[kStagedConfig], NT = kTileThreads;
   constexpr int NP = kStagedThreads<T, FAST>;
   const int4* tl = static_cast<const int4*>(tiles);
   T* W = static_cast<T*>(ws);
@@ -113,7 +100,7 @@ cudaError_t BatchLaunch<H, FAST>::cfl(int cfg, const SolveDesc* solves, SolveCtl
   using T = dev_t<H>;
   if (ntiles <= 0 || grid <= 0) return cudaSuccess;
   const int tx = kTileTX[cfg < kNumTileConfigs ? cfg : 0], ty = kTileTY[cfg < kNumTileConfigs ? cfg : 0];
-  k_cfl_tiles<T, bdetail::kNT><<<grid, bdetail::kNT, 0, st>>>(solves, ctl, static_cast<const int4*>(tiles), ntiles,
+  k_cfl_tiles<T, kTileThreads><<<grid, kTileThreads, 0, st>>>(solves, ctl, static_cast<const int4*>(tiles), ntiles,
                                                               tx, ty, static_cast<const T*>(q), (T)gamma);
   return cudaGetLastError();
 }

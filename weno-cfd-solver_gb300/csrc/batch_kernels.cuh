@@ -116,6 +116,13 @@ struct TileGeom {
   static constexpr int DX_ELEMS = 4 * TX * TY;
   static constexpr int TOTAL = U_ELEMS + P1_ELEMS + F_ELEMS + DX_ELEMS;
 };
+// Dynamic shared memory of a fused tile, and the threads of its block (of the staged
+// residual and the first CFL reduction too).
+template <class T, int TX, int TY, bool BLEND>
+constexpr size_t tile_smem() {
+  return sizeof(T) * (size_t)TileGeom<TX, TY, BLEND>::TOTAL;
+}
+constexpr int kTileThreads = 256;
 
 // Sensor weight at element e, row pitch C, of a local face array: face (gr, gc) of a
 // global face array of GR x GC entries (riemann.rs:352-410: central differences,

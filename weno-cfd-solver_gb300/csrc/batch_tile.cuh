@@ -9,13 +9,6 @@ namespace weno {
 inline namespace WENO_TU_NS {
 namespace tdetail {
 
-constexpr int kNT = 256;
-
-template <class T, int TX, int TY, bool BLEND>
-constexpr size_t tile_smem() {
-  return sizeof(T) * (size_t)TileGeom<TX, TY, BLEND>::TOTAL;
-}
-
 template <class T, bool FAST, bool CHAR, bool BLEND, int TX, int TY>
 cudaError_t launch_stage(const SolveDesc* solves, SolveCtl* ctl, const int4* tiles, int ntiles, int grid,
                          const CUtensorMap* tmaps, const T* qn, T* qo, int stage, T gamma, T jp_lo, T jp_hi, T weps,
@@ -24,12 +17,12 @@ cudaError_t launch_stage(const SolveDesc* solves, SolveCtl* ctl, const int4* til
   if constexpr (sm > 227 * 1024) {
     return cudaErrorInvalidConfiguration;
   } else {
-    auto k = k_stage_tiles<T, FAST, CHAR, BLEND, TX, TY, kNT>;
+    auto k = k_stage_tiles<T, FAST, CHAR, BLEND, TX, TY, kTileThreads>;
     // The attribute is per device and cheap to set: set it on every launch (also
     // keeps host threads from racing on a cached flag).
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    k<<<grid, kNT, sm, st>>>(solves, ctl, tiles, ntiles, tmaps, qn, qo, stage, gamma, jp_lo, jp_hi, weps, skip_tile,
+    k<<<grid, kTileThreads, sm, st>>>(solves, ctl, tiles, ntiles, tmaps, qn, qo, stage, gamma, jp_lo, jp_hi, weps, skip_tile,
                              wait_ns);
     return cudaGetLastError();
   }
@@ -41,10 +34,10 @@ int occupancy() {
   if constexpr (sm > 227 * 1024) {
     return 0;
   } else {
-    auto k = k_stage_tiles<T, FAST, CHAR, BLEND, TX, TY, kNT>;
+    auto k = k_stage_tiles<T, FAST, CHAR, BLEND, TX, TY, kTileThreads>;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) return 0;
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kNT, sm) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kTileThreads, sm) != cudaSuccess) return 0;
     return n;
   }
 }

@@ -125,18 +125,16 @@ cudaError_t residual_pipeline(HostView u, int64_t m, int64_t n, const ResidualLa
                                      nullptr, Lo.FY, n - 5, weps, st));
   }
   HostPlanes Fx{fx, Lo.FX, n - 6}, Fy{fy, Lo.FY, n - 5};
-  if (std::is_same<T, float>::value && !force_hlle) {
-    // (timing: the blend is part of the residual's class)
-    WENO_TIMED(HC_RESIDUAL, Lx::residual_blend(Fx, Fy, m - 6, n - 6, dx, jp_lo, jp_hi, stage, Qn, Qs, Qo, ctl, st));
-    return cudaSuccess;
-  }
-  if (!force_hlle) {
-    HostPlanes C{fx, Lo.FX, n - 6}, E{fx + 4 * Lo.FX, Lo.FX, n - 6}, P{fx + 8 * Lo.FX, Lo.FX, n - 6};
-    WENO_TIMED(HC_BLEND, Lx::blend(C, E, P, m - 5, n - 6, jp_lo, jp_hi, nullptr, st));
-  }
-  if (!force_hlle) {
-    HostPlanes C{fy, Lo.FY, n - 5}, E{fy + 4 * Lo.FY, Lo.FY, n - 5}, P{fy + 8 * Lo.FY, Lo.FY, n - 5};
-    WENO_TIMED(HC_BLEND, Lx::blend(C, E, P, m - 6, n - 5, jp_lo, jp_hi, nullptr, st));
+  if constexpr (std::is_same<T, float>::value) {
+    if (!force_hlle) {  // (timing: the blend is part of the residual's class)
+      WENO_TIMED(HC_RESIDUAL, Lx::residual_blend(Fx, Fy, m - 6, n - 6, dx, jp_lo, jp_hi, stage, Qn, Qs, Qo, ctl, st));
+      return cudaSuccess;
+    }
+  } else if (!force_hlle) {
+    HostPlanes Cx{fx, Lo.FX, n - 6}, Ex{fx + 4 * Lo.FX, Lo.FX, n - 6}, Px{fx + 8 * Lo.FX, Lo.FX, n - 6};
+    WENO_TIMED(HC_BLEND, Lx::blend(Cx, Ex, Px, m - 5, n - 6, jp_lo, jp_hi, nullptr, st));
+    HostPlanes Cy{fy, Lo.FY, n - 5}, Ey{fy + 4 * Lo.FY, Lo.FY, n - 5}, Py{fy + 8 * Lo.FY, Lo.FY, n - 5};
+    WENO_TIMED(HC_BLEND, Lx::blend(Cy, Ey, Py, m - 6, n - 5, jp_lo, jp_hi, nullptr, st));
   }
   WENO_TIMED(HC_RESIDUAL, Lx::residual(Fx, Fy, m - 6, n - 6, dx, stage, out, Qn, Qs, Qo, ctl, st));
 #undef WENO_TIMED

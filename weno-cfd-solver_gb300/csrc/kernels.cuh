@@ -763,11 +763,9 @@ __global__ void __launch_bounds__(128) k_bc_dmr(S3<T> Q, int64_t nx, int64_t ny,
       v[2] = -v[2];
       if constexpr (NC == 8) v[6] = -v[6];
     }
-  } else if (i >= nx + 3) {
+  } else {  // i >= nx + 3
 #pragma unroll
     for (int k = 0; k < NC; ++k) v[k] = Q.at(nx + 2, j, k);
-  } else {
-    return;
   }
 #pragma unroll
   for (int k = 0; k < NC; ++k) Q.at(i, j, k) = v[k];

@@ -204,11 +204,15 @@ cudaError_t Launch<H, FAST>::blend(HostPlanes Fc, HostPlanes Fe, HostPlanes Pbar
   using T = dev_t<H>;
   using namespace detail;
   if (rows <= 0 || cols <= 0) return cudaSuccess;
-  const Shape g = shape<T>(rows, cols);
-  auto C = planes<T>(Fc), E = planes<T>(Fe), P = planes<T>(Pbar);
-  if (out) k_blend<T, FAST, true><<<g.grid, g.block, 0, st>>>(C, E, P, rows, cols, (T)jp_lo, (T)jp_hi, static_cast<T*>(out), C);
-  else k_blend<T, FAST, false><<<g.grid, g.block, 0, st>>>(C, E, P, rows, cols, (T)jp_lo, (T)jp_hi, nullptr, C);
-  return cudaGetLastError();
+  if constexpr (!is_f32<T>) {
+    const Shape g = shape<T>(rows, cols);
+    auto C = planes<T>(Fc), E = planes<T>(Fe), P = planes<T>(Pbar);
+    if (out) k_blend<T, FAST, true><<<g.grid, g.block, 0, st>>>(C, E, P, rows, cols, (T)jp_lo, (T)jp_hi, static_cast<T*>(out), C);
+    else k_blend<T, FAST, false><<<g.grid, g.block, 0, st>>>(C, E, P, rows, cols, (T)jp_lo, (T)jp_hi, nullptr, C);
+    return cudaGetLastError();
+  } else {
+    return cudaErrorNotSupported;  // residual_blend
+  }
 }
 
 template <class H, bool FAST>
