@@ -14,11 +14,12 @@
  *   WENO_EXACT  the reference's operation order with no FMA contraction: the
  *               doubles are bit-identical to the Rust core's.
  *   WENO_FAST   the same scheme with fewer FP64 operations and FMA
- *               contraction: reciprocals / square roots within 1-2 ulp
- *               (seeded Newton steps, see weno_fast_math_eval), the WENO
- *               weight normalisations within 2^-41; agrees with WENO_EXACT
- *               to rounding (about 1e-16 relative L1 on a step, within 1e-10
- *               over multi-step runs).
+ *               contraction: quotients and square roots correctly rounded, the
+ *               WENO weights within 2^-44 of their sum (formed as pairs of
+ *               floats; for field differences from 2^22 or an epsilon outside
+ *               [2^-48, 2^40) in FP64, normalised within 2^-41); agrees with
+ *               WENO_EXACT to rounding (about 1e-16 relative L1 on a step,
+ *               within 1e-10 over multi-step runs).
  *
  * Return value: WENO_OK (0) or an error code; weno_last_error() describes the
  * last error of the calling thread.
@@ -276,12 +277,12 @@ int weno_init_refac(double* out, int64_t nx, int64_t ny, double lx, double ly, d
  * denominators, with no counterpart in the reference. */
 int weno_probe_rates(double* fp64_tflops, double* fp64_div_per_s, double* fp32_tflops, void* stream);
 
-/* Diagnostics: the FAST-mode FP64 reciprocal, reciprocal square root and
- * square root (an FP32 hardware seed and one third-order Newton step; within
- * 1, 1 and 2 ulp) and the second-order reciprocal (relative error below
- * 2^-41) of n device doubles x, written to the device array out as
- * [1/x | 1/sqrt(x) | sqrt(x) | 1/x second order] (4n doubles), for tests of
- * their error bounds. */
+/* Diagnostics: the kernels' FP64 reciprocal and square root (integer forms,
+ * correctly rounded, subnormals and specials included), a reciprocal square
+ * root within 1 ulp, and the second-order reciprocal of the FAST WENO weights
+ * (relative error below 2^-41) of n device doubles x, written to the device
+ * array out as [1/x | 1/sqrt(x) | sqrt(x) | 1/x second order] (4n doubles), for
+ * tests of their error bounds. */
 int weno_fast_math_eval(const double* x, double* out, int64_t n, void* stream);
 
 #ifdef __cplusplus

@@ -1,11 +1,13 @@
 // Live arithmetic-rate probe: the denominators of the compute roofline
 // (FP64 FMA, FP64 divide and FP32 FMA throughput of this GPU), measured with
-// CUDA events on independent FMA chains; and an evaluator of the FAST FP64
-// reciprocal / square-root forms for their error-bound tests.
+// CUDA events on independent FMA chains; and an evaluator of the kernels' FP64
+// reciprocals and square root for the tests of their error bounds.
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#define WENO_TU_NS probe
 #include "../../include/weno_gb300.h"
+#include "f64.cuh"
 #include "fp64_fast.cuh"
 
 namespace {
@@ -28,13 +30,30 @@ __global__ void div_chains(double* out, int iters, double b) {
   out[blockIdx.x * blockDim.x + threadIdx.x] = x0 + x1 + x2 + x3;
 }
 
+// 1/sqrt(x) within 1 ulp, for weno_fast_math_eval only (the kernels multiply the
+// correctly rounded root and reciprocal): third order, e = 1 - m y0^2 and
+// y0 (1 + e/2 + 3 e^2 / 8), on an FP32 seed for m in [1, 4) with x = m 2^E, E even;
+// CUDA's rsqrt outside [2^-1000, 2^1000].
+__device__ double rsqrt_1ulp(double x) {
+  using namespace weno::f64fast;
+  const int hi = __double2hiint(x), lo = __double2loint(x);
+  const int ex = biased_exp(hi);
+  if (hi < 0 || ex < kExpLo || ex > kExpHi) return ::rsqrt(x);
+  const int e2 = ex - 1023, odd = e2 & 1;
+  const double m = __hiloint2double((hi & 0x000fffff) | ((1023 + odd) << 20), lo);
+  const double y0 = widen(weno::rsqrt_seed(narrow(hi, lo, 127u + (unsigned)odd)));
+  const double e = fma(-m, y0 * y0, 1.0);
+  const double y = fma(y0 * e, fma(0.375, e, 0.5), y0);  // in [0.5, 1]
+  return __hiloint2double(__double2hiint(y) - ((e2 - odd) / 2) * (1 << 20), __double2loint(y));
+}
+
 __global__ void k_fast_math(const double* x, double* out, int64_t n) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double v = x[i];
-  out[i] = weno::f64fast::rcp(v);
-  out[n + i] = weno::f64fast::rsqrt(v);
-  out[2 * n + i] = weno::f64fast::sqrt(v);
+  out[i] = weno::xdiv(1.0, v);
+  out[n + i] = rsqrt_1ulp(v);
+  out[2 * n + i] = weno::xsqrt(v);
   out[3 * n + i] = weno::f64fast::rcp2(v);
 }
 
