@@ -46,6 +46,43 @@ def test_l_local(wx, orc, mode, state, cons, hlle):  # noqa: F811
     check(wx.l_local_py(q, *args), orc.l_local_py(q, *args), mode, "L", tol_for(state))
 
 
+def tiny_cells(rng, m, n):
+    """Ordinary cells beside cells with subnormal momenta, densities or energies."""
+    q = noisy(rng, m, n)
+    for k in range(4):
+        hit = rng.random((m, n)) < 0.15
+        q[hit, k] = rng.choice([-1.0, 1.0], hit.sum()) * 2.0 ** rng.integers(-1074, -1015, hit.sum())
+    return q
+
+
+ENDS = {
+    "tiny_cells": tiny_cells,
+    "1e-300": lambda rng, m, n: noisy(rng, m, n) * 1e-300,
+    "1e-318": lambda rng, m, n: noisy(rng, m, n) * 1e-318,
+    "1e-80": lambda rng, m, n: noisy(rng, m, n) * 1e-80,
+    "1e76": lambda rng, m, n: noisy(rng, m, n) * 1e76,  # weights d / (eps + beta)^2 near the smallest double
+    "1e80": lambda rng, m, n: noisy(rng, m, n) * 1e80,  # subnormal and vanishing weights
+    "1e152": lambda rng, m, n: noisy(rng, m, n) * 1e152,
+    "1e300": lambda rng, m, n: noisy(rng, m, n) * 1e300,
+}
+
+
+@pytest.mark.parametrize("state", list(ENDS))
+@pytest.mark.parametrize("cons", [False, True], ids=["char", "cons"])
+@pytest.mark.parametrize("shape", [LARGE[0], SMALL[2]], ids=ids)
+def test_exact_at_the_ends_of_the_range(wx, orc, state, cons, shape):
+    """Quotients with subnormal operands and results, zeros, infinities and NaN inside the loops of the exact
+    kernels (and of the four-lane ones): the oracle's bits."""
+    q = ENDS[state](np.random.default_rng(77), *shape)
+    with np.errstate(all="ignore"):
+        for ydir, fw, fo in ((0, wx.weno_x_py, orc.weno_x_py), (1, wx.weno_y_py, orc.weno_y_py)):
+            for got, ref, nm in zip(fw(q, G, cons=cons), fo(q, G, cons=cons), ("q_l", "f_l", "q_r", "f_r")):
+                check(got, ref, "exact", f"{nm} y={ydir}")
+        for hlle in (True, False):
+            args = (0.01, G, hlle, (0.05, 0.4), cons)
+            check(wx.l_local_py(q, *args), orc.l_local_py(q, *args), "exact", "L")
+
+
 def _residual(wx, q, cons, hlle, m_, nan_scratch, one_sweep):
     """l_local through the C interface, scratch and output filled with NaN patterns."""
     import torch

@@ -17,9 +17,9 @@
 // with two guard bits is round-to-nearest-even.
 //
 // Zeros, subnormals, infinities, NaN and results outside the normal range take
-// the same digits with integer code before and after them (the compiler's own
-// division is not called: with it on the cold side of a rolled loop, kernels
-// built here returned wrong values for faces that held subnormals).
+// the same digits with integer code before and after them: bit for bit the IEEE
+// results as well, without the call and the second division routine that the
+// compiler's own quotient would put into every loop that divides.
 #pragma once
 
 #include <cstdint>
