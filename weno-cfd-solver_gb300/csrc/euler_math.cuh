@@ -467,7 +467,7 @@ __device__ __forceinline__ f64 face_slope(f64 dn, f64 fn, f64 dm, f64 df, double
 }
 
 // Both states of one field at the face between u2 and u3 with float-pair weights
-// (ffw.cuh): 21 FP64 operations, where the FP64 weights below take 69.
+// (ffw.cuh): 19 FP64 operations, where the FP64 weights below take 69.
 __device__ __forceinline__ void weno5_lr_ffw(f64 u2, f64 u3, f64 d0, f64 d1, f64 d2, f64 d3, f64 d4, f64 weps,
                                              f64& left, f64& right) {
   const ffw::ff w = ffw::eps75(weps.v);

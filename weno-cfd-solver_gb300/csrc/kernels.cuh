@@ -94,7 +94,8 @@ __global__ void __launch_bounds__(128, kPass1Blocks<T>) k_pass1(CView<T> u, int6
     // df64 has the float exponent range: a face whose stencil holds a tiny
     // density or a huge value (near vacuum the characteristic projection scales
     // by 1/(rho*c)) is left to k_pass1_marked, in native double: with that code
-    // in this kernel its registers (168 against 96) would bind every face.
+    // in this kernel its registers would bind every face (168 where 128, with 64 bytes
+    // of spills in the characteristic form, serve without it).
     bool safe = true;
 #pragma unroll
     for (int s = 0; s < 6; ++s) {
